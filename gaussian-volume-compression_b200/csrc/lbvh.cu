@@ -80,19 +80,29 @@ __global__ void __launch_bounds__(256) k_bounds(Src src, int64_t n, uint32_t* bo
             }
         }
     }
+    // One atomic per bound and block: all of them go to six words of one line, and one per
+    // warp of 1184 blocks (57k atomics) took 36-47 us at any n.
+    __shared__ uint32_t s_mn[8][3], s_mx[8][3];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        for (int off = 16; off > 0; off >>= 1) {
-            mn[a] = min(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], off));
-            mx[a] = max(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], off));
+        const uint32_t lo = __reduce_min_sync(0xffffffffu, mn[a]), hi = __reduce_max_sync(0xffffffffu, mx[a]);
+        if (lane == 0) {
+            s_mn[warp][a] = lo;
+            s_mx[warp][a] = hi;
         }
     }
-    if ((threadIdx.x & 31) == 0) {
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        const int a = threadIdx.x;
+        uint32_t lo = 0xffffffffu, hi = 0u;
 #pragma unroll
-        for (int a = 0; a < 3; a++) {
-            atomicMin(&bounds[a], mn[a]);
-            atomicMax(&bounds[3 + a], mx[a]);
+        for (int w = 0; w < 8; w++) {
+            lo = min(lo, s_mn[w][a]);
+            hi = max(hi, s_mx[w][a]);
         }
+        atomicMin(&bounds[a], lo);
+        atomicMax(&bounds[3 + a], hi);
     }
 }
 
