@@ -831,8 +831,7 @@ def run_ours(args):
     t_bwd = kt["bwd_kernel_ms"] / max(kt["bwd_kernel_calls"], 1)
     hbm, bf16, bf16s, src = measured_peaks()
     bwd_kernel = "k_backward_cta" if args.bwd_mode == "tensor_core" or (
-        args.eval_path == "tensor_core" and args.bwd_mode == "auto") else (
-        "k_backward_tiles" if args.bwd_mode == "atomic" or (args.bwd_mode == "auto" and ugb) else "k_backward_gauss")
+        args.eval_path == "tensor_core" and args.bwd_mode == "auto") else "k_backward_gauss"
     fwd_kernel = "k_forward" if args.eval_path == "plain_tile" else "k_forward_cta"
     if t_bwd >= t_fwd:
         name, flops, t_k = bwd_kernel, f_bwd, t_bwd

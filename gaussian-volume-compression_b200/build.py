@@ -29,6 +29,7 @@ SOURCES = {
     "cta.cu": [],
     "fwd_tc.cu": [],
     "bwd_tc.cu": [],
+    "bwd_gauss.cu": [],
     "knn.cu": [],
     "trainsamp.cu": [],
 }

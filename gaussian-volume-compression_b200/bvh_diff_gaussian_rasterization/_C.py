@@ -185,8 +185,8 @@ def set_cov_grad_mode(mode, device=None):
 
 
 def set_backward_mode(mode, device=None):
-    """'auto' (follow use_gaussian_bvh; the tensor-core reduction on the tensor-core eval
-    path), 'deterministic', 'atomic' (sample-tile traversal) or 'tensor_core'."""
+    """'auto' (Gaussian-owned sums; the tensor-core reduction on the tensor-core eval path),
+    'deterministic' or 'atomic' (both the Gaussian-owned sums) or 'tensor_core'."""
     set_option(_n.OPT_BWD_MODE, {"auto": 0, "deterministic": 1, "atomic": 2, "tensor_core": 3}[mode], device)
 
 

@@ -509,7 +509,7 @@ static cudaError_t launch_bwd_cta_impl(const BwdArgs& a, int64_t n_blocks, const
         cudaFuncSetAttribute(k_backward_cta<COUNT, STACKLESS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     k_backward_cta<COUNT, STACKLESS><<<(unsigned)n_blocks, kBRows + 64, smem, st>>>(
-        a.n_tiles * kTile, bdesc, bboxes, a.gnodes, a.g_internal, a.recs, a.gperm, a.s_grad, a.s_gyz, a.s_ok,
+        a.n_slots, bdesc, bboxes, a.gnodes, a.g_internal, a.recs, a.gperm, a.s_grad, a.s_gyz, a.s_ok,
         a.clog, a.cend, a.cdesc, a.gacc, a.status, a.stats);
     gvc::note_launch();
     return cudaGetLastError();

@@ -179,7 +179,7 @@ int gvc_ctx_create(gvc_ctx** out) {
     GVC_CUDA(cudaMalloc(&c->d_stats, sizeof(unsigned long long) * 16), "cudaMalloc stats");
     GVC_CUDA(cudaMemset(c->d_stats, 0, sizeof(unsigned long long) * 16), "cudaMemset stats");
     GVC_CUDA(cudaMallocHost(&c->h_status, sizeof(int)), "cudaMallocHost");
-    Lbvh* sorted[] = {&c->s_sort, &c->tiles, &c->gbvh, &c->cells, &c->knn, &c->ts_sort, &c->scratch.dbg,
+    Lbvh* sorted[] = {&c->s_sort, &c->gbvh, &c->cells, &c->knn, &c->ts_sort, &c->scratch.dbg,
                       &c->scratch.msamp};
     for (Lbvh* L : sorted) L->status = c->d_status;
     *out = c;
@@ -192,15 +192,15 @@ void gvc_ctx_destroy(gvc_ctx* ctx) {
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(c->device);
-    Lbvh* lbvhs[] = {&c->s_sort,  &c->tiles,      &c->gbvh,          &c->cells,
-                     &c->knn,     &c->ts_sort,    &c->scratch.dbg,   &c->scratch.msamp};
+    Lbvh* lbvhs[] = {&c->s_sort,  &c->gbvh,        &c->cells,       &c->knn,
+                     &c->ts_sort, &c->scratch.dbg, &c->scratch.msamp};
     for (Lbvh* L : lbvhs) {
         DevBuf* bufs[] = {&L->keys, &L->keys_alt, &L->perm, &L->perm_alt, &L->boxes, &L->sorted_boxes, &L->left,
                           &L->right, &L->parent, &L->flags, &L->node_boxes, &L->nodes, &L->hist, &L->bounds,
                           &L->onesweep};
         for (DevBuf* b : bufs) b->release();
     }
-    DevBuf* bufs[] = {&c->s_sorted, &c->fwd_sorted, &c->tile_boxes, &c->tile_keys, &c->tile_gdesc, &c->blk_desc, &c->blk_boxes, &c->blk_desc_b, &c->blk_boxes_b, &c->s_grad, &c->s_gyz, &c->s_ok, &c->grec, &c->gtmp,
+    DevBuf* bufs[] = {&c->s_sorted, &c->fwd_sorted, &c->tile_boxes, &c->tile_gdesc, &c->b_rows, &c->b_boxes, &c->blk_desc, &c->blk_boxes, &c->blk_desc_b, &c->blk_boxes_b, &c->s_grad, &c->s_gyz, &c->s_ok, &c->grec, &c->gtmp,
                       &c->m_out_sorted, &c->knn_boxes, &c->ts_points, &c->ts_words, &c->ts_gt64, &c->scratch.gacc, &c->scratch.tmp_boxes, &c->scratch.tmp_out,
                       &c->clog, &c->cend};
     for (DevBuf* b : bufs) b->release();
@@ -281,32 +281,18 @@ int gvc_sync_status(gvc_ctx* ctx, void* stream) {
     return debug_check(ctx, (cudaStream_t)stream);
 }
 
-// Lane groups of the 32-sample tiles (forward per tile, sample-side backward kernels).
+// Lane groups of the 32-sample tiles (forward per tile).
 static int ensure_tile_groups(gvc_ctx* ctx, cudaStream_t st) {
     if (ctx->tile_groups_ready || ctx->n_tiles == 0) return GVC_OK;
     const int64_t slots_g = ctx->n_tiles * kGroups;
     GVC_CUDA(ctx->tile_boxes.ensure(sizeof(float4) * 2 * slots_g), "alloc tile_boxes");
-    GVC_CUDA(ctx->tile_keys.ensure(sizeof(uint32_t) * slots_g), "alloc tile_keys");
     GVC_CUDA(ctx->tile_gdesc.ensure(sizeof(uint32_t) * ctx->n_tiles), "alloc tile_gdesc");
     // reads the context's own sorted samples (the caller's array may be gone by now)
     GVC_CUDA(launch_sample_tiles(ctx->S, ctx->n_tiles, nullptr, nullptr, ctx->s_sort.keys.as<uint32_t>(),
                                  ctx->s_sorted.as<float4>(),
-                                 ctx->tile_boxes.as<float4>(), ctx->tile_keys.as<uint32_t>(),
-                                 ctx->tile_gdesc.as<uint32_t>(), true, st),
+                                 ctx->tile_boxes.as<float4>(), ctx->tile_gdesc.as<uint32_t>(), true, st),
              "sample tile groups");
     ctx->tile_groups_ready = true;
-    return GVC_OK;
-}
-
-// The LBVH over the tile lane groups (the deterministic Gaussian-owned backward).
-static int ensure_tile_lbvh(gvc_ctx* ctx, cudaStream_t st) {
-    if (ctx->tiles_ready || ctx->n_tiles == 0) return GVC_OK;
-    const int rc = ensure_tile_groups(ctx, st);
-    if (rc != GVC_OK) return rc;
-    GVC_CUDA(lbvh_hierarchy(ctx->tiles, ctx->n_tiles * kGroups, ctx->tile_keys.as<uint32_t>(),
-                            ctx->tile_boxes.as<float4>(), st),
-             "sample-group LBVH");
-    ctx->tiles_ready = true;
     return GVC_OK;
 }
 
@@ -325,17 +311,15 @@ int gvc_build_bvh(gvc_ctx* ctx, const float* samples, int64_t S, int debug, int 
     ctx->blk_b_ready = false;
     ctx->clog_ready = false;
     ctx->fwd_sorted_ready = false;
-    ctx->tiles_ready = false;        // the sample-group LBVH is built by its first user
-    ctx->tile_groups_ready = false;  // so are the lane groups of the 32-sample tiles
+    ctx->tile_groups_ready = false;  // the lane groups of the 32-sample tiles are built by their first user
     if (S > 0) {
         GVC_CUDA(morton_sort_points(ctx->s_sort, S, samples, st), "sample sort");
         const int64_t slots = ctx->n_tiles * kTile;
         GVC_CUDA(ctx->s_sorted.ensure(sizeof(float4) * slots), "alloc s_sorted");
-        // sorted samples only; the 32-sample lane groups and their LBVH are built by their
-        // first user (ensure_tile_groups / ensure_tile_lbvh)
+        // sorted samples only; the 32-sample lane groups are built by their first user
         GVC_CUDA(launch_sample_tiles(S, ctx->n_tiles, samples, ctx->s_sort.perm.as<int32_t>(),
                                      ctx->s_sort.keys.as<uint32_t>(), ctx->s_sorted.as<float4>(), nullptr, nullptr,
-                                     nullptr, false, st),
+                                     false, st),
                  "sample tiles");
         const int64_t n_blocks = (S + 127) / 128;
         GVC_CUDA(ctx->blk_desc.ensure(sizeof(uint2) * n_blocks), "alloc blk_desc");
@@ -531,53 +515,39 @@ int gvc_rasterize_gaussians_backward(gvc_ctx* ctx, int64_t P, const float* means
         GVC_CUDA(launch_preprocess(P, means3D, scales, rotations, weights, scale_modifier, nullptr, boxes, st),
                  "preprocess");
     }
+    (void)use_gaussian_bvh;  // both reference modes sum over the same pairs
     GVC_CUDA(sc->gacc.ensure(sizeof(float) * 16 * P), "alloc gacc");
     float* gacc = sc->gacc.as<float>();
-    // mode 3, or the tensor-core path in auto mode: reduction over samples on tcgen05
+    // mode 3, or the tensor-core path in auto mode: reduction over samples on tcgen05; every
+    // other mode: the Gaussian-owned sums
     const bool tc_bwd = ctx->bwd_mode == 3 || (ctx->bwd_mode == 0 && ctx->eval_path == 1);
-    const bool atomic_mode = ctx->bwd_mode == 2 || (ctx->bwd_mode == 0 && use_gaussian_bvh);
     const bool have_order = ctx->gauss_ready && ctx->P == P;
     if (ctx->n_tiles == 0) {
         GVC_CUDA(cudaMemsetAsync(gacc, 0, sizeof(float) * 16 * P, st), "zero gacc");
+        tm.mark();
     } else {
-        const int64_t slots = ctx->n_tiles * kTile;
-        GVC_CUDA(ctx->s_grad.ensure(sizeof(float4) * slots), "alloc s_grad");
-        GVC_CUDA(ctx->s_gyz.ensure(sizeof(float) * slots), "alloc s_gyz");
-        GVC_CUDA(ctx->s_ok.ensure(slots), "alloc s_ok");
         // the forward's sorted copy of (out, W) when these are the arrays it wrote
         const bool same_out = ctx->fwd_sorted_ready && have_order && out_cells == ctx->fwd_out_cells &&
                               out_weights == ctx->fwd_out_weights;
-        GVC_CUDA(launch_sample_grads(slots, ctx->s_sorted.as<float4>(),
-                                     same_out ? ctx->fwd_sorted.as<float2>() : nullptr, out_cells, out_weights,
-                                     dL_dout_cells, dL_dout_weights, ctx->s_grad.as<float4>(), ctx->s_gyz.as<float>(),
-                                     ctx->s_ok.as<uint8_t>(), st),
-                 "sample grads");
+        const float2* out_sorted = same_out ? ctx->fwd_sorted.as<float2>() : nullptr;
         BwdArgs ba{};
         ba.P = P;
-        ba.means = means3D;
-        ba.values = values;
-        ba.weights = weights;
         ba.conics = conics;
         ba.boxes = boxes;
-        ba.s_sorted = ctx->s_sorted.as<float4>();
-        ba.s_grad = ctx->s_grad.as<float4>();
-        ba.s_gyz = ctx->s_gyz.as<float>();
-        ba.s_ok = ctx->s_ok.as<uint8_t>();
-        if (!tc_bwd) {
-            // the deterministic reduction walks the sample groups; the atomic one uses their boxes
-            const int rc = atomic_mode ? ensure_tile_groups(ctx, st) : ensure_tile_lbvh(ctx, st);
-            if (rc != GVC_OK) return rc;
-        }
-        ba.tile_boxes = ctx->tile_boxes.as<float4>();
-        ba.gdesc = ctx->tile_gdesc.as<uint32_t>();
-        ba.n_tiles = ctx->n_tiles;
-        ba.tnodes = ctx->tiles.nodes.as<BvhNode>();
         ba.gacc = gacc;
         ba.status = ctx->d_status;
         ba.stats = ctx->d_stats;
         ba.count = ctx->count_pairs != 0;
-        tm.mark();
         if (tc_bwd) {
+            const int64_t slots = ctx->n_tiles * kTile;
+            GVC_CUDA(ctx->s_grad.ensure(sizeof(float4) * slots), "alloc s_grad");
+            GVC_CUDA(ctx->s_gyz.ensure(sizeof(float) * slots), "alloc s_gyz");
+            GVC_CUDA(ctx->s_ok.ensure(slots), "alloc s_ok");
+            GVC_CUDA(launch_sample_grads(slots, ctx->s_sorted.as<float4>(), out_sorted, out_cells, out_weights,
+                                         dL_dout_cells, dL_dout_weights, ctx->s_grad.as<float4>(),
+                                         ctx->s_gyz.as<float>(), ctx->s_ok.as<uint8_t>(), st),
+                     "sample grads");
+            tm.mark();
             if (!have_order) GVC_CUDA(lbvh_build_boxes(ctx->gbvh, P, boxes, st), "Gaussian LBVH");
             if (!same_gauss) {
                 GVC_CUDA(ctx->grec.ensure(sizeof(GaussRec) * P), "alloc records");
@@ -586,8 +556,11 @@ int gvc_rasterize_gaussians_backward(gvc_ctx* ctx, int64_t P, const float* means
                          "gather records");
             }
             GVC_CUDA(cudaMemsetAsync(gacc, 0, sizeof(float) * 16 * P, st), "zero gacc");
-            ba.gorder = nullptr;
             ba.gperm = ctx->gbvh.perm.as<int32_t>();
+            ba.n_slots = slots;
+            ba.s_grad = ctx->s_grad.as<float4>();
+            ba.s_gyz = ctx->s_gyz.as<float>();
+            ba.s_ok = ctx->s_ok.as<uint8_t>();
             ba.gnodes = ctx->gbvh.nodes.as<BvhNode>();
             ba.g_internal = ctx->gbvh.n > 1 ? ctx->gbvh.n - 1 : 1;
             ba.stackless = ctx->traversal == 1;
@@ -614,29 +587,22 @@ int gvc_rasterize_gaussians_backward(gvc_ctx* ctx, int64_t P, const float* means
             const float4* bboxes = ctx->blk_boxes_b.as<float4>();
             GVC_CUDA(launch_backward_cta(ba, n_blocks, bdesc, bboxes, st), "backward (tensor core)");
             timer_end(ctx, st, tk);
-        } else if (atomic_mode) {
-            if (!have_order) GVC_CUDA(lbvh_build_boxes(ctx->gbvh, P, boxes, st), "Gaussian LBVH");
-            if (!same_gauss) {
-                GVC_CUDA(ctx->grec.ensure(sizeof(GaussRec) * P), "alloc records");
-                GVC_CUDA(launch_gather_recs(P, ctx->gbvh.perm.as<int32_t>(), means3D, values, weights, conics,
-                                            boxes, ctx->grec.as<GaussRec>(), st),
-                         "gather records");
-            }
-            GVC_CUDA(cudaMemsetAsync(gacc, 0, sizeof(float) * 16 * P, st), "zero gacc");
-            ba.gorder = nullptr;
-            ba.gperm = ctx->gbvh.perm.as<int32_t>();
-            ba.gnodes = ctx->gbvh.nodes.as<BvhNode>();
-            ba.recs = ctx->grec.as<GaussRec>();
-            const int tk = timer_begin(ctx, st, 1);
-            GVC_CUDA(launch_backward_tiles(ba, st), "backward (atomic)");
-            timer_end(ctx, st, tk);
         } else {
+            const SampleTreeSize z = sample_tree_size(S);
+            GVC_CUDA(ctx->b_rows.ensure(z.rows_bytes), "alloc gradient rows");
+            GVC_CUDA(ctx->b_boxes.ensure(sizeof(float4) * 2 * z.boxes), "alloc sample tree");
+            SampleTree tree;
+            GVC_CUDA(launch_backward_rows(S, z, ctx->s_sorted.as<float4>(), out_sorted, out_cells, out_weights,
+                                          dL_dout_cells, dL_dout_weights, ctx->b_rows.as<float>(),
+                                          ctx->b_boxes.as<float4>(), &tree, st),
+                     "gradient rows");
+            tm.mark();
             ba.gorder = have_order ? ctx->gbvh.perm.as<int32_t>() : nullptr;
-            ba.gperm = nullptr;
-            ba.gnodes = nullptr;
-            ba.recs = nullptr;
+            ba.means = means3D;
+            ba.values = values;
+            ba.weights = weights;
             const int tk = timer_begin(ctx, st, 1);
-            GVC_CUDA(launch_backward_gauss(ba, st), "backward (deterministic)");
+            GVC_CUDA(launch_backward_gauss(ba, tree, ctx->b_rows.as<float>(), st), "backward (Gaussian-owned)");
             timer_end(ctx, st, tk);
         }
     }

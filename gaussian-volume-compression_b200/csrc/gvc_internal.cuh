@@ -14,8 +14,7 @@ constexpr float kWeightCutoff = 1e-2f;
 constexpr float kPowerFloor = -14.0f;
 // Tile of Morton-sorted samples handled by one warp.
 constexpr int kTile = 32;
-// Each tile is split into at most this many lane groups at Morton-order jumps; the
-// sample-side LBVH has one leaf slot per (tile, group).
+// Each tile is split into at most this many lane groups at Morton-order jumps.
 constexpr int kGroups = 4;
 // Per-warp traversal stack (entries of int32) in shared memory.
 constexpr int kStackCap = 512;
@@ -136,7 +135,6 @@ struct gvc_ctx {
     bool fwd_recs_ready = false;
     gvc::DevBuf s_sorted;   // [n_tiles*32] float4 (x, y, z, bits of caller index or -1)
     gvc::DevBuf tile_boxes; // [n_tiles * kGroups] group boxes, 2 x float4 (empty for unused slots)
-    gvc::DevBuf tile_keys;  // [n_tiles * kGroups] uint32 Morton key of each group's first sample
     gvc::DevBuf tile_gdesc; // [n_tiles] group starts: bytes 0..2 = start lane of groups 1..3
                             // (32 if unused), byte 3 = number of groups
     gvc::DevBuf blk_desc;   // [ceil(S/128)] uint2 block-group descriptors (CTA kernels)
@@ -144,13 +142,13 @@ struct gvc_ctx {
     gvc::DevBuf blk_desc_b;   // the same with the backward's finer split (built on first use)
     gvc::DevBuf blk_boxes_b;
     bool blk_b_ready = false;
-    bool tiles_ready = false;        // sample-group LBVH built for the current samples
     bool tile_groups_ready = false;  // tile lane groups built for the current samples
     gvc::DevBuf s_grad;     // [n_tiles*32] float4 (x, y, z, gx) backward sample records
     gvc::DevBuf s_gyz;      // [n_tiles*32] float gyz (see k_sample_grads)
     gvc::DevBuf s_ok;       // [n_tiles*32] uint8 1 iff W > 0.01 (pair statistics only)
     gvc::Lbvh s_sort;       // sample sort (keys/perm only)
-    gvc::Lbvh tiles;        // tile LBVH
+    gvc::DevBuf b_rows;     // gradient rows in chunks of 16 (Gaussian-owned backward, bwd_gauss.cu)
+    gvc::DevBuf b_boxes;    // boxes of the chunks and of the levels above them
     // Gaussian state (forward)
     int64_t P = 0;
     bool gauss_ready = false;

@@ -170,9 +170,8 @@ __global__ void __launch_bounds__(256) k_gather_recs(int64_t P, const int32_t* _
 // most kGroups contiguous lane groups: a group [a, b) is split at the Morton bit where
 // its first and last keys first differ when both halves' boxes are at most half the
 // group's size (half-perimeter).  A tile that straddles a jump of the Z-order curve thus
-// becomes compact groups instead of one box spanning the jump.  Writes one box and
-// key per group slot (unused slots: empty box, key of the last sample) and the group
-// descriptor of the tile.
+// becomes compact groups instead of one box spanning the jump.  Writes one box per group
+// slot (unused slots: empty box) and the group descriptor of the tile.
 struct WBox {
     float lx, ly, lz, hx, hy, hz;
 };
@@ -224,8 +223,8 @@ __device__ int try_split(int a, int b, uint32_t key, int lane, float x, float y,
 __global__ void __launch_bounds__(256) k_sample_tiles(int64_t S, int64_t n_tiles, const float* __restrict__ samples,
                                                       const int32_t* __restrict__ perm,
                                                       const uint32_t* __restrict__ skeys, float4* __restrict__ s_sorted,
-                                                      float4* __restrict__ group_boxes, uint32_t* __restrict__ group_keys,
-                                                      uint32_t* __restrict__ gdesc, int with_groups) {
+                                                      float4* __restrict__ group_boxes, uint32_t* __restrict__ gdesc,
+                                                      int with_groups) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t t = i >> 5;
     if (t >= n_tiles) return;
@@ -264,14 +263,11 @@ __global__ void __launch_bounds__(256) k_sample_tiles(int64_t S, int64_t n_tiles
         if (m2 >= 0) starts[ng++] = m2;
     }
     for (int g = ng; g <= kGroups; g++) starts[g] = 32;
-    const uint32_t last_key = __shfl_sync(0xffffffffu, key, nvalid - 1);
     for (int g = 0; g < kGroups; g++) {
         const int a = starts[g], b = (g + 1 < ng) ? starts[g + 1] : nvalid;
         WBox B;
-        uint32_t k = last_key;
         if (g < ng) {
             B = warp_box(lane >= a && lane < b, x, y, z);
-            k = __shfl_sync(0xffffffffu, key, a);
         } else {
             B.lx = B.ly = B.lz = INFINITY;
             B.hx = B.hy = B.hz = -INFINITY;
@@ -279,7 +275,6 @@ __global__ void __launch_bounds__(256) k_sample_tiles(int64_t S, int64_t n_tiles
         if (lane == 0) {
             group_boxes[2 * (kGroups * t + g)] = make_float4(B.lx, B.ly, B.lz, 0.f);
             group_boxes[2 * (kGroups * t + g) + 1] = make_float4(B.hx, B.hy, B.hz, 0.f);
-            group_keys[kGroups * t + g] = k;
         }
     }
     if (lane == 0)
@@ -343,11 +338,11 @@ cudaError_t launch_gather_recs(int64_t P, const int32_t* perm, const float* mean
 }
 
 cudaError_t launch_sample_tiles(int64_t S, int64_t n_tiles, const float* samples, const int32_t* perm,
-                                const uint32_t* skeys, float4* s_sorted, float4* group_boxes, uint32_t* group_keys,
-                                uint32_t* gdesc, bool with_groups, cudaStream_t st) {
+                                const uint32_t* skeys, float4* s_sorted, float4* group_boxes, uint32_t* gdesc,
+                                bool with_groups, cudaStream_t st) {
     if (n_tiles <= 0) return cudaSuccess;
     k_sample_tiles<<<nb256(n_tiles * 32), 256, 0, st>>>(S, n_tiles, samples, perm, skeys, s_sorted, group_boxes,
-                                                        group_keys, gdesc, with_groups ? 1 : 0); gvc::note_launch();
+                                                        gdesc, with_groups ? 1 : 0); gvc::note_launch();
     return cudaGetLastError();
 }
 

@@ -1,23 +1,16 @@
-// render.cu -- fused traversal + Gaussian evaluation (forward) and the adjoint
-// (backward) of the mixture field at Morton-sorted sample tiles.
+// render.cu -- fused traversal + Gaussian evaluation of the mixture field at 32-sample
+// tiles (forward), and the per-Gaussian end of the backward.
 //
-// Forward (replaces FORWARD::sampleRenderCUDA / renderCUDA + normalizeCUDA,
+// Forward per tile (replaces FORWARD::sampleRenderCUDA / renderCUDA + normalizeCUDA,
 // diff-gaussian-rasterization/cuda_rasterizer/forward.cu:116-274): one warp per tile of
 // 32 Morton-sorted samples walks the Gaussian LBVH with the tile's box; candidate
 // Gaussians are staged 32 at a time in shared memory and every lane evaluates its own
 // sample against each of them, accumulating W and V in registers (no atomics).
 //
-// Backward, deterministic (replaces BACKWARD::renderCUDA, backward.cu:127-337): one
-// warp per Gaussian walks the sample-group LBVH with the Gaussian's AABB; the rows of the
-// candidate groups are packed densely onto the lanes; per-lane partial moments are
-// reduced once per Gaussian (a fixed-order segmented reduction, no atomics).
+// k_finalize turns the backward's eleven sums per Gaussian (bwd_gauss.cu, bwd_tc.cu) into
+// the gradients of its parameters (backward.cu:9-125).
 //
-// Backward, atomic (replaces BACKWARD::sampleRenderCUDA, backward.cu:339-559): one warp
-// per sample tile re-walks the Gaussian LBVH; the 11 per-pair terms are pre-reduced over
-// the tile with 16 shuffles and added with one FP32 atomic per field and Gaussian.
-//
-// Pair math follows forward.cu:224-256 and backward.cu:252-298; the per-sample factors
-// 1/W, -out/W are folded into the sample record once per sample.
+// Pair math follows forward.cu:224-256.
 #include "pair.cuh"
 #include "render.cuh"
 #include "traverse.cuh"
@@ -149,267 +142,6 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) k_forward(const float4* _
             atomicMax(&stats[3], (unsigned long long)tc.max_sp);
             atomicAdd(&stats[5], (unsigned long long)tc.leaves);
             atomicAdd(&stats[6], (unsigned long long)tc.nodes);
-        }
-    }
-}
-
-// --------------------------------------------------------------------------------
-// Backward, deterministic Gaussian-owned reduction with densely packed sample rows.
-// --------------------------------------------------------------------------------
-// A candidate leaf is one lane group of a sample tile (rows [start, end) of the tile).
-// Groups hold 1..32 rows, so mapping lanes to a group's rows leaves lanes idle; instead
-// the rows of successive candidate groups are appended to a per-warp ring and evaluated
-// kFlush at a time (kRowsPerLane rows per lane, all loads issued before the arithmetic:
-// the kernel is bound by the latency of these gathers).  The order in which rows reach
-// lanes depends only on the traversal order, so the sums are deterministic.
-constexpr int kRowsPerLane = 2;
-constexpr int kFlush = 32 * kRowsPerLane;  // rows per evaluation
-constexpr int kRing = 2 * kFlush;          // queued rows stay below kFlush + 32
-
-template <bool COUNT>
-struct BwdDenseVisitor {
-    const float4* __restrict__ s_grad;
-    const float* __restrict__ s_gyz;
-    const uint8_t* __restrict__ s_ok;
-    const uint32_t* __restrict__ gdesc;
-    int* ring;     // shared [kRing]
-    int4* leaves;  // shared [32]: (first slot of tile, start lane, end lane, rows queued through this leaf)
-    uint32_t head, tail;
-    GaussB g;
-    float m[11];
-    int npairs;
-    int nrows;  // rows evaluated (warp-uniform, statistics)
-
-    // evaluates the n (1..kFlush) rows at the ring head
-    __device__ __forceinline__ void eval(int n) {
-        const int lane = threadIdx.x & 31;
-        float4 p[kRowsPerLane];
-        float y[kRowsPerLane];
-        int r[kRowsPerLane];
-#pragma unroll
-        for (int k = 0; k < kRowsPerLane; k++) {
-            p[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-            y[k] = 0.f;
-            r[k] = -1;
-            if (lane + 32 * k < n) {
-                r[k] = ring[(head + (uint32_t)(32 * k + lane)) & (kRing - 1)];
-                p[k] = __ldg(s_grad + r[k]);
-                y[k] = __ldg(s_gyz + r[k]);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < kRowsPerLane; k++) {
-            if (32 * k < n) {
-                const bool c = pair_moments(g, p[k], y[k], m);
-                if (COUNT && c && r[k] >= 0 && s_ok[r[k]]) npairs++;
-            }
-        }
-        if (COUNT) nrows += n;
-        head += (uint32_t)n;
-    }
-
-    __device__ __forceinline__ void operator()(const int* c, int nb) {
-        const int lane = threadIdx.x & 31;
-        int sz = 0;
-        int4 L = make_int4(0, 0, 0, 0);
-        if (lane < nb) {
-            const int leaf = c[lane];
-            const int t = leaf >> 2;  // leaf = tile * kGroups + group
-            const int gi = leaf & 3;
-            const uint32_t gd = __ldg(gdesc + t);
-            const int start = gi == 0 ? 0 : (int)((gd >> (8 * (gi - 1))) & 0xffu);
-            const int end = gi < 3 ? (int)((gd >> (8 * gi)) & 0xffu) : 32;
-            sz = end - start;
-            L = make_int4(t * 32, start, end, 0);
-        }
-        int incl = sz;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, off);
-            if (lane >= off) incl += v;
-        }
-        L.w = incl;
-        leaves[lane] = L;
-        __syncwarp();
-        const uint32_t base = tail;
-        for (int j = 0; j < nb; j++) {
-            const int4 q = leaves[j];
-            const int excl = q.w - (q.z - q.y);
-            if (lane >= q.y && lane < q.z) ring[(base + (uint32_t)(excl + lane - q.y)) & (kRing - 1)] = q.x + lane;
-            if (base + (uint32_t)q.w - head >= (uint32_t)kFlush) {
-                __syncwarp();
-                eval(kFlush);
-            }
-        }
-        tail = base + (uint32_t)__shfl_sync(0xffffffffu, incl, 31);
-        __syncwarp();
-    }
-
-    __device__ __forceinline__ void drain() {
-        while (tail != head) {
-            __syncwarp();
-            const uint32_t n = tail - head;
-            eval(n < (uint32_t)kFlush ? (int)n : kFlush);
-        }
-        __syncwarp();
-    }
-};
-
-// Warps (consecutive Gaussians in Morton order) per block: neighbouring Gaussians gather
-// overlapping sample rows, which then hit in the SM's L1.
-constexpr int kBwdWarps = 4;
-
-template <bool COUNT>
-__global__ void __launch_bounds__(kBwdWarps * 32) k_backward_gauss(
-    int P, const int32_t* __restrict__ gorder, const float* __restrict__ means, const float* __restrict__ values,
-    const float* __restrict__ weights, const float* __restrict__ conics, const float4* __restrict__ boxes,
-    const float4* __restrict__ s_grad, const float* __restrict__ s_gyz, const uint8_t* __restrict__ s_ok,
-    const uint32_t* __restrict__ gdesc, const BvhNode* __restrict__ tnodes, float* __restrict__ gacc, int* status,
-    unsigned long long* stats) {
-    __shared__ int s_stack[kBwdWarps][kStackCap];
-    __shared__ int s_cand[kBwdWarps][kCandCap];
-    __shared__ int s_ring[kBwdWarps][kRing];
-    __shared__ int4 s_leaves[kBwdWarps][32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int gi = blockIdx.x * kBwdWarps + warp;
-    if (gi >= P) return;
-    const int64_t o = gorder ? gorder[gi] : gi;
-    BwdDenseVisitor<COUNT> vis;
-    vis.s_grad = s_grad;
-    vis.s_gyz = s_gyz;
-    vis.s_ok = s_ok;
-    vis.gdesc = gdesc;
-    vis.ring = s_ring[warp];
-    vis.leaves = s_leaves[warp];
-    vis.head = vis.tail = 0u;
-    const float* cp = conics + 6 * o;
-    const float4 lo = __ldg(boxes + 2 * o), hi = __ldg(boxes + 2 * o + 1);
-    vis.g = gauss_b(__ldg(means + 3 * o), __ldg(means + 3 * o + 1), __ldg(means + 3 * o + 2), __ldg(values + o),
-                    __ldg(cp), __ldg(cp + 1), __ldg(cp + 2), __ldg(cp + 3), __ldg(cp + 4), __ldg(cp + 5), lo, hi);
-#pragma unroll
-    for (int k = 0; k < 11; k++) vis.m[k] = 0.f;
-    vis.npairs = 0;
-    vis.nrows = 0;
-    TravCount tc;
-    const int st = warp_traverse(tnodes, make_float3(lo.x, lo.y, lo.z), make_float3(hi.x, hi.y, hi.z), s_stack[warp],
-                                 s_cand[warp], vis, tc);
-    vis.drain();
-    float v16[16];
-#pragma unroll
-    for (int k = 0; k < 16; k++) v16[k] = k < 11 ? vis.m[k] : 0.f;
-    const float tot = warp_transpose_reduce16(v16);
-    const float term = moments_to_terms(tot, __ldg(weights + o), __ldg(cp), __ldg(cp + 1), __ldg(cp + 2),
-                                        __ldg(cp + 3), __ldg(cp + 4), __ldg(cp + 5));
-    if (!(lane & 1)) gacc[16 * o + (lane >> 1)] = term;
-    if (st && lane == 0) atomicOr(status, st);
-    if (COUNT) {
-        unsigned long long a = (unsigned long long)vis.npairs;
-        for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
-        if (lane == 0) {
-            atomicAdd(&stats[2], a);
-            atomicMax(&stats[4], (unsigned long long)tc.max_sp);
-            atomicAdd(&stats[7], (unsigned long long)tc.leaves);
-            atomicAdd(&stats[8], (unsigned long long)tc.nodes);
-            atomicAdd(&stats[10], (unsigned long long)vis.nrows);
-        }
-    }
-}
-
-// --------------------------------------------------------------------------------
-// Backward, sample-tile traversal with warp pre-reduction + FP32 atomics.
-// --------------------------------------------------------------------------------
-struct BwdTileVisitor {
-    const GaussRec* __restrict__ recs;
-    const int32_t* __restrict__ gperm;
-    float4* batch;  // shared [32 * 5]
-    float4 p;       // (x, y, z, gx); gx = 0 outside the current group
-    float gyz;      // 0 outside the current group
-    bool act;       // lane in the current group
-    bool ok;
-    float* __restrict__ gacc;
-    int npairs;
-
-    __device__ __forceinline__ void operator()(const int* c, int nb) {
-        const int lane = threadIdx.x & 31;
-        if (lane < nb) {
-            const float4* rp = reinterpret_cast<const float4*>(recs + c[lane]);
-            batch[lane * 5 + 0] = __ldg(rp);
-            batch[lane * 5 + 1] = __ldg(rp + 1);
-            batch[lane * 5 + 2] = __ldg(rp + 2);
-            batch[lane * 5 + 3] = __ldg(rp + 3);
-            batch[lane * 5 + 4] = __ldg(rp + 4);
-        }
-        __syncwarp();
-        for (int gi = 0; gi < nb; gi++) {
-            const float4 r0 = batch[gi * 5 + 0], r1 = batch[gi * 5 + 1], r2 = batch[gi * 5 + 2];
-            const GaussB g = gauss_b(r0.x, r0.y, r0.z, r2.z, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, batch[gi * 5 + 3],
-                                     batch[gi * 5 + 4]);
-            float m[11];
-#pragma unroll
-            for (int k = 0; k < 11; k++) m[k] = 0.f;
-            const bool hit = pair_moments(g, p, gyz, m) && act;
-            if (!__any_sync(0xffffffffu, hit)) continue;
-            npairs += (hit && ok) ? 1 : 0;
-            float v16[16];
-#pragma unroll
-            for (int k = 0; k < 16; k++) v16[k] = k < 11 ? m[k] : 0.f;
-            const float tot = warp_transpose_reduce16(v16);
-            const float term = moments_to_terms(tot, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y);
-            const int k = lane >> 1;
-            if (!(lane & 1) && k < 11) {
-                const int o = gperm[c[gi]];
-                atomicAdd(gacc + 16 * (int64_t)o + k, term);
-            }
-        }
-        __syncwarp();
-    }
-};
-
-template <bool COUNT>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) k_backward_tiles(
-    const float4* __restrict__ s_grad, const float* __restrict__ s_gyz, const uint8_t* __restrict__ s_ok,
-    const float4* __restrict__ group_boxes, const uint32_t* __restrict__ gdesc, int n_tiles,
-    const BvhNode* __restrict__ gnodes, const GaussRec* __restrict__ recs, const int32_t* __restrict__ gperm,
-    float* __restrict__ gacc, int* status, unsigned long long* stats) {
-    __shared__ int s_stack[kWarpsPerBlock][kStackCap];
-    __shared__ int s_cand[kWarpsPerBlock][kCandCap];
-    __shared__ float4 s_batch[kWarpsPerBlock][32 * 5];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tile = blockIdx.x * kWarpsPerBlock + warp;
-    if (tile >= n_tiles) return;
-    BwdTileVisitor vis;
-    vis.recs = recs;
-    vis.gperm = gperm;
-    vis.batch = s_batch[warp];
-    const int64_t slot = (int64_t)tile * 32 + lane;
-    const float4 sp = s_grad[slot];
-    const float syz = s_gyz[slot];
-    vis.ok = s_ok[slot] != 0;
-    vis.gacc = gacc;
-    vis.npairs = 0;
-    const uint32_t gd = gdesc[tile];
-    const int ng = (int)(gd >> 24), mygroup = lane_group(gd, lane);
-    TravCount tc;
-    int st = 0;
-    for (int g = 0; g < ng; g++) {
-        const int64_t gslot = (int64_t)tile * kGroups + g;
-        const float4 tlo = group_boxes[2 * gslot], thi = group_boxes[2 * gslot + 1];
-        // lanes outside the group carry zero gradients and are not counted
-        vis.act = mygroup == g;
-        vis.p = make_float4(sp.x, sp.y, sp.z, vis.act ? sp.w : 0.f);
-        vis.gyz = vis.act ? syz : 0.f;
-        st |= warp_traverse(gnodes, make_float3(tlo.x, tlo.y, tlo.z), make_float3(thi.x, thi.y, thi.z),
-                            s_stack[warp], s_cand[warp], vis, tc);
-    }
-    if (st && lane == 0) atomicOr(status, st);
-    if (COUNT) {
-        unsigned long long a = (unsigned long long)vis.npairs;
-        for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
-        if (lane == 0) {
-            atomicAdd(&stats[2], a);
-            atomicMax(&stats[4], (unsigned long long)tc.max_sp);
-            atomicAdd(&stats[7], (unsigned long long)tc.leaves);
-            atomicAdd(&stats[8], (unsigned long long)tc.nodes);
         }
     }
 }
@@ -578,36 +310,6 @@ cudaError_t launch_forward(const FwdArgs& a, cudaStream_t st) {
         k_forward<false><<<nblk(a.n_tiles, kWarpsPerBlock), kWarpsPerBlock * 32, 0, st>>>(
             a.s_sorted, a.tile_boxes, a.gdesc, (int)a.n_tiles, a.gnodes, a.recs, a.out_cells, a.out_weights, a.status,
             a.stats);
-    }
-    gvc::note_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t launch_backward_gauss(const BwdArgs& a, cudaStream_t st) {
-    if (a.P <= 0) return cudaSuccess;
-    if (a.count) {
-        k_backward_gauss<true><<<nblk(a.P, kBwdWarps), kBwdWarps * 32, 0, st>>>(
-            (int)a.P, a.gorder, a.means, a.values, a.weights, a.conics, a.boxes, a.s_grad, a.s_gyz, a.s_ok, a.gdesc,
-            a.tnodes, a.gacc, a.status, a.stats);
-    } else {
-        k_backward_gauss<false><<<nblk(a.P, kBwdWarps), kBwdWarps * 32, 0, st>>>(
-            (int)a.P, a.gorder, a.means, a.values, a.weights, a.conics, a.boxes, a.s_grad, a.s_gyz, a.s_ok, a.gdesc,
-            a.tnodes, a.gacc, a.status, a.stats);
-    }
-    gvc::note_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t launch_backward_tiles(const BwdArgs& a, cudaStream_t st) {
-    if (a.n_tiles <= 0) return cudaSuccess;
-    if (a.count) {
-        k_backward_tiles<true><<<nblk(a.n_tiles, kWarpsPerBlock), kWarpsPerBlock * 32, 0, st>>>(
-            a.s_grad, a.s_gyz, a.s_ok, a.tile_boxes, a.gdesc, (int)a.n_tiles, a.gnodes, a.recs, a.gperm, a.gacc,
-            a.status, a.stats);
-    } else {
-        k_backward_tiles<false><<<nblk(a.n_tiles, kWarpsPerBlock), kWarpsPerBlock * 32, 0, st>>>(
-            a.s_grad, a.s_gyz, a.s_ok, a.tile_boxes, a.gdesc, (int)a.n_tiles, a.gnodes, a.recs, a.gperm, a.gacc,
-            a.status, a.stats);
     }
     gvc::note_launch();
     return cudaGetLastError();

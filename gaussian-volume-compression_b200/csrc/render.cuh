@@ -21,29 +21,27 @@ struct FwdArgs {
 
 struct BwdArgs {
     int64_t P;
-    const int32_t* gorder;  // processing order (sorted pos -> caller idx) or null
-    const int32_t* gperm;   // LBVH order -> caller idx (atomic mode)
+    const float4* boxes;       // caller order, lo/hi
+    const float* conics;
+    // Gaussian-owned sums
+    const int32_t* gorder;     // processing order (sorted pos -> caller idx) or null
     const float* means;
     const float* values;
     const float* weights;
-    const float* conics;
-    const float4* boxes;  // caller order, lo/hi
-    const float4* s_sorted;
+    // tensor-core sums
+    const int32_t* gperm;      // LBVH order -> caller idx
+    int64_t n_slots;           // sorted sample slots
     const float4* s_grad;      // (x, y, z, gx) per sorted slot
     const float* s_gyz;        // gyz per sorted slot
     const uint8_t* s_ok;       // W > 0.01 per sorted slot (pair statistics)
-    const float4* tile_boxes;  // group boxes [n_tiles * kGroups]
-    const uint32_t* gdesc;     // [n_tiles]
-    int64_t n_tiles;
-    const BvhNode* tnodes;  // sample-group LBVH
-    const BvhNode* gnodes;  // Gaussian LBVH (atomic and tensor-core modes)
-    int64_t g_internal;     // its internal nodes
-    bool stackless;         // tensor-core mode: traverse by escape edges (warp_traverse_stackless)
-    const int32_t* clog;    // tensor-core mode: the forward's candidate log (null: traverse)
+    const BvhNode* gnodes;     // Gaussian LBVH
+    int64_t g_internal;        // its internal nodes
+    bool stackless;            // traverse by escape edges (warp_traverse_stackless)
+    const int32_t* clog;       // the forward's candidate log (null: traverse)
     const int32_t* cend;
-    const uint2* cdesc;     // the forward's block groups (the log's groups)
-    const GaussRec* recs;   // LBVH order (atomic mode)
-    float* gacc;            // [P][16] caller order
+    const uint2* cdesc;        // the forward's block groups (the log's groups)
+    const GaussRec* recs;      // LBVH order
+    float* gacc;               // [P][16] caller order
     int* status;
     unsigned long long* stats;
     bool count;
@@ -118,11 +116,37 @@ cudaError_t launch_tc_gemm_test(const void* A, const void* B, int N, float* D, i
 // One block waiting on an mbarrier nothing arrives on: the bounded wait runs out and
 // records kStatusTimeout (tests the host-side report of device timeouts).
 cudaError_t launch_wait_timeout_test(int* status, cudaStream_t st);
-cudaError_t launch_backward_gauss(const BwdArgs& a, cudaStream_t st);
+
+// bwd_gauss.cu: gradient rows in chunks of 16, a tree of boxes over them (level 0: chunks,
+// level 1: 8 chunks, every further level: 32 children per node), and the Gaussian-owned
+// sums that walk it
+constexpr int kChunkRows = 16;
+constexpr int kChunkFloats = 5 * kChunkRows;  // x, y, z, gx, gyz
+constexpr int kNodeChunks = 8;                // chunks of a level-1 node
+constexpr int kNodeRows = kNodeChunks * kChunkRows;
+constexpr int kTreeLevels = 6;
+struct SampleTree {
+    const float4* box[kTreeLevels];  // per level: (lo, hi) of each node
+    int n[kTreeLevels];
+    int top;
+};
+struct SampleTreeSize {
+    int64_t n[kTreeLevels];
+    int top;
+    int64_t boxes;      // all levels together
+    size_t rows_bytes;  // gradient rows
+};
+SampleTreeSize sample_tree_size(int64_t S);
+// out_sorted: the forward's (out, W) per sorted slot when the caller's out_cells /
+// out_weights are that forward's outputs (else null: they are gathered).
+cudaError_t launch_backward_rows(int64_t S, const SampleTreeSize& z, const float4* s_sorted, const float2* out_sorted,
+                                 const float* out_cells, const float* out_weights, const float* gout, const float* gw,
+                                 float* rows, float4* boxes, SampleTree* tree, cudaStream_t st);
+cudaError_t launch_backward_gauss(const BwdArgs& a, const SampleTree& tree, const float* rows, cudaStream_t st);
+
 // bwd_tc.cu: backward on 128-sample blocks with the reduction over samples on tcgen05
 cudaError_t launch_backward_cta(const BwdArgs& a, int64_t n_blocks, const uint2* bdesc, const float4* bboxes,
                                 cudaStream_t st);
-cudaError_t launch_backward_tiles(const BwdArgs& a, cudaStream_t st);
 cudaError_t launch_finalize(int64_t P, const float* gacc, const float* scales, const float* rots, const float* conics,
                             float sm, int ref_compat, float* dmeans, float* dscales, float* drots, float* dvalues,
                             float* dweights, cudaStream_t st);
@@ -134,8 +158,8 @@ cudaError_t launch_gather_recs(int64_t P, const int32_t* perm, const float* mean
                                const float* weights, const float* conics, const float4* boxes, GaussRec* recs,
                                cudaStream_t st);
 cudaError_t launch_sample_tiles(int64_t S, int64_t n_tiles, const float* samples, const int32_t* perm,
-                                const uint32_t* skeys, float4* s_sorted, float4* group_boxes, uint32_t* group_keys,
-                                uint32_t* gdesc, bool with_groups, cudaStream_t st);
+                                const uint32_t* skeys, float4* s_sorted, float4* group_boxes, uint32_t* gdesc,
+                                bool with_groups, cudaStream_t st);
 // out_sorted: the forward's (out, W) per sorted slot when the caller's out_cells /
 // out_weights are that forward's outputs (else null: they are gathered).
 cudaError_t launch_sample_grads(int64_t n_slots, const float4* s_sorted, const float2* out_sorted,

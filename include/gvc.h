@@ -40,13 +40,12 @@ typedef enum {
     GVC_OPT_COV_GRAD = 1,   /* 0 = true gradient of the forward (default),
                                1 = reference-compatible formula of
                                    diff-gaussian-rasterization/cuda_rasterizer/backward.cu:50-124 */
-    GVC_OPT_BWD_MODE = 2,   /* 0 = follow use_gaussian_bvh (default):
-                                   use_gaussian_bvh == 0 -> Gaussian-owned segmented reduction
-                                   (deterministic, no atomics; mirrors backward.cu:127-337),
-                                   use_gaussian_bvh != 0 -> sample-tile traversal with warp
-                                   pre-reduction + FP32 atomics (mirrors backward.cu:339-559);
-                                   (with GVC_OPT_EVAL_PATH = 1: the tensor-core reduction, 3);
-                               1 = always deterministic, 2 = always sample-tile atomic,
+    GVC_OPT_BWD_MODE = 2,   /* 0 = Gaussian-owned sums (default: deterministic, no atomics;
+                                   stands for both backward.cu:127-337 and, with
+                                   use_gaussian_bvh, backward.cu:339-559), or with
+                                   GVC_OPT_EVAL_PATH = 1 the tensor-core reduction, 3;
+                               1, 2 = always the Gaussian-owned sums (2 named a sample-side
+                                   reduction with atomics, slower at every size),
                                3 = tensor core: per 128-sample block, the per-Gaussian sums
                                    over samples as a tcgen05 BF16 3-way split GEMM in TMEM,
                                    FP32 atomics (not bitwise reproducible)                  */
@@ -81,7 +80,8 @@ typedef enum {
 typedef struct {
     int64_t fwd_candidates;   /* (sample, Gaussian) pairs with the sample inside the AABB   */
     int64_t fwd_contributing; /* ... and -14 <= power <= 0                                  */
-    int64_t bwd_contributing; /* contributing pairs of samples with W > 0.01                */
+    int64_t bwd_contributing; /* contributing pairs of samples with W > 0.01 (Gaussian-owned
+                                 backward: of samples with a non-zero gradient)            */
     int32_t max_stack_fwd;    /* deepest traversal stack seen (entries)                     */
     int32_t max_stack_bwd;
     double fwd_kernel_ms;     /* summed duration of the forward evaluation kernel          */
@@ -90,8 +90,8 @@ typedef struct {
     int64_t bwd_kernel_calls;
     int64_t fwd_leaf_hits;    /* (tile, Gaussian) pairs evaluated by the forward            */
     int64_t fwd_node_visits;  /* internal LBVH nodes popped by the forward traversal        */
-    int64_t bwd_leaf_hits;    /* (Gaussian or tile) leaves evaluated by the backward        */
-    int64_t bwd_node_visits;
+    int64_t bwd_leaf_hits;    /* (group, Gaussian) or (16-row chunk, Gaussian) pairs evaluated */
+    int64_t bwd_node_visits;  /* LBVH nodes popped, or sample-tree boxes tested                */
     int64_t fwd_lane_evals;   /* (sample, Gaussian) lane slots the forward evaluated (CTA paths) */
     int64_t bwd_rows;         /* (sample, Gaussian) rows the deterministic backward evaluated   */
 } gvc_stats;
@@ -116,9 +116,9 @@ int gvc_sync_status(gvc_ctx* ctx, void* stream);
 /* Replaces BuildBVH (diff-gaussian-rasterization/ext.cu:28-65).
    samples: [S,3] float32.  The context keeps the POINTER: the caller keeps the buffer
    alive and unchanged until the next gvc_build_bvh (the reference keeps a tensor
-   reference, ext.cu:29).  Sorts the samples by a 30-bit Morton key, forms 32-sample
-   tiles and builds the tile LBVH (the reference's leaf threshold 257, ext.cu:51, has
-   no counterpart: tiles are 32 samples). */
+   reference, ext.cu:29).  Sorts the samples by a 30-bit Morton key and forms
+   blocks of 128 of them (the reference's leaf threshold 257, ext.cu:51, has no
+   counterpart). */
 int gvc_build_bvh(gvc_ctx* ctx, const float* samples, int64_t S, int debug, int use_gaussian_bvh, void* stream);
 
 /* Replaces RasterizeGaussiansCUDAWrapper / RasterizeGaussiansCUDA
