@@ -960,12 +960,11 @@ def run_ours(args):
         # (forward path, backward mode, traversal, candidate log): FP32 throughout, tensor cores
         # throughout, the FP32 forward with the tensor-core backward reduction, and (timed
         # only) that with the backward walking the tree again instead of reading the forward's
-        # candidate log, and with the stackless Gaussian-LBVH traversal in both kernels
+        # candidate log
         for name, path, bmode, trav, clog in (("plain", "plain", "auto", "stack", True),
                                               ("tensor_core", "tensor_core", "auto", "stack", True),
                                               ("plain_fwd_tc_bwd", "plain", "tensor_core", "stack", True),
-                                              ("walk", "plain", "tensor_core", "stack", False),
-                                              ("stackless", "plain", "tensor_core", "stackless", False)):
+                                              ("walk", "plain", "tensor_core", "stack", False)):
             _C.set_eval_path(path)
             _C.set_backward_mode(bmode)
             _C.set_traversal(trav)
@@ -982,7 +981,7 @@ def run_ours(args):
             b1.record(stream)
             torch.cuda.synchronize()
             pm = gvc_dist.max_over_ranks(b0.elapsed_time(b1) / args.steps, dev)
-            if name in ("walk", "stackless"):
+            if name == "walk":
                 paths_extra["plain_fwd_tc_bwd_%s_ms_per_step" % name] = pm
                 continue
             # one more step, outputs and gradients kept (untimed)
@@ -1024,9 +1023,7 @@ def run_ours(args):
                                  "plain_fwd_tc_bwd": "FP32 CTA forward + tcgen05 moment backward",
                                  "plain_fwd_tc_bwd_walk": "the same with the backward walking the Gaussian "
                                                           "LBVH again instead of reading the forward's "
-                                                          "candidate log",
-                                 "plain_fwd_tc_bwd_stackless": "the same walking in both kernels by the "
-                                                               "stackless traversal (escape edges)"},
+                                                          "candidate log"},
                        "fp64_error": fp64}
         tc_vs_plain.update(paths_extra)
 

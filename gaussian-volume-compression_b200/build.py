@@ -26,7 +26,10 @@ SOURCES = {
     "prep.cu": ["--fmad=false"],
     "mesh.cu": ["--fmad=false"],
     "noalloc.cu": [],
+    "wide_tree.cu": [],
     "cta.cu": [],
+    "fwd_blocks.cu": [],
+    "fwd_points.cu": [],
     "fwd_tc.cu": [],
     "bwd_tc.cu": [],
     "bwd_gauss.cu": [],

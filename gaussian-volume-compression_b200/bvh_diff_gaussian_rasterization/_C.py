@@ -191,22 +191,21 @@ def set_backward_mode(mode, device=None):
 
 
 def set_eval_path(path, device=None):
-    """Forward kernel: 'plain' (default: FP32, CTA per 128 samples), 'tensor_core'
-    (tcgen05 BF16 split exponent, same pipeline) or 'plain_tile' (FP32, warp per 32 samples)."""
+    """Forward kernel: 'plain' or 'plain_tile' (default: FP32) or 'tensor_core' (tcgen05 BF16
+    split exponent)."""
     set_option(_n.OPT_EVAL_PATH, {"plain": 0, "tensor_core": 1, "plain_tile": 2}[path], device)
 
 
 def set_traversal(kind, device=None):
-    """Gaussian-LBVH traversal of the block-group forwards and the tensor-core backward:
-    'stack' (default: warp-cooperative, shared-memory node stack) or 'stackless' (escape
-    edges, one subtree per lane below the levels that fit the warp).  Same candidates."""
+    """'stack' or 'stackless': accepted, without effect (the walk without a stack was slower at
+    every size)."""
     set_option(_n.OPT_TRAVERSAL, {"stack": 0, "stackless": 1}[kind], device)
 
 
 def set_candidate_log(on, device=None):
-    """With the tensor-core backward selected, the forward records each block's candidate
-    Gaussians and the backward reads them back instead of walking the tree again (on by
-    default; off: the backward walks the tree on its own, finer block groups)."""
+    """With the tensor-core backward selected, the forward records the candidates of each block
+    and the backward reads them back instead of walking the tree again (on by default;
+    off: the backward walks)."""
     set_option(_n.OPT_CAND_LOG, 1 if on else 0, device)
 
 

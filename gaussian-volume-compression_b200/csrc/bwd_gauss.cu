@@ -5,8 +5,8 @@
 // Rows.  k_backward_rows turns the Morton-sorted samples into gradient rows, stored by
 // chunks of 16: 16 x, 16 y, 16 z, 16 gx, 16 gyz (320 bytes), so that a lane reads two
 // neighbouring rows of each field as one float2.  The same kernel reduces the boxes of the
-// chunks (level 0) and of runs of 8 chunks (level 1); k_tree_up adds levels of 32 children each.  A row without a
-// gradient (W below the cutoff, or an upstream gradient of zero) adds nothing to any sum
+// chunks and of runs of 8 chunks, the lower levels of a wide tree (wide_tree.cuh).  A row
+// without a gradient (W below the cutoff, or an upstream gradient of zero) adds nothing to any sum
 // and is left out of the boxes.
 //
 // Sums.  A warp walks that tree with its Gaussian's AABB, 32 children per step:
@@ -27,47 +27,18 @@
 #include "cull.cuh"
 #include "pair.cuh"
 #include "render.cuh"
-#include "traverse.cuh"
+#include "wide_tree.cuh"
 
 namespace gvc {
 
 namespace {
 
 constexpr int kRowThreads = 256;   // k_backward_rows: four rows per thread, one level-1 node per warp
-constexpr int kGaussWarps = 4;     // warps per CTA: neighbours in Morton order share rows in L1
-// Resident CTAs per SM asked of the register allocator: 64 registers, 32 warps.  Packed
-// f32x2 arithmetic needs a quarter fewer instructions but 96 registers, and measured slower
-// (300k Gaussians x 2.1M samples: 2.67 against 2.56 ms before the shared walk).
-constexpr int kGaussMinCtas = 8;
+constexpr int kGaussMinWarps = 32;  // resident warps per SM asked of the register allocator
 constexpr int kFlushChunks = 4;    // chunks per evaluation
 constexpr int kChunkCap = 64;      // queued chunks: below kFlushChunks + 32
-constexpr int kNodeCap = 64;       // queued level-1 nodes: below 4 + 32
 constexpr int kUnionCap = 512;     // chunks listed for the Gaussians of one warp
 constexpr int kShare = 4;          // Gaussians of one warp where they share a walk
-
-struct MinMax {
-    float lx, ly, lz, hx, hy, hz;
-};
-
-__device__ __forceinline__ void grow(MinMax& b, const MinMax& o) {
-    b.lx = fminf(b.lx, o.lx);
-    b.ly = fminf(b.ly, o.ly);
-    b.lz = fminf(b.lz, o.lz);
-    b.hx = fmaxf(b.hx, o.hx);
-    b.hy = fmaxf(b.hy, o.hy);
-    b.hz = fmaxf(b.hz, o.hz);
-}
-
-__device__ __forceinline__ MinMax shfl_xor_box(const MinMax& b, int off) {
-    return MinMax{__shfl_xor_sync(0xffffffffu, b.lx, off), __shfl_xor_sync(0xffffffffu, b.ly, off),
-                  __shfl_xor_sync(0xffffffffu, b.lz, off), __shfl_xor_sync(0xffffffffu, b.hx, off),
-                  __shfl_xor_sync(0xffffffffu, b.hy, off), __shfl_xor_sync(0xffffffffu, b.hz, off)};
-}
-
-__device__ __forceinline__ void store_box(float4* dst, int64_t i, const MinMax& b) {
-    dst[2 * i] = make_float4(b.lx, b.ly, b.lz, 0.f);
-    dst[2 * i + 1] = make_float4(b.hx, b.hy, b.hz, 0.f);
-}
 
 // One warp per level-1 node: 128 sorted rows, four per lane.  Per row (x, y, z) and, where
 // W > 0.01, gx = dL/dout / W and gyz = -dL/dout * out / W + dL/dW (backward.cu:252-298 folds
@@ -81,9 +52,9 @@ __global__ void __launch_bounds__(kRowThreads) k_backward_rows(
     const int lane = threadIdx.x & 31;
     const int node = blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5);
     if (node >= n_nodes) return;  // warp-uniform
-    const int64_t r0 = (int64_t)node * kNodeRows + 4 * lane;
+    const int64_t r0 = (int64_t)node * kRowsPerNode + 4 * lane;
     float x[4], y[4], z[4], gx[4], gyz[4];
-    MinMax b{INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    Box6 b = empty_box();
     float4 sp[4];
 #pragma unroll
     for (int k = 0; k < 4; k++)
@@ -103,7 +74,7 @@ __global__ void __launch_bounds__(kRowThreads) k_backward_rows(
                 gyz[k] = __fadd_rn(__fdiv_rn(-__fmul_rn(g, ow.x), ow.y), gw[o]);
             }
         }
-        if (!(gx[k] == 0.f && gyz[k] == 0.f)) grow(b, MinMax{x[k], y[k], z[k], x[k], y[k], z[k]});
+        if (!(gx[k] == 0.f && gyz[k] == 0.f)) grow(b, Box6{x[k], y[k], z[k], x[k], y[k], z[k]});
     }
     float4* dst = reinterpret_cast<float4*>(rows + (r0 / kChunkRows) * kChunkFloats) + (lane & 3);
     dst[0] = make_float4(x[0], x[1], x[2], x[3]);
@@ -120,94 +91,11 @@ __global__ void __launch_bounds__(kRowThreads) k_backward_rows(
     if (lane == 0) store_box(level1, node, b);
 }
 
-// One warp per node: the box of its up to 32 children.
-__global__ void __launch_bounds__(256) k_tree_up(int n_child, const float4* __restrict__ child, int n_node,
-                                                 float4* __restrict__ node) {
-    const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (i >= n_node) return;
-    MinMax b{INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    const int c = 32 * i + lane;
-    if (c < n_child) {
-        const float4 lo = child[2 * (int64_t)c], hi = child[2 * (int64_t)c + 1];
-        b = MinMax{lo.x, lo.y, lo.z, hi.x, hi.y, hi.z};
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) grow(b, shfl_xor_box(b, off));
-    if (lane == 0) store_box(node, i, b);
-}
-
-
-
-// Tests the children [first, first + 32) of a level above 0 against a box: lane i tests
-// first + i.
-__device__ __forceinline__ uint32_t node_hits(const SampleTree& tree, int level, int first, float3 lo, float3 hi) {
-    const int i = first + (threadIdx.x & 31);
-    bool h = false;
-    if (i < tree.n[level]) {
-        const float4* p = tree.box[level] + 2 * (int64_t)i;
-        h = box_overlap(__ldg(p), __ldg(p + 1), lo, hi);
-    }
-    return __ballot_sync(0xffffffffu, h);
-}
-
-// Walks the tree with the box [lo, hi] and hands the chunks of the level-1 nodes it meets to
-// visit(chunk, valid), 32 per call: eight lanes for each of four nodes.  `mine` selects
-// level-1 nodes by their number modulo 32.  Warp-collective; visit returns false to stop.
-template <bool COUNT, class Visit>
-__device__ __forceinline__ void walk_chunks(const SampleTree& tree, float3 lo, float3 hi, uint32_t mine, int2* stack,
-                                            int* node_list, int& n_tested, Visit visit) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t lt = lane_lt_mask();
-    int queued = 0;  // level-1 nodes in node_list: at most 3 before a round adds up to 32
-    for (int f = 0; f < tree.n[tree.top]; f += 32) {
-        int level = tree.top, first = f;
-        uint32_t m = node_hits(tree, level, f, lo, hi);
-        if (COUNT) n_tested += 32;
-        while (true) {
-            if (level == 1) {
-                m &= mine;
-                if ((m >> lane) & 1u) node_list[queued + __popc(m & lt)] = first + lane;
-                queued += __popc(m);
-                __syncwarp();
-                while (queued >= 4) {
-                    queued -= 4;
-                    if (COUNT) n_tested += 32;
-                    if (!visit(node_list[queued + (lane >> 3)] * kNodeChunks + (lane & 7), true)) return;
-                }
-                __syncwarp();
-                m = 0;
-            }
-            if (m == 0) {
-                if (level == tree.top) break;
-                level++;
-                const int2 s = stack[level];  // (children left, first child)
-                m = (uint32_t)s.x;
-                first = s.y;
-                continue;
-            }
-            const int node = first + __ffs(m) - 1;
-            m &= m - 1;
-            __syncwarp();
-            if (lane == 0) stack[level] = make_int2((int)m, first);
-            __syncwarp();
-            level--;
-            first = 32 * node;
-            m = node_hits(tree, level, first, lo, hi);
-            if (COUNT) n_tested += 32;
-        }
-    }
-    if (queued > 0) {
-        const bool v = (lane >> 3) < queued;
-        if (COUNT) n_tested += 32;
-        visit(v ? node_list[lane >> 3] * kNodeChunks + (lane & 7) : 0, v);
-    }
-}
-
 // One Gaussian's sums over the chunks handed to it (every value but the moments is
 // warp-uniform).
 template <bool COUNT>
 struct GaussSums {
-    const SampleTree& tree;
+    const WideTree& tree;
     const float* __restrict__ rows;
     int* queue;  // shared [kChunkCap]
     int n_queue;
@@ -287,21 +175,19 @@ struct GaussSums {
 // WPG > 1: a Gaussian is owned by WPG warps: warp `part` takes the level-1 nodes whose
 // number is part modulo WPG, and the warps' sums are added in that order.
 template <int WPG, int GPW, bool COUNT>
-__global__ void __launch_bounds__(kGaussWarps * 32, kGaussMinCtas) k_backward_gauss(
+__global__ void __launch_bounds__(WPG * 32, kGaussMinWarps / WPG) k_backward_gauss(
     int P, const int32_t* __restrict__ gorder, const float* __restrict__ means, const float* __restrict__ values,
     const float* __restrict__ weights, const float* __restrict__ conics, const float4* __restrict__ boxes,
-    const __grid_constant__ SampleTree tree, const float* __restrict__ rows, float* __restrict__ gacc,
+    const __grid_constant__ WideTree tree, const float* __restrict__ rows, float* __restrict__ gacc,
     unsigned long long* stats) {
     static_assert(WPG == 1 || GPW == 1, "one of the two");
-    constexpr int kPerCta = kGaussWarps * GPW / WPG;
-    __shared__ int s_queue[kGaussWarps][kChunkCap];
-    __shared__ int s_nodes[kGaussWarps][kNodeCap];
-    __shared__ int2 s_stack[kGaussWarps][kTreeLevels];
-    __shared__ int s_list[kGaussWarps][GPW > 1 ? kUnionCap : 1];
-    __shared__ float s_part[WPG > 1 ? kGaussWarps : 1][16];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int part = warp % WPG;
-    const int g0 = blockIdx.x * kPerCta + (warp / WPG) * GPW;
+    __shared__ int s_queue[WPG][kChunkCap];
+    __shared__ WideStack s_walk[WPG];
+    __shared__ int s_list[WPG][GPW > 1 ? kUnionCap : 1];
+    __shared__ float s_part[WPG][16];
+    const int warp = WPG > 1 ? threadIdx.x >> 5 : 0, lane = threadIdx.x & 31;
+    const int part = WPG > 1 ? warp : 0;
+    const int g0 = blockIdx.x * GPW;
     int n_tested = 0, n_pairs = 0, n_chunks = 0;
     int n_list = 0;  // chunks listed, kUnionCap + 1: they did not fit
     if (GPW > 1) {
@@ -312,7 +198,7 @@ __global__ void __launch_bounds__(kGaussWarps * 32, kGaussMinCtas) k_backward_ga
             blo = __ldg(boxes + 2 * o);
             bhi = __ldg(boxes + 2 * o + 1);
         }
-        MinMax u{blo.x, blo.y, blo.z, bhi.x, bhi.y, bhi.z};
+        Box6 u{blo.x, blo.y, blo.z, bhi.x, bhi.y, bhi.z};
 #pragma unroll
         for (int off = GPW / 2; off > 0; off >>= 1) grow(u, shfl_xor_box(u, off));
         const float3 lo = make_float3(__shfl_sync(0xffffffffu, u.lx, 0), __shfl_sync(0xffffffffu, u.ly, 0),
@@ -320,7 +206,7 @@ __global__ void __launch_bounds__(kGaussWarps * 32, kGaussMinCtas) k_backward_ga
         const float3 hi = make_float3(__shfl_sync(0xffffffffu, u.hx, 0), __shfl_sync(0xffffffffu, u.hy, 0),
                                       __shfl_sync(0xffffffffu, u.hz, 0));
         int* list = s_list[warp];
-        walk_chunks<COUNT>(tree, lo, hi, 0xffffffffu, s_stack[warp], s_nodes[warp], n_tested,
+        wide_walk<COUNT>(tree, lo, hi, 0xffffffffu, s_walk[warp], n_tested,
                            [&](int c, bool valid) -> bool {
                                bool h = false;
                                if (valid) {
@@ -338,7 +224,7 @@ __global__ void __launch_bounds__(kGaussWarps * 32, kGaussMinCtas) k_backward_ga
                            });
         __syncwarp();
     }
-    uint32_t mine = 0xffffffffu;  // level-1 nodes of this warp (runs of 32 start at multiples of 32)
+    uint32_t mine = 0xffffffffu;  // level-1 nodes of this warp (by number modulo 32)
     if (WPG > 1) {
         mine = 0u;
 #pragma unroll
@@ -368,7 +254,7 @@ __global__ void __launch_bounds__(kGaussWarps * 32, kGaussMinCtas) k_backward_ga
                 sums.test(v ? s_list[warp][i + lane] : 0, v);
             }
         } else if (live) {
-            walk_chunks<COUNT>(tree, sums.lo, sums.hi, mine, s_stack[warp], s_nodes[warp], n_tested,
+            wide_walk<COUNT>(tree, sums.lo, sums.hi, mine, s_walk[warp], n_tested,
                                [&](int c, bool valid) -> bool {
                                    sums.test(c, valid);
                                    return true;
@@ -389,7 +275,7 @@ __global__ void __launch_bounds__(kGaussWarps * 32, kGaussMinCtas) k_backward_ga
             if (part == 0) {
                 tot = 0.f;
 #pragma unroll
-                for (int w = 0; w < WPG; w++) tot += s_part[warp + w][lane >> 1];
+                for (int w = 0; w < WPG; w++) tot += s_part[w][lane >> 1];
             }
         }
         if (live && part == 0) {
@@ -423,56 +309,37 @@ constexpr int kManyGaussians = 100000;
 
 }  // namespace
 
-SampleTreeSize sample_tree_size(int64_t S) {
-    SampleTreeSize z{};
-    int64_t n = (S + kNodeRows - 1) / kNodeRows;
-    z.rows_bytes = sizeof(float) * kChunkFloats * kNodeChunks * (size_t)n;
-    z.n[0] = n * kNodeChunks;
-    z.n[1] = n;
-    z.top = 1;
-    while (n > 64 && z.top + 1 < kTreeLevels) {  // at most two steps over the top level
-        n = (n + 31) / 32;
-        z.n[++z.top] = n;
-    }
-    for (int l = 0; l <= z.top; l++) z.boxes += z.n[l];
+RowTreeSize row_tree_size(int64_t S) {
+    RowTreeSize z;
+    const int64_t nodes = (S + kRowsPerNode - 1) / kRowsPerNode;
+    z.tree = wide_tree_size(nodes * kWideLeaves);
+    z.rows_bytes = sizeof(float) * kChunkFloats * kWideLeaves * (size_t)nodes;
     return z;
 }
 
-cudaError_t launch_backward_rows(int64_t S, const SampleTreeSize& z, const float4* s_sorted, const float2* out_sorted,
+cudaError_t launch_backward_rows(int64_t S, const RowTreeSize& z, const float4* s_sorted, const float2* out_sorted,
                                  const float* out_cells, const float* out_weights, const float* gout, const float* gw,
-                                 float* rows, float4* boxes, SampleTree* tree, cudaStream_t st) {
-    tree->top = z.top;
-    float4* p = boxes;
-    float4* level[kTreeLevels] = {};
-    for (int l = 0; l <= z.top; l++) {
-        level[l] = p;
-        tree->box[l] = p;
-        tree->n[l] = (int)z.n[l];
-        p += 2 * z.n[l];
-    }
+                                 float* rows, float4* boxes, cudaStream_t st) {
     if (S <= 0) return cudaSuccess;
-    k_backward_rows<<<nblk(z.n[1], kRowThreads / 32), kRowThreads, 0, st>>>(
-        S, (int)z.n[1], s_sorted, out_sorted, out_cells, out_weights, gout, gw, rows, level[0], level[1]);
+    const int64_t nodes = z.tree.n[1];
+    k_backward_rows<<<nblk(nodes, kRowThreads / 32), kRowThreads, 0, st>>>(
+        S, (int)nodes, s_sorted, out_sorted, out_cells, out_weights, gout, gw, rows, boxes, boxes + 2 * z.tree.n[0]);
     note_launch();
-    for (int l = 2; l <= z.top; l++) {
-        k_tree_up<<<nblk(z.n[l], 8), 256, 0, st>>>((int)z.n[l - 1], level[l - 1], (int)z.n[l], level[l]);
-        note_launch();
-    }
-    return cudaGetLastError();
+    return launch_wide_levels(z.tree, boxes, st);
 }
 
 template <int WPG, int GPW>
-static void launch_gauss(const BwdArgs& a, const SampleTree& tree, const float* rows, cudaStream_t st) {
-    const unsigned nb = nblk(a.P, kGaussWarps * GPW / WPG);
+static void launch_gauss(const BwdArgs& a, const WideTree& tree, const float* rows, cudaStream_t st) {
+    const unsigned nb = nblk(a.P, GPW);
     if (a.count)
-        k_backward_gauss<WPG, GPW, true><<<nb, kGaussWarps * 32, 0, st>>>(
+        k_backward_gauss<WPG, GPW, true><<<nb, WPG * 32, 0, st>>>(
             (int)a.P, a.gorder, a.means, a.values, a.weights, a.conics, a.boxes, tree, rows, a.gacc, a.stats);
     else
-        k_backward_gauss<WPG, GPW, false><<<nb, kGaussWarps * 32, 0, st>>>(
+        k_backward_gauss<WPG, GPW, false><<<nb, WPG * 32, 0, st>>>(
             (int)a.P, a.gorder, a.means, a.values, a.weights, a.conics, a.boxes, tree, rows, a.gacc, a.stats);
 }
 
-cudaError_t launch_backward_gauss(const BwdArgs& a, const SampleTree& tree, const float* rows, cudaStream_t st) {
+cudaError_t launch_backward_gauss(const BwdArgs& a, const WideTree& tree, const float* rows, cudaStream_t st) {
     if (a.P <= 0) return cudaSuccess;
     if (a.P < kFewGaussians) launch_gauss<4, 1>(a, tree, rows, st);
     else if (a.P < kManyGaussians) launch_gauss<1, 1>(a, tree, rows, st);

@@ -56,7 +56,7 @@ __global__ void k_boxes6_to_f4(int64_t n, const float* __restrict__ b6, float4* 
     out[2 * i + 1] = make_float4(b6[6 * i + 3], b6[6 * i + 4], b6[6 * i + 5], 0.f);
 }
 
-// escape edges of the stackless traversal (BvhNode c.w)
+// escape edges (BvhNode c.w)
 __global__ void k_node_escape(int64_t n, const BvhNode* __restrict__ nodes, int32_t* __restrict__ out) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -179,7 +179,7 @@ int gvc_ctx_create(gvc_ctx** out) {
     GVC_CUDA(cudaMalloc(&c->d_stats, sizeof(unsigned long long) * 16), "cudaMalloc stats");
     GVC_CUDA(cudaMemset(c->d_stats, 0, sizeof(unsigned long long) * 16), "cudaMemset stats");
     GVC_CUDA(cudaMallocHost(&c->h_status, sizeof(int)), "cudaMallocHost");
-    Lbvh* sorted[] = {&c->s_sort, &c->gbvh, &c->cells, &c->knn, &c->ts_sort, &c->scratch.dbg,
+    Lbvh* sorted[] = {&c->s_sort, &c->gsort, &c->cells, &c->knn, &c->ts_sort, &c->scratch.dbg,
                       &c->scratch.msamp};
     for (Lbvh* L : sorted) L->status = c->d_status;
     *out = c;
@@ -192,7 +192,7 @@ void gvc_ctx_destroy(gvc_ctx* ctx) {
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(c->device);
-    Lbvh* lbvhs[] = {&c->s_sort,  &c->gbvh,        &c->cells,       &c->knn,
+    Lbvh* lbvhs[] = {&c->s_sort,  &c->gsort,        &c->cells,       &c->knn,
                      &c->ts_sort, &c->scratch.dbg, &c->scratch.msamp};
     for (Lbvh* L : lbvhs) {
         DevBuf* bufs[] = {&L->keys, &L->keys_alt, &L->perm, &L->perm_alt, &L->boxes, &L->sorted_boxes, &L->left,
@@ -200,9 +200,9 @@ void gvc_ctx_destroy(gvc_ctx* ctx) {
                           &L->onesweep};
         for (DevBuf* b : bufs) b->release();
     }
-    DevBuf* bufs[] = {&c->s_sorted, &c->fwd_sorted, &c->tile_boxes, &c->tile_gdesc, &c->b_rows, &c->b_boxes, &c->blk_desc, &c->blk_boxes, &c->blk_desc_b, &c->blk_boxes_b, &c->s_grad, &c->s_gyz, &c->s_ok, &c->grec, &c->gtmp,
+    DevBuf* bufs[] = {&c->s_sorted, &c->fwd_sorted, &c->blk_desc, &c->blk_boxes, &c->blk_desc_c, &c->blk_boxes_c, &c->b_rows, &c->b_boxes, &c->gtree, &c->s_grad, &c->s_gyz, &c->s_ok, &c->grec, &c->gtmp,
                       &c->m_out_sorted, &c->knn_boxes, &c->ts_points, &c->ts_words, &c->ts_gt64, &c->scratch.gacc, &c->scratch.tmp_boxes, &c->scratch.tmp_out,
-                      &c->clog, &c->cend};
+                      &c->clog, &c->cmask, &c->cend};
     for (DevBuf* b : bufs) b->release();
     if (c->d_status) cudaFree(c->d_status);
     if (c->d_stats) cudaFree(c->d_stats);
@@ -281,18 +281,51 @@ int gvc_sync_status(gvc_ctx* ctx, void* stream) {
     return debug_check(ctx, (cudaStream_t)stream);
 }
 
-// Lane groups of the 32-sample tiles (forward per tile).
-static int ensure_tile_groups(gvc_ctx* ctx, cudaStream_t st) {
-    if (ctx->tile_groups_ready || ctx->n_tiles == 0) return GVC_OK;
-    const int64_t slots_g = ctx->n_tiles * kGroups;
-    GVC_CUDA(ctx->tile_boxes.ensure(sizeof(float4) * 2 * slots_g), "alloc tile_boxes");
-    GVC_CUDA(ctx->tile_gdesc.ensure(sizeof(uint32_t) * ctx->n_tiles), "alloc tile_gdesc");
-    // reads the context's own sorted samples (the caller's array may be gone by now)
-    GVC_CUDA(launch_sample_tiles(ctx->S, ctx->n_tiles, nullptr, nullptr, ctx->s_sort.keys.as<uint32_t>(),
-                                 ctx->s_sorted.as<float4>(),
-                                 ctx->tile_boxes.as<float4>(), ctx->tile_gdesc.as<uint32_t>(), true, st),
-             "sample tile groups");
-    ctx->tile_groups_ready = true;
+// Whether S samples are sparse among P Gaussians, S < 600 sqrt(P): below the line a warp per
+// sample (fwd_points.cu) beats a warp per block of 128 (fwd_blocks.cu), whose box then spans
+// many Gaussians that reach one or two of its rows.  Both, us, on either side of it: 2k
+// Gaussians 30k samples 24 / 36, 60k 41 / 28; 20k: 60k 98 / 151, 130k 192 / 131; 200k: 130k
+// 560 / 870, 262k 1087 / 725; 1M (clustered): 524k 2207 / 2409, 1M 4108 / 1775; far below it,
+// 1M Gaussians and 14k samples, 104 / 14395.
+static bool sparse_samples(int64_t S, int64_t P) { return (double)S * (double)S < 360000.0 * (double)P; }
+
+// Whether the tensor-core kernels are selected for a call (the forward then prepares what the
+// backward reads).
+static bool tensor_core_backward(const gvc_ctx* ctx) {
+    return ctx->bwd_mode == 3 || (ctx->bwd_mode == 0 && ctx->eval_path == 1);
+}
+
+// Morton order of the Gaussians' AABBs, their records in that order and the tree over them:
+// the LBVH for the tensor-core kernels, else the wide tree (new_order false: the order of the
+// last forward still holds).
+static int prepare_gaussians(gvc_ctx* ctx, int64_t P, const float* means, const float* values, const float* weights,
+                             const float* conics, bool new_order, bool linked, cudaStream_t st) {
+    const float4* boxes = ctx->gtmp.as<float4>();
+    if (new_order) GVC_CUDA(morton_sort_boxes(ctx->gsort, P, boxes, st), "Gaussian order");
+    GVC_CUDA(ctx->grec.ensure(sizeof(GaussRec) * P), "alloc records");
+    GVC_CUDA(ctx->gtree.ensure(sizeof(float4) * 2 * wide_tree_size(P).boxes), "alloc Gaussian tree");
+    GVC_CUDA(launch_gather_recs(P, ctx->gsort.perm.as<int32_t>(), means, values, weights, conics, boxes,
+                                ctx->grec.as<GaussRec>(), ctx->gtree.as<float4>(), !linked, st),
+             "gather records");
+    ctx->glinks_ready = false;
+    if (linked) {
+        GVC_CUDA(lbvh_hierarchy(ctx->gsort, P, ctx->gsort.keys.as<uint32_t>(), ctx->gtree.as<float4>(), st),
+                 "Gaussian LBVH");
+        ctx->glinks_ready = true;
+    }
+    return GVC_OK;
+}
+
+// The coarser block groups of the tensor-core kernels' forward.
+static int ensure_coarse_groups(gvc_ctx* ctx, cudaStream_t st) {
+    if (ctx->blk_c_ready || ctx->S == 0) return GVC_OK;
+    const int64_t n_blocks = (ctx->S + 127) / 128;
+    GVC_CUDA(ctx->blk_desc_c.ensure(sizeof(uint2) * n_blocks), "alloc blk_desc_c");
+    GVC_CUDA(ctx->blk_boxes_c.ensure(sizeof(float4) * 2 * 8 * n_blocks), "alloc blk_boxes_c");
+    GVC_CUDA(launch_sample_blocks(ctx->S, ctx->s_sorted.as<float4>(), ctx->s_sort.keys.as<uint32_t>(),
+                                  ctx->blk_desc_c.as<uint2>(), ctx->blk_boxes_c.as<float4>(), kBlockSplitCoarse, st),
+             "coarse block groups");
+    ctx->blk_c_ready = true;
     return GVC_OK;
 }
 
@@ -308,35 +341,31 @@ int gvc_build_bvh(gvc_ctx* ctx, const float* samples, int64_t S, int debug, int 
     ctx->S = S;
     ctx->n_tiles = (S + kTile - 1) / kTile;
     ctx->samples_ready = false;
-    ctx->blk_b_ready = false;
+    ctx->blk_c_ready = false;
     ctx->clog_ready = false;
     ctx->fwd_sorted_ready = false;
-    ctx->tile_groups_ready = false;  // the lane groups of the 32-sample tiles are built by their first user
     if (S > 0) {
         GVC_CUDA(morton_sort_points(ctx->s_sort, S, samples, st), "sample sort");
         const int64_t slots = ctx->n_tiles * kTile;
         GVC_CUDA(ctx->s_sorted.ensure(sizeof(float4) * slots), "alloc s_sorted");
-        // sorted samples only; the 32-sample lane groups are built by their first user
-        GVC_CUDA(launch_sample_tiles(S, ctx->n_tiles, samples, ctx->s_sort.perm.as<int32_t>(),
-                                     ctx->s_sort.keys.as<uint32_t>(), ctx->s_sorted.as<float4>(), nullptr, nullptr,
-                                     false, st),
-                 "sample tiles");
+        GVC_CUDA(launch_sample_slots(S, slots, samples, ctx->s_sort.perm.as<int32_t>(), ctx->s_sorted.as<float4>(), st),
+                 "sorted samples");
         const int64_t n_blocks = (S + 127) / 128;
         GVC_CUDA(ctx->blk_desc.ensure(sizeof(uint2) * n_blocks), "alloc blk_desc");
         GVC_CUDA(ctx->blk_boxes.ensure(sizeof(float4) * 2 * 8 * n_blocks), "alloc blk_boxes");
-        // when the options already select the tensor-core backward, its finer block groups
-        // come from the same launch; otherwise that backward builds them on first use
-        const bool tc_bwd = ctx->bwd_mode == 3 || (ctx->bwd_mode == 0 && ctx->eval_path == 1);
-        if (tc_bwd) {
-            GVC_CUDA(ctx->blk_desc_b.ensure(sizeof(uint2) * n_blocks), "alloc blk_desc_b");
-            GVC_CUDA(ctx->blk_boxes_b.ensure(sizeof(float4) * 2 * 8 * n_blocks), "alloc blk_boxes_b");
+        // when the options already select the tensor-core kernels, their coarser groups come
+        // from the same launch
+        const bool coarse = tensor_core_backward(ctx) || ctx->eval_path == 1;
+        if (coarse) {
+            GVC_CUDA(ctx->blk_desc_c.ensure(sizeof(uint2) * n_blocks), "alloc blk_desc_c");
+            GVC_CUDA(ctx->blk_boxes_c.ensure(sizeof(float4) * 2 * 8 * n_blocks), "alloc blk_boxes_c");
         }
         GVC_CUDA(launch_sample_blocks(S, ctx->s_sorted.as<float4>(), ctx->s_sort.keys.as<uint32_t>(),
-                                      ctx->blk_desc.as<uint2>(), ctx->blk_boxes.as<float4>(), kBlockSplitForward, st,
-                                      tc_bwd ? ctx->blk_desc_b.as<uint2>() : nullptr,
-                                      tc_bwd ? ctx->blk_boxes_b.as<float4>() : nullptr, kBlockSplitBackward),
+                                      ctx->blk_desc.as<uint2>(), ctx->blk_boxes.as<float4>(), kBlockSplit, st,
+                                      coarse ? ctx->blk_desc_c.as<uint2>() : nullptr,
+                                      coarse ? ctx->blk_boxes_c.as<float4>() : nullptr, kBlockSplitCoarse),
                  "sample blocks");
-        ctx->blk_b_ready = tc_bwd;
+        ctx->blk_c_ready = coarse;
     }
     ctx->samples_ready = true;
     tm.mark();
@@ -382,81 +411,75 @@ int gvc_rasterize_gaussians(gvc_ctx* ctx, int64_t P, const float* means3D, const
     GVC_CUDA(launch_preprocess(P, means3D, scales, rotations, weights, scale_modifier, conics, boxes, st),
              "preprocess");
     tm.mark();
-    GVC_CUDA(lbvh_build_boxes(ctx->gbvh, P, boxes, st), "Gaussian LBVH");
-    GVC_CUDA(ctx->grec.ensure(sizeof(GaussRec) * P), "alloc records");
-    GVC_CUDA(launch_gather_recs(P, ctx->gbvh.perm.as<int32_t>(), means3D, values, weights, conics, boxes,
-                                ctx->grec.as<GaussRec>(), st),
-             "gather records");
+    // with the tensor-core kernels selected, the forward walks the LBVH by the coarser groups
+    const bool tc_bwd = tensor_core_backward(ctx);
+    const bool linked = tc_bwd || ctx->eval_path == 1;
+    int rc = prepare_gaussians(ctx, P, means3D, values, weights, conics, true, linked, st);
+    if (rc == GVC_OK && linked) rc = ensure_coarse_groups(ctx, st);
+    if (rc != GVC_OK) return rc;
     tm.mark();
-    if (ctx->eval_path == 2) {
-        const int rc = ensure_tile_groups(ctx, st);
-        if (rc != GVC_OK) return rc;
-    }
     FwdArgs fa{};
+    fa.P = P;
     fa.s_sorted = ctx->s_sorted.as<float4>();
-    fa.tile_boxes = ctx->tile_boxes.as<float4>();
-    fa.gdesc = ctx->tile_gdesc.as<uint32_t>();
-    fa.n_tiles = ctx->n_tiles;
-    fa.gnodes = ctx->gbvh.nodes.as<BvhNode>();
+    fa.S = S;
+    fa.bdesc = (linked ? ctx->blk_desc_c : ctx->blk_desc).as<uint2>();
+    fa.bboxes = (linked ? ctx->blk_boxes_c : ctx->blk_boxes).as<float4>();
+    fa.tree = wide_tree_at(wide_tree_size(P), ctx->gtree.as<float4>());
+    fa.nodes = linked ? ctx->gsort.nodes.as<BvhNode>() : nullptr;
     fa.recs = ctx->grec.as<GaussRec>();
     fa.out_cells = out_cells;
     fa.out_weights = out_weights;
     fa.status = ctx->d_status;
     fa.stats = ctx->d_stats;
     fa.count = ctx->count_pairs != 0;
+    // the candidates are logged for the tensor-core backward when it is the one selected
+    if (tc_bwd && ctx->cand_log && S > 0) {
+        // 20 KB per 128 samples: where that does not fit in device memory, the forward runs
+        // without the log and the backward walks the tree
+        const int64_t n_blocks = (S + 127) / 128;
+        if (ctx->clog.ensure(sizeof(int32_t) * kCandLogPerBlock * n_blocks) == cudaSuccess &&
+            ctx->cmask.ensure(kCandLogPerBlock * n_blocks) == cudaSuccess &&
+            ctx->cend.ensure(sizeof(int32_t) * 8 * n_blocks) == cudaSuccess) {
+            fa.clog = ctx->clog.as<int32_t>();
+            fa.cmask = ctx->cmask.as<uint8_t>();
+            fa.cend = ctx->cend.as<int32_t>();
+            fa.fdesc = ctx->blk_desc.as<uint2>();
+            fa.fboxes = ctx->blk_boxes.as<float4>();
+        } else {
+            (void)cudaGetLastError();  // a failed allocation is not sticky: clear it
+            ctx->clog.release();
+            ctx->cmask.release();
+            ctx->cend.release();
+        }
+    }
+    // (out, W) in sorted order as well, for the backward's rows
+    if (S > 0) {
+        if (ctx->fwd_sorted.ensure(sizeof(float2) * ctx->n_tiles * kTile) == cudaSuccess) {
+            fa.out_sorted = ctx->fwd_sorted.as<float2>();
+        } else {
+            (void)cudaGetLastError();
+            ctx->fwd_sorted.release();
+        }
+    }
     const int tk = timer_begin(ctx, st, 0);
-    if (ctx->eval_path == 2) {
-        GVC_CUDA(launch_forward(fa, st), "forward");
+    bool masks = false;
+    cudaError_t e;
+    if (ctx->eval_path == 1) {
+        e = launch_forward_tc(fa, st);
+    } else if (!linked) {
+        e = sparse_samples(S, P) ? launch_forward_points(fa, st) : launch_forward_blocks(fa, st);
+    } else if (forward_linked_rows(S, P) == 0) {
+        e = launch_forward_cta(fa, st);
     } else {
-        CtaArgs ca{};
-        ca.s_sorted = ctx->s_sorted.as<float4>();
-        ca.S = ctx->S;
-        ca.bdesc = ctx->blk_desc.as<uint2>();
-        ca.bboxes = ctx->blk_boxes.as<float4>();
-        ca.gnodes = ctx->gbvh.nodes.as<BvhNode>();
-        ca.n_internal = ctx->gbvh.n > 1 ? ctx->gbvh.n - 1 : 1;
-        ca.stackless = ctx->traversal == 1;
-        ca.recs = ctx->grec.as<GaussRec>();
-        ca.out_cells = out_cells;
-        ca.out_weights = out_weights;
-        ca.status = ctx->d_status;
-        ca.stats = ctx->d_stats;
-        ca.count = ctx->count_pairs != 0;
-        // the candidates are logged for the tensor-core backward when it is the one selected
-        const bool tc_bwd = ctx->bwd_mode == 3 || (ctx->bwd_mode == 0 && ctx->eval_path == 1);
-        if (tc_bwd && ctx->cand_log && ctx->S > 0) {
-            // 16 KB per 128 samples: where that does not fit in device memory, the forward
-            // runs without the log and the backward walks the tree
-            const int64_t n_blocks = (ctx->S + 127) / 128;
-            if (ctx->clog.ensure(sizeof(int32_t) * kCandLogPerBlock * n_blocks) == cudaSuccess &&
-                ctx->cend.ensure(sizeof(int32_t) * 8 * n_blocks) == cudaSuccess) {
-                ca.clog = ctx->clog.as<int32_t>();
-                ca.cend = ctx->cend.as<int32_t>();
-            } else {
-                (void)cudaGetLastError();  // a failed allocation is not sticky: clear it
-                ctx->clog.release();
-                ctx->cend.release();
-            }
-        }
-        // the FP32 forward also stores (out, W) in sorted order for the backward's sample records
-        if (ctx->eval_path == 0 && ctx->S > 0) {
-            if (ctx->fwd_sorted.ensure(sizeof(float2) * ctx->n_tiles * kTile) == cudaSuccess) {
-                ca.out_sorted = ctx->fwd_sorted.as<float2>();
-            } else {
-                (void)cudaGetLastError();
-                ctx->fwd_sorted.release();
-            }
-        }
-        GVC_CUDA(launch_forward_cta(ca, ctx->eval_path == 1, st), "forward (CTA)");
-        ctx->clog_ready = ca.clog != nullptr;
-        ctx->fwd_sorted_ready = ca.out_sorted != nullptr;
-        ctx->fwd_out_cells = out_cells;
-        ctx->fwd_out_weights = out_weights;
+        e = launch_forward_blocks(fa, st);
+        masks = true;
     }
-    if (ctx->eval_path == 2) {
-        ctx->clog_ready = false;
-        ctx->fwd_sorted_ready = false;
-    }
+    GVC_CUDA(e, "forward");
+    ctx->clog_ready = fa.clog != nullptr;
+    ctx->clog_masks = masks;
+    ctx->fwd_sorted_ready = fa.out_sorted != nullptr;
+    ctx->fwd_out_cells = out_cells;
+    ctx->fwd_out_weights = out_weights;
     timer_end(ctx, st, tk);
     tm.mark();
     ctx->P = P;
@@ -520,7 +543,7 @@ int gvc_rasterize_gaussians_backward(gvc_ctx* ctx, int64_t P, const float* means
     float* gacc = sc->gacc.as<float>();
     // mode 3, or the tensor-core path in auto mode: reduction over samples on tcgen05; every
     // other mode: the Gaussian-owned sums
-    const bool tc_bwd = ctx->bwd_mode == 3 || (ctx->bwd_mode == 0 && ctx->eval_path == 1);
+    const bool tc_bwd = tensor_core_backward(ctx);
     const bool have_order = ctx->gauss_ready && ctx->P == P;
     if (ctx->n_tiles == 0) {
         GVC_CUDA(cudaMemsetAsync(gacc, 0, sizeof(float) * 16 * P, st), "zero gacc");
@@ -548,61 +571,55 @@ int gvc_rasterize_gaussians_backward(gvc_ctx* ctx, int64_t P, const float* means
                                          ctx->s_gyz.as<float>(), ctx->s_ok.as<uint8_t>(), st),
                      "sample grads");
             tm.mark();
-            if (!have_order) GVC_CUDA(lbvh_build_boxes(ctx->gbvh, P, boxes, st), "Gaussian LBVH");
             if (!same_gauss) {
-                GVC_CUDA(ctx->grec.ensure(sizeof(GaussRec) * P), "alloc records");
-                GVC_CUDA(launch_gather_recs(P, ctx->gbvh.perm.as<int32_t>(), means3D, values, weights, conics,
-                                            boxes, ctx->grec.as<GaussRec>(), st),
-                         "gather records");
+                if (!have_order) ctx->gauss_ready = false;  // the order below is not the forward's
+                const int rc = prepare_gaussians(ctx, P, means3D, values, weights, conics, !have_order, true, st);
+                if (rc != GVC_OK) return rc;
+            } else if (!ctx->glinks_ready) {
+                GVC_CUDA(lbvh_hierarchy(ctx->gsort, P, ctx->gsort.keys.as<uint32_t>(), ctx->gtree.as<float4>(), st),
+                         "Gaussian LBVH");
+                ctx->glinks_ready = true;
             }
             GVC_CUDA(cudaMemsetAsync(gacc, 0, sizeof(float) * 16 * P, st), "zero gacc");
-            ba.gperm = ctx->gbvh.perm.as<int32_t>();
-            ba.n_slots = slots;
+            ba.gperm = ctx->gsort.perm.as<int32_t>();
+            ba.S = S;
+            ba.bdesc = ctx->blk_desc.as<uint2>();
+            ba.bboxes = ctx->blk_boxes.as<float4>();
             ba.s_grad = ctx->s_grad.as<float4>();
             ba.s_gyz = ctx->s_gyz.as<float>();
             ba.s_ok = ctx->s_ok.as<uint8_t>();
-            ba.gnodes = ctx->gbvh.nodes.as<BvhNode>();
-            ba.g_internal = ctx->gbvh.n > 1 ? ctx->gbvh.n - 1 : 1;
-            ba.stackless = ctx->traversal == 1;
+            ba.nodes = ctx->gsort.nodes.as<BvhNode>();
             ba.recs = ctx->grec.as<GaussRec>();
-            const int tk = timer_begin(ctx, st, 1);
-            const int64_t n_blocks = (S + 127) / 128;
-            if (!ctx->blk_b_ready) {
-                GVC_CUDA(ctx->blk_desc_b.ensure(sizeof(uint2) * n_blocks), "alloc blk_desc_b");
-                GVC_CUDA(ctx->blk_boxes_b.ensure(sizeof(float4) * 2 * 8 * n_blocks), "alloc blk_boxes_b");
-                GVC_CUDA(launch_sample_blocks(S, ctx->s_sorted.as<float4>(), ctx->s_sort.keys.as<uint32_t>(),
-                                              ctx->blk_desc_b.as<uint2>(), ctx->blk_boxes_b.as<float4>(),
-                                              kBlockSplitBackward, st),
-                         "backward block groups");
-                ctx->blk_b_ready = true;
-            }
             // the forward's candidate log, when it belongs to these Gaussians and samples,
             // replaces the backward's own walk of the tree
             if (have_order && ctx->clog_ready) {
                 ba.clog = ctx->clog.as<int32_t>();
+                ba.cmask = ctx->cmask.as<uint8_t>();
                 ba.cend = ctx->cend.as<int32_t>();
-                ba.cdesc = ctx->blk_desc.as<uint2>();
+                ba.cdesc = ctx->blk_desc_c.as<uint2>();
+                if (!ctx->clog_masks || !same_gauss) GVC_CUDA(launch_log_masks(ba, ctx->cmask.as<uint8_t>(), st), "log masks");
+                ctx->clog_masks = true;
             }
-            const uint2* bdesc = ctx->blk_desc_b.as<uint2>();
-            const float4* bboxes = ctx->blk_boxes_b.as<float4>();
-            GVC_CUDA(launch_backward_cta(ba, n_blocks, bdesc, bboxes, st), "backward (tensor core)");
+            const int tk = timer_begin(ctx, st, 1);
+            GVC_CUDA(launch_backward_tc(ba, st), "backward (tensor core)");
             timer_end(ctx, st, tk);
         } else {
-            const SampleTreeSize z = sample_tree_size(S);
+            const RowTreeSize z = row_tree_size(S);
             GVC_CUDA(ctx->b_rows.ensure(z.rows_bytes), "alloc gradient rows");
-            GVC_CUDA(ctx->b_boxes.ensure(sizeof(float4) * 2 * z.boxes), "alloc sample tree");
-            SampleTree tree;
+            GVC_CUDA(ctx->b_boxes.ensure(sizeof(float4) * 2 * z.tree.boxes), "alloc sample tree");
             GVC_CUDA(launch_backward_rows(S, z, ctx->s_sorted.as<float4>(), out_sorted, out_cells, out_weights,
                                           dL_dout_cells, dL_dout_weights, ctx->b_rows.as<float>(),
-                                          ctx->b_boxes.as<float4>(), &tree, st),
+                                          ctx->b_boxes.as<float4>(), st),
                      "gradient rows");
             tm.mark();
-            ba.gorder = have_order ? ctx->gbvh.perm.as<int32_t>() : nullptr;
+            ba.gorder = have_order ? ctx->gsort.perm.as<int32_t>() : nullptr;
             ba.means = means3D;
             ba.values = values;
             ba.weights = weights;
             const int tk = timer_begin(ctx, st, 1);
-            GVC_CUDA(launch_backward_gauss(ba, tree, ctx->b_rows.as<float>(), st), "backward (Gaussian-owned)");
+            GVC_CUDA(launch_backward_gauss(ba, wide_tree_at(z.tree, ctx->b_boxes.as<float4>()),
+                                           ctx->b_rows.as<float>(), st),
+                     "backward (Gaussian-owned)");
             timer_end(ctx, st, tk);
         }
     }

@@ -1,28 +1,13 @@
-// cta.cu -- CTA-level forward evaluation in FP32 (SIMT), the 128-sample block groups the
-// CTA kernels run on, and a tcgen05 GEMM test hook.  The forward with the exponent on the
-// tensor cores is in fwd_tc.cu.
+// cta.cu -- the 128-sample block groups the forward and the tensor-core backward run on, the
+// forward with a CTA per block, and the tcgen05 and bounded-wait test hooks.
 //
-// One CTA owns 128 consecutive Morton-sorted samples.  build_bvh splits each such block
-// into at most 8 contiguous "block groups" at Z-order jumps (the rule of the 32-sample
-// tiles, applied to 128 rows).  For each group the CTA walks the Gaussian LBVH (a
-// producer warp, warp-cooperative traversal) and stages candidate Gaussians 32 at a time;
-// two consumer warps (two rows per thread) evaluate, for the columns whose box overlaps
-// their rows, the exact AABB test, the base-2 power, the window, ex2 and the sums.
+// build_bvh's 128-sample blocks are split into at most 8 contiguous "block groups" at
+// Z-order jumps.
 #include "cta.cuh"
+#include "pair.cuh"
 #include "tc.cuh"
-#include "traverse.cuh"
 
 namespace gvc {
-
-
-constexpr float kHalfLog2eC = -0.72134752044448170368f;
-constexpr float kLog2FloorC = -20.197570572173914f;
-
-__device__ __forceinline__ float ex2_apx(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 
 __device__ __forceinline__ float hp6(const Box6& b) { return (b.hx - b.lx) + (b.hy - b.ly) + (b.hz - b.lz); }
 
@@ -290,7 +275,11 @@ __global__ void __launch_bounds__(128) k_tc_gemm_test(const __nv_bfloat16* __res
 }
 
 // ---------------------------------------------------------------------------------------
-// CTA forward (FP32): warp-specialised pipeline.
+// CTA forward (FP32) by the LBVH and the coarse groups, for the tensor-core kernels' order of
+// the sums (fwd_blocks.cu) where samples are too few to fill the chip with a warp per block:
+// the walk, the staging and the evaluation of a block go on in three warps at once.
+// 1M clustered Gaussians x 262k samples 1.81 ms, one warp per block 3.09, one per 32 rows 2.40.
+// Warp-specialised pipeline:
 //   warp 2 (producer): walks the Gaussian LBVH with each group's box (warp-cooperative
 //     traversal), copies each batch of up to 32 candidate records into one of kStages
 //     stages with cp.async and, one call later, finalises it (base-2 conic, per-consumer
@@ -348,7 +337,7 @@ struct Producer {
         if (lane < nb) {
             const float4 r1 = sm.gd[s][lane][1], r2 = sm.gd[s][lane][2], r3 = sm.gd[s][lane][3],
                          r4 = sm.gd[s][lane][4];
-            const float k = kHalfLog2eC;
+            const float k = kHalfLog2e;
             const float c0 = k * r1.x, c1 = k * r1.y, c2 = k * r1.z, c3 = k * r1.w, c4 = k * r2.x, c5 = k * r2.y;
             sm.gd[s][lane][1] = make_float4(c0, 2.f * c1, 2.f * c2, c3);
             sm.gd[s][lane][2] = make_float4(2.f * c4, c5, r2.z, 0.f);
@@ -380,7 +369,7 @@ struct Producer {
 
     __device__ __forceinline__ void operator()(const int* c, int nb) {
         const int lane = threadIdx.x & 31;
-        log.append(c, nb);
+        if (log.ids) log.append(nb, lane < nb ? c[lane] : 0, 0u);
         if (failed || !acquire_batch(total)) {
             failed = true;
             __syncwarp();
@@ -406,10 +395,10 @@ struct Producer {
     }
 };
 
-template <bool COUNT, bool STACKLESS>
+template <bool COUNT>
 __global__ void __launch_bounds__(kConsumerWarps * 32 + 32, kCtaMinBlocks)
     k_forward_cta(const float4* __restrict__ s_sorted, int64_t S, const uint2* __restrict__ bdesc,
-                  const float4* __restrict__ bboxes, const BvhNode* __restrict__ nodes, int64_t n_internal,
+                  const float4* __restrict__ bboxes, const BvhNode* __restrict__ nodes,
                   const GaussRec* __restrict__ recs, float* __restrict__ out_cells, float* __restrict__ out_weights,
                   float2* __restrict__ out_sorted, int32_t* __restrict__ clog, int32_t* __restrict__ cend, int* status,
                   unsigned long long* stats) {
@@ -451,7 +440,7 @@ __global__ void __launch_bounds__(kConsumerWarps * 32 + 32, kCtaMinBlocks)
                 const bool in = row < S && r >= ra && r < rb;
                 float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (in) p = s_sorted[row];
-                const Box6 bq = warp_box6(in, p.x, p.y, p.z);
+                const Box6 bq = warp_point_box(in, p.x, p.y, p.z);
                 if (lane == 0) {
                     if (q % RPT == 0) {
                         sm.wb[q / RPT] = bq;
@@ -467,8 +456,8 @@ __global__ void __launch_bounds__(kConsumerWarps * 32 + 32, kCtaMinBlocks)
                 }
             }
             __syncwarp();
-            st |= warp_traverse_sel<STACKLESS>(nodes, n_internal, make_float3(glo.x, glo.y, glo.z),
-                                               make_float3(ghi.x, ghi.y, ghi.z), sm.stack, sm.cand, pr, tc);
+            st |= warp_traverse(nodes, make_float3(glo.x, glo.y, glo.z), make_float3(ghi.x, ghi.y, ghi.z), sm.stack,
+                                sm.cand, pr, tc);
             pr.log.end_group(g);
         }
         if (pr.failed || st) pr.log.over = true;
@@ -550,8 +539,8 @@ __global__ void __launch_bounds__(kConsumerWarps * 32 + 32, kCtaMinBlocks)
                     const float dx = x - r0.x, dy = y - r0.y, dz = z - r0.z;
                     const float p2 = dx * fmaf(r1.x, dx, fmaf(r1.y, dy, r1.z * dz)) + dy * fmaf(r1.w, dy, r2.x * dz) +
                                      dz * (r2.y * dz);
-                    const bool cc = in && p2 >= kLog2FloorC && p2 <= 0.0f;
-                    const float wt = cc ? r0.w * ex2_apx(p2) : 0.f;
+                    const bool cc = in && p2 >= kLog2Floor && p2 <= 0.0f;
+                    const float wt = cc ? r0.w * ex2_approx(p2) : 0.f;
                     Wr[k] += wt;
                     Vr[k] = fmaf(wt, r2.z, Vr[k]);
                     if (COUNT) {
@@ -597,8 +586,6 @@ __global__ void __launch_bounds__(kConsumerWarps * 32 + 32, kCtaMinBlocks)
     }
 }
 
-static inline unsigned nblk128(int64_t n) { return (unsigned)((n + kBlockRows - 1) / kBlockRows); }
-
 cudaError_t launch_sample_blocks(int64_t S, const float4* s_sorted, const uint32_t* skeys, uint2* bdesc,
                                  float4* bboxes, float ratio, cudaStream_t st, uint2* bdesc2, float4* bboxes2,
                                  float ratio2) {
@@ -610,24 +597,21 @@ cudaError_t launch_sample_blocks(int64_t S, const float4* s_sorted, const uint32
     return cudaGetLastError();
 }
 
-template <bool COUNT, bool STACKLESS>
-static cudaError_t launch_cta_impl(const CtaArgs& a, cudaStream_t st) {
+template <bool COUNT>
+static cudaError_t launch_cta_impl(const FwdArgs& a, cudaStream_t st) {
     const size_t smem = sizeof(CtaSmem);
-    cudaError_t e =
-        cudaFuncSetAttribute(k_forward_cta<COUNT, STACKLESS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_forward_cta<COUNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_forward_cta<COUNT, STACKLESS><<<nblk128(a.S), kConsumerWarps * 32 + 32, smem, st>>>(
-        a.s_sorted, a.S, a.bdesc, a.bboxes, a.gnodes, a.n_internal, a.recs, a.out_cells, a.out_weights,
-        a.out_sorted, a.clog, a.cend, a.status, a.stats);
+    k_forward_cta<COUNT><<<(unsigned)((a.S + kBlockRows - 1) / kBlockRows), kConsumerWarps * 32 + 32, smem, st>>>(
+        a.s_sorted, a.S, a.bdesc, a.bboxes, a.nodes, a.recs, a.out_cells, a.out_weights, a.out_sorted, a.clog, a.cend,
+        a.status, a.stats);
     gvc::note_launch();
     return cudaGetLastError();
 }
 
-cudaError_t launch_forward_cta(const CtaArgs& a, bool tc, cudaStream_t st) {
+cudaError_t launch_forward_cta(const FwdArgs& a, cudaStream_t st) {
     if (a.S <= 0) return cudaSuccess;
-    if (tc) return launch_forward_tc(a, st);
-    if (a.stackless) return a.count ? launch_cta_impl<true, true>(a, st) : launch_cta_impl<false, true>(a, st);
-    return a.count ? launch_cta_impl<true, false>(a, st) : launch_cta_impl<false, false>(a, st);
+    return a.count ? launch_cta_impl<true>(a, st) : launch_cta_impl<false>(a, st);
 }
 
 cudaError_t launch_tc_gemm_test(const void* A, const void* B, int N, float* D, int* status, cudaStream_t st) {

@@ -1,5 +1,5 @@
-// cta.cuh -- pieces shared by the CTA-level kernels on 128-sample blocks (the FP32 forward
-// in cta.cu, the tensor-core forward in fwd_tc.cu): block-group descriptors, box helpers.
+// cta.cuh -- pieces shared by the kernels on 128-sample blocks (fwd_blocks.cu, fwd_tc.cu,
+// bwd_tc.cu): block-group descriptors, box helpers.
 #pragma once
 #include "render.cuh"
 
@@ -7,25 +7,6 @@ namespace gvc {
 
 constexpr int kBlockRows = 128;
 constexpr int kBlockGroups = 8;
-
-struct Box6 {
-    float lx, ly, lz, hx, hy, hz;
-};
-
-// Box of the lanes with `in` set (empty box if none), on every lane of the warp.
-__device__ __forceinline__ Box6 warp_box6(bool in, float x, float y, float z) {
-    Box6 b{in ? x : INFINITY, in ? y : INFINITY, in ? z : INFINITY, in ? x : -INFINITY, in ? y : -INFINITY,
-           in ? z : -INFINITY};
-    for (int off = 16; off > 0; off >>= 1) {
-        b.lx = fminf(b.lx, __shfl_xor_sync(0xffffffffu, b.lx, off));
-        b.ly = fminf(b.ly, __shfl_xor_sync(0xffffffffu, b.ly, off));
-        b.lz = fminf(b.lz, __shfl_xor_sync(0xffffffffu, b.lz, off));
-        b.hx = fmaxf(b.hx, __shfl_xor_sync(0xffffffffu, b.hx, off));
-        b.hy = fmaxf(b.hy, __shfl_xor_sync(0xffffffffu, b.hy, off));
-        b.hz = fmaxf(b.hz, __shfl_xor_sync(0xffffffffu, b.hz, off));
-    }
-    return b;
-}
 
 __device__ __forceinline__ bool overlap6(const Box6& b, float4 lo, float4 hi) {
     return lo.x <= b.hx && hi.x >= b.lx && lo.y <= b.hy && hi.y >= b.ly && lo.z <= b.hz && hi.z >= b.lz;

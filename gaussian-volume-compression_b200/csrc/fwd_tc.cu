@@ -37,7 +37,6 @@
 // 0 (e = 1) instead of dropping the pair.
 #include "cta.cuh"
 #include "tc.cuh"
-#include "traverse.cuh"
 
 // Batches in flight and resident CTAs per SM requested from the register allocator
 // (measured at 2M x 16M: 2 stages at 6 CTAs per SM 23.7 ms, 4 stages at 4 CTAs 25.1 ms).
@@ -133,7 +132,7 @@ struct FwdTcStager {
 
     __device__ __forceinline__ void operator()(const int* c, int nb) {
         const int lane = threadIdx.x & 31;
-        log.append(c, nb);
+        if (log.ids) log.append(nb, lane < nb ? c[lane] : 0, 0u);
         if (failed || !acquire(total)) {
             failed = true;
             __syncwarp();
@@ -178,7 +177,7 @@ struct FwdTcFinaliser {
             const bool in = rr < S && r >= ra && r < rb;
             float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
             if (in) p = s_sorted[rr];
-            wb[q] = warp_box6(in, p.x, p.y, p.z);
+            wb[q] = warp_point_box(in, p.x, p.y, p.z);
         }
     }
 
@@ -256,12 +255,12 @@ struct FwdTcFinaliser {
 
 }  // namespace
 
-template <bool COUNT, bool STACKLESS>
+template <bool COUNT>
 __global__ void __launch_bounds__(192, kMinBlocks)
     k_forward_tc(const float4* __restrict__ s_sorted, int64_t S, const uint2* __restrict__ bdesc,
-                 const float4* __restrict__ bboxes, const BvhNode* __restrict__ nodes, int64_t n_internal,
+                 const float4* __restrict__ bboxes, const BvhNode* __restrict__ nodes,
                  const GaussRec* __restrict__ recs, float* __restrict__ out_cells, float* __restrict__ out_weights,
-                 int32_t* __restrict__ clog, int32_t* __restrict__ cend, int* status, unsigned long long* stats) {
+                 float2* __restrict__ out_sorted, int32_t* __restrict__ clog, int32_t* __restrict__ cend, int* status, unsigned long long* stats) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     FwdTcSmem& sm = *reinterpret_cast<FwdTcSmem*>(
         smem_raw + ((1024 - (static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw)) & 1023)) & 1023));
@@ -333,8 +332,8 @@ __global__ void __launch_bounds__(192, kMinBlocks)
             sg.flush();  // the pending batch belongs to the previous group
             sg.g = g;
             const float4 glo = bboxes[2 * (blk * kBlockGroups + g)], ghi = bboxes[2 * (blk * kBlockGroups + g) + 1];
-            st |= warp_traverse_sel<STACKLESS>(nodes, n_internal, make_float3(glo.x, glo.y, glo.z),
-                                               make_float3(ghi.x, ghi.y, ghi.z), sm.stack, sm.cand, sg, tc);
+            st |= warp_traverse(nodes, make_float3(glo.x, glo.y, glo.z), make_float3(ghi.x, ghi.y, ghi.z), sm.stack,
+                                sm.cand, sg, tc);
             sg.log.end_group(g);
         }
         if (sg.failed || st) sg.log.over = true;
@@ -456,6 +455,7 @@ __global__ void __launch_bounds__(192, kMinBlocks)
             }
             out_cells[orig] = o;
             out_weights[orig] = ww;
+            if (out_sorted) out_sorted[row] = make_float2(o, ww);
         }
         if (COUNT) {
             unsigned long long a = (unsigned long long)ncand, b = (unsigned long long)ncontrib;
@@ -476,24 +476,21 @@ __global__ void __launch_bounds__(192, kMinBlocks)
     if (w == 0) tmem_dealloc(tmem, kStages * kBatch);
 }
 
-template <bool COUNT, bool STACKLESS>
-static cudaError_t launch_fwd_tc_impl(const CtaArgs& a, cudaStream_t st) {
+template <bool COUNT>
+static cudaError_t launch_fwd_tc_impl(const FwdArgs& a, cudaStream_t st) {
     const size_t smem = sizeof(FwdTcSmem) + 1024;
-    cudaError_t e =
-        cudaFuncSetAttribute(k_forward_tc<COUNT, STACKLESS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_forward_tc<COUNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const unsigned nb = (unsigned)((a.S + kBlockRows - 1) / kBlockRows);
-    k_forward_tc<COUNT, STACKLESS><<<nb, 192, smem, st>>>(a.s_sorted, a.S, a.bdesc, a.bboxes, a.gnodes, a.n_internal,
-                                                          a.recs, a.out_cells, a.out_weights, a.clog, a.cend,
-                                                          a.status, a.stats);
+    k_forward_tc<COUNT><<<nb, 192, smem, st>>>(a.s_sorted, a.S, a.bdesc, a.bboxes, a.nodes, a.recs, a.out_cells,
+                                               a.out_weights, a.out_sorted, a.clog, a.cend, a.status, a.stats);
     gvc::note_launch();
     return cudaGetLastError();
 }
 
-cudaError_t launch_forward_tc(const CtaArgs& a, cudaStream_t st) {
+cudaError_t launch_forward_tc(const FwdArgs& a, cudaStream_t st) {
     if (a.S <= 0) return cudaSuccess;
-    if (a.stackless) return a.count ? launch_fwd_tc_impl<true, true>(a, st) : launch_fwd_tc_impl<false, true>(a, st);
-    return a.count ? launch_fwd_tc_impl<true, false>(a, st) : launch_fwd_tc_impl<false, false>(a, st);
+    return a.count ? launch_fwd_tc_impl<true>(a, st) : launch_fwd_tc_impl<false>(a, st);
 }
 
 }  // namespace gvc

@@ -14,8 +14,6 @@ constexpr float kWeightCutoff = 1e-2f;
 constexpr float kPowerFloor = -14.0f;
 // Tile of Morton-sorted samples handled by one warp.
 constexpr int kTile = 32;
-// Each tile is split into at most this many lane groups at Morton-order jumps.
-constexpr int kGroups = 4;
 // Per-warp traversal stack (entries of int32) in shared memory.
 constexpr int kStackCap = 512;
 // Gaussians whose covariance condition estimate exceeds this get an FP64 inverse.
@@ -28,10 +26,10 @@ void note_launch(int n = 1);
 constexpr int kStatusStackOverflow = 1;
 constexpr int kStatusTimeout = 2;  // a bounded wait gave up (mbarrier, radix-sort look-back)
 
-// Gaussian evaluation record, one per Gaussian in LBVH (Morton) order: 80 bytes.
+// Gaussian evaluation record, one per Gaussian in Morton order: 80 bytes.
 //   r0 = (mu.x, mu.y, mu.z, w)
 //   r1 = (c0, c1, c2, c3)  -- conic xx, xy, xz, yy as written to the conics output
-//   r2 = (c4, c5, v, 0)    -- conic yz, zz, value
+//   r2 = (c4, c5, v, cover) -- conic yz, zz, value; cover = 1 where the window covers the AABB
 //   r3 = (lo.x, lo.y, lo.z, 0), r4 = (hi.x, hi.y, hi.z, 0): the AABB
 struct __align__(16) GaussRec {
     float4 r0, r1, r2, r3, r4;
@@ -42,7 +40,7 @@ struct __align__(16) GaussRec {
 //   c = (R.lo.xyz, escape edge),     d = (R.hi.xyz, right child bits)
 // Child encoding: internal node k >= 0; leaf i stored as (i | 0x80000000).  The escape
 // edge (2p + s: child s of node p, 0xffffffff for none) is the edge that follows this
-// node's subtree in pre-order; the stackless traversal (traverse.cuh) walks by it.
+// node's subtree in pre-order: a walk by it needs no stack.
 struct __align__(16) BvhNode {
     float4 a, b, c, d;
 };
@@ -99,7 +97,7 @@ struct gvc_ctx {
     int cov_grad_mode = 0;
     int bwd_mode = 0;
     int eval_path = 0;
-    int traversal = 0;      // 0 = node stack, 1 = stackless (GVC_OPT_TRAVERSAL)
+    int traversal = 0;      // GVC_OPT_TRAVERSAL
     int cand_log = 1;       // GVC_OPT_CAND_LOG
     int count_pairs = 0;
     int time_kernels = 0;   // record CUDA events around the evaluation kernels
@@ -114,10 +112,11 @@ struct gvc_ctx {
     int64_t S = 0;
     int64_t n_tiles = 0;
     bool samples_ready = false;
-    // candidate log of the last block-group forward (for the tensor-core backward)
-    gvc::DevBuf clog, cend;
+    // candidate log of the last forward (for the tensor-core backward)
+    gvc::DevBuf clog, cmask, cend;
     bool clog_ready = false;
-    // (out, W) per sorted slot as the last FP32 block-group forward wrote them, and the
+    bool clog_masks = false;  // its masks are written
+    // (out, W) per sorted slot as the last forward wrote them, and the
     // output arrays it wrote them to (the backward uses the copy for those arrays only)
     gvc::DevBuf fwd_sorted;
     const float* fwd_out_cells = nullptr;
@@ -134,26 +133,25 @@ struct gvc_ctx {
     float fwd_scale_mod = 0.f;
     bool fwd_recs_ready = false;
     gvc::DevBuf s_sorted;   // [n_tiles*32] float4 (x, y, z, bits of caller index or -1)
-    gvc::DevBuf tile_boxes; // [n_tiles * kGroups] group boxes, 2 x float4 (empty for unused slots)
-    gvc::DevBuf tile_gdesc; // [n_tiles] group starts: bytes 0..2 = start lane of groups 1..3
-                            // (32 if unused), byte 3 = number of groups
-    gvc::DevBuf blk_desc;   // [ceil(S/128)] uint2 block-group descriptors (CTA kernels)
+    gvc::DevBuf blk_desc;   // [ceil(S/128)] uint2 block-group descriptors
     gvc::DevBuf blk_boxes;  // [ceil(S/128) * 8] block-group boxes, 2 x float4
-    gvc::DevBuf blk_desc_b;   // the same with the backward's finer split (built on first use)
-    gvc::DevBuf blk_boxes_b;
-    bool blk_b_ready = false;
-    bool tile_groups_ready = false;  // tile lane groups built for the current samples
+    gvc::DevBuf blk_desc_c;   // the same with the coarser split of the tensor-core kernels' forward
+    gvc::DevBuf blk_boxes_c;
+    bool blk_c_ready = false;
     gvc::DevBuf s_grad;     // [n_tiles*32] float4 (x, y, z, gx) backward sample records
     gvc::DevBuf s_gyz;      // [n_tiles*32] float gyz (see k_sample_grads)
     gvc::DevBuf s_ok;       // [n_tiles*32] uint8 1 iff W > 0.01 (pair statistics only)
     gvc::Lbvh s_sort;       // sample sort (keys/perm only)
     gvc::DevBuf b_rows;     // gradient rows in chunks of 16 (Gaussian-owned backward, bwd_gauss.cu)
-    gvc::DevBuf b_boxes;    // boxes of the chunks and of the levels above them
+    gvc::DevBuf b_boxes;    // wide tree over the chunks
     // Gaussian state (forward)
     int64_t P = 0;
     bool gauss_ready = false;
-    gvc::Lbvh gbvh;         // Gaussian LBVH
-    gvc::DevBuf grec;       // [P] GaussRec in LBVH order
+    gvc::Lbvh gsort;        // Gaussian order (Morton order of the AABBs' centres), and with the
+                            // tensor-core kernels the LBVH over it
+    bool glinks_ready = false;  // its LBVH is built
+    gvc::DevBuf gtree;      // leaf boxes in that order, and the wide tree's levels over them
+    gvc::DevBuf grec;       // [P] GaussRec in Morton order
     gvc::DevBuf gtmp;       // preprocess scratch: AABBs in caller order
     // mesh sampler
     gvc::Lbvh cells;

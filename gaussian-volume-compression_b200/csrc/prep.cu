@@ -148,138 +148,62 @@ __global__ void __launch_bounds__(256) k_preprocess(int64_t P, const float* __re
     }
 }
 
+// Whether every point of the AABB is inside the power window: sum |c_ij| h_i h_j, the largest
+// d^T C d over the box |d_i| <= h_i, is at most 28 (with room for rounding).  The window then
+// culls nothing that the box test keeps, as at the w = 0.1 a fit starts with (3.03 sigma).
+__device__ __forceinline__ bool window_covers(const GaussRec& r) {
+    const float hx = fmaxf(r.r4.x - r.r0.x, r.r0.x - r.r3.x), hy = fmaxf(r.r4.y - r.r0.y, r.r0.y - r.r3.y),
+                hz = fmaxf(r.r4.z - r.r0.z, r.r0.z - r.r3.z);
+    const float q = fabsf(r.r1.x) * hx * hx + fabsf(r.r1.w) * hy * hy + fabsf(r.r2.y) * hz * hz +
+                    2.f * (fabsf(r.r1.y) * hx * hy + fabsf(r.r1.z) * hx * hz + fabsf(r.r2.x) * hy * hz);
+    return q <= 27.9f;
+}
+
+// One thread per Gaussian in Morton order: its record, its box as a leaf of the wide tree,
+// and (eight neighbouring lanes together) the box of its level-1 node.
 __global__ void __launch_bounds__(256) k_gather_recs(int64_t P, const int32_t* __restrict__ perm,
                                                      const float* __restrict__ means, const float* __restrict__ values,
                                                      const float* __restrict__ weights,
                                                      const float* __restrict__ conics, const float4* __restrict__ boxes,
-                                                     GaussRec* __restrict__ recs) {
+                                                     GaussRec* __restrict__ recs, float4* __restrict__ leaf,
+                                                     float4* __restrict__ level1) {
     const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (g >= P) return;
-    const int64_t o = perm[g];
-    GaussRec r;
-    r.r0 = make_float4(means[3 * o], means[3 * o + 1], means[3 * o + 2], weights[o]);
-    r.r1 = make_float4(conics[6 * o], conics[6 * o + 1], conics[6 * o + 2], conics[6 * o + 3]);
-    r.r2 = make_float4(conics[6 * o + 4], conics[6 * o + 5], values[o], 0.f);
-    r.r3 = boxes[2 * o];
-    r.r4 = boxes[2 * o + 1];
-    recs[g] = r;
+    Box6 b = empty_box();
+    if (g < P) {
+        const int64_t o = perm[g];
+        GaussRec r;
+        r.r0 = make_float4(means[3 * o], means[3 * o + 1], means[3 * o + 2], weights[o]);
+        r.r1 = make_float4(conics[6 * o], conics[6 * o + 1], conics[6 * o + 2], conics[6 * o + 3]);
+        r.r2 = make_float4(conics[6 * o + 4], conics[6 * o + 5], values[o], 0.f);
+        r.r3 = boxes[2 * o];
+        r.r4 = boxes[2 * o + 1];
+        r.r2.w = window_covers(r) ? 1.f : 0.f;
+        recs[g] = r;
+        b = Box6{r.r3.x, r.r3.y, r.r3.z, r.r4.x, r.r4.y, r.r4.z};
+        store_box(leaf, g, b);
+    }
+    grow(b, shfl_xor_box(b, 1));
+    grow(b, shfl_xor_box(b, 2));
+    grow(b, shfl_xor_box(b, 4));
+    if (g < P && (g & (kWideLeaves - 1)) == 0) store_box(level1, g / kWideLeaves, b);
 }
 
 // Sorted sample slots: (x, y, z, caller index as int bits); padding slots carry NaN
-// coordinates and index -1.  One warp per tile of 32 slots also splits the tile into at
-// most kGroups contiguous lane groups: a group [a, b) is split at the Morton bit where
-// its first and last keys first differ when both halves' boxes are at most half the
-// group's size (half-perimeter).  A tile that straddles a jump of the Z-order curve thus
-// becomes compact groups instead of one box spanning the jump.  Writes one box per group
-// slot (unused slots: empty box) and the group descriptor of the tile.
-struct WBox {
-    float lx, ly, lz, hx, hy, hz;
-};
-
-__device__ __forceinline__ WBox warp_box(bool in, float x, float y, float z) {
-    WBox b;
-    b.lx = in ? x : INFINITY;
-    b.ly = in ? y : INFINITY;
-    b.lz = in ? z : INFINITY;
-    b.hx = in ? x : -INFINITY;
-    b.hy = in ? y : -INFINITY;
-    b.hz = in ? z : -INFINITY;
-    for (int off = 16; off > 0; off >>= 1) {
-        b.lx = fminf(b.lx, __shfl_xor_sync(0xffffffffu, b.lx, off));
-        b.ly = fminf(b.ly, __shfl_xor_sync(0xffffffffu, b.ly, off));
-        b.lz = fminf(b.lz, __shfl_xor_sync(0xffffffffu, b.lz, off));
-        b.hx = fmaxf(b.hx, __shfl_xor_sync(0xffffffffu, b.hx, off));
-        b.hy = fmaxf(b.hy, __shfl_xor_sync(0xffffffffu, b.hy, off));
-        b.hz = fmaxf(b.hz, __shfl_xor_sync(0xffffffffu, b.hz, off));
-    }
-    return b;
-}
-
-__device__ __forceinline__ float half_perimeter(const WBox& b) {
-    return (b.hx - b.lx) + (b.hy - b.ly) + (b.hz - b.lz);
-}
-
-// A lane group is split when both halves' boxes have at most this fraction of the whole's
-// half-perimeter (0.65 measured best for the backward's candidate rows: 0.5 gathers 9.4e9
-// rows at 2M x 16M, 0.65 8.5e9; from 0.8 on the extra leaves cost more than they save).
-constexpr float kTileSplitRatio = 0.65f;
-
-// Split lane of group [a, b), or -1 (warp-uniform).
-__device__ int try_split(int a, int b, uint32_t key, int lane, float x, float y, float z) {
-    if (b - a < 2) return -1;
-    const uint32_t ka = __shfl_sync(0xffffffffu, key, a), kb = __shfl_sync(0xffffffffu, key, b - 1);
-    if (ka == kb) return -1;
-    const int bit = 31 - __clz(ka ^ kb);
-    const bool in = lane >= a && lane < b;
-    const uint32_t hi = __ballot_sync(0xffffffffu, in && ((key >> bit) & 1u));
-    const int m = __ffs(hi) - 1;  // keys are sorted: a < m < b
-    const WBox B = warp_box(in, x, y, z);
-    const WBox B1 = warp_box(in && lane < m, x, y, z);
-    const WBox B2 = warp_box(in && lane >= m, x, y, z);
-    const float h = half_perimeter(B);
-    return fmaxf(half_perimeter(B1), half_perimeter(B2)) <= kTileSplitRatio * h ? m : -1;
-}
-
-__global__ void __launch_bounds__(256) k_sample_tiles(int64_t S, int64_t n_tiles, const float* __restrict__ samples,
+// coordinates and index -1.
+__global__ void __launch_bounds__(256) k_sample_slots(int64_t S, int64_t n_slots, const float* __restrict__ samples,
                                                       const int32_t* __restrict__ perm,
-                                                      const uint32_t* __restrict__ skeys, float4* __restrict__ s_sorted,
-                                                      float4* __restrict__ group_boxes, uint32_t* __restrict__ gdesc,
-                                                      int with_groups) {
+                                                      float4* __restrict__ s_sorted) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t t = i >> 5;
-    if (t >= n_tiles) return;
-    const int lane = threadIdx.x & 31;
+    if (i >= n_slots) return;
     float x = NAN, y = NAN, z = NAN;
     int o = -1;
-    uint32_t key = 0xffffffffu;
-    if (!with_groups) {
-        // pass 1 (build_bvh): gather the sorted samples
-        if (i < S) {
-            o = perm[i];
-            x = samples[3 * (int64_t)o];
-            y = samples[3 * (int64_t)o + 1];
-            z = samples[3 * (int64_t)o + 2];
-        }
-        s_sorted[i] = make_float4(x, y, z, __int_as_float(o));
-        return;  // warp-uniform
+    if (i < S) {
+        o = perm[i];
+        x = samples[3 * (int64_t)o];
+        y = samples[3 * (int64_t)o + 1];
+        z = samples[3 * (int64_t)o + 2];
     }
-    // pass 2 (first user of the lane groups): read them back from s_sorted
-    const float4 sp = s_sorted[i];
-    x = sp.x;
-    y = sp.y;
-    z = sp.z;
-    o = __float_as_int(sp.w);
-    if (i < S) key = skeys[i];
-    const int nvalid = __popc(__ballot_sync(0xffffffffu, o >= 0));
-    int starts[kGroups + 1];
-    int ng = 1;
-    starts[0] = 0;
-    const int m = try_split(0, nvalid, key, lane, x, y, z);
-    if (m >= 0) {
-        const int m1 = try_split(0, m, key, lane, x, y, z);
-        const int m2 = try_split(m, nvalid, key, lane, x, y, z);
-        if (m1 >= 0) starts[ng++] = m1;
-        starts[ng++] = m;
-        if (m2 >= 0) starts[ng++] = m2;
-    }
-    for (int g = ng; g <= kGroups; g++) starts[g] = 32;
-    for (int g = 0; g < kGroups; g++) {
-        const int a = starts[g], b = (g + 1 < ng) ? starts[g + 1] : nvalid;
-        WBox B;
-        if (g < ng) {
-            B = warp_box(lane >= a && lane < b, x, y, z);
-        } else {
-            B.lx = B.ly = B.lz = INFINITY;
-            B.hx = B.hy = B.hz = -INFINITY;
-        }
-        if (lane == 0) {
-            group_boxes[2 * (kGroups * t + g)] = make_float4(B.lx, B.ly, B.lz, 0.f);
-            group_boxes[2 * (kGroups * t + g) + 1] = make_float4(B.hx, B.hy, B.hz, 0.f);
-        }
-    }
-    if (lane == 0)
-        gdesc[t] = (uint32_t)starts[1] | ((uint32_t)starts[2] << 8) | ((uint32_t)starts[3] << 16) |
-                   ((uint32_t)ng << 24);
+    s_sorted[i] = make_float4(x, y, z, __int_as_float(o));
 }
 
 // Per sorted sample: (gO / W, -gO * out / W, gW, 1) if W > 0.01, else zeros
@@ -331,18 +255,19 @@ cudaError_t launch_preprocess(int64_t P, const float* means, const float* scales
 
 cudaError_t launch_gather_recs(int64_t P, const int32_t* perm, const float* means, const float* values,
                                const float* weights, const float* conics, const float4* boxes, GaussRec* recs,
-                               cudaStream_t st) {
+                               float4* tree_boxes, bool levels, cudaStream_t st) {
     if (P <= 0) return cudaSuccess;
-    k_gather_recs<<<nb256(P), 256, 0, st>>>(P, perm, means, values, weights, conics, boxes, recs); gvc::note_launch();
-    return cudaGetLastError();
+    const WideTreeSize z = wide_tree_size(P);
+    k_gather_recs<<<nb256(P), 256, 0, st>>>(P, perm, means, values, weights, conics, boxes, recs, tree_boxes,
+                                            tree_boxes + 2 * z.n[0]); gvc::note_launch();
+    if (!levels) return cudaGetLastError();
+    return launch_wide_levels(z, tree_boxes, st);
 }
 
-cudaError_t launch_sample_tiles(int64_t S, int64_t n_tiles, const float* samples, const int32_t* perm,
-                                const uint32_t* skeys, float4* s_sorted, float4* group_boxes, uint32_t* gdesc,
-                                bool with_groups, cudaStream_t st) {
-    if (n_tiles <= 0) return cudaSuccess;
-    k_sample_tiles<<<nb256(n_tiles * 32), 256, 0, st>>>(S, n_tiles, samples, perm, skeys, s_sorted, group_boxes,
-                                                        gdesc, with_groups ? 1 : 0); gvc::note_launch();
+cudaError_t launch_sample_slots(int64_t S, int64_t n_slots, const float* samples, const int32_t* perm,
+                                float4* s_sorted, cudaStream_t st) {
+    if (n_slots <= 0) return cudaSuccess;
+    k_sample_slots<<<nb256(n_slots), 256, 0, st>>>(S, n_slots, samples, perm, s_sorted); gvc::note_launch();
     return cudaGetLastError();
 }
 

@@ -1,150 +1,9 @@
-// render.cu -- fused traversal + Gaussian evaluation of the mixture field at 32-sample
-// tiles (forward), and the per-Gaussian end of the backward.
-//
-// Forward per tile (replaces FORWARD::sampleRenderCUDA / renderCUDA + normalizeCUDA,
-// diff-gaussian-rasterization/cuda_rasterizer/forward.cu:116-274): one warp per tile of
-// 32 Morton-sorted samples walks the Gaussian LBVH with the tile's box; candidate
-// Gaussians are staged 32 at a time in shared memory and every lane evaluates its own
-// sample against each of them, accumulating W and V in registers (no atomics).
-//
-// k_finalize turns the backward's eleven sums per Gaussian (bwd_gauss.cu, bwd_tc.cu) into
-// the gradients of its parameters (backward.cu:9-125).
-//
-// Pair math follows forward.cu:224-256.
-#include "pair.cuh"
+// render.cu -- the per-Gaussian end of the backward: the eleven sums of bwd_gauss.cu or
+// bwd_tc.cu become the gradients of a Gaussian's parameters
+// (diff-gaussian-rasterization/cuda_rasterizer/backward.cu:9-125).
 #include "render.cuh"
-#include "traverse.cuh"
 
 namespace gvc {
-
-constexpr int kWarpsPerBlock = 4;
-
-// --------------------------------------------------------------------------------
-// Forward
-// --------------------------------------------------------------------------------
-template <bool COUNT>
-struct FwdVisitor {
-    const GaussRec* __restrict__ recs;
-    float4* batch;  // shared [32 * 5]
-    float x, y, z;
-    bool valid;
-    float W, V;
-    int ncand, ncontrib;
-
-    __device__ __forceinline__ void operator()(const int* c, int nb) {
-        const int lane = threadIdx.x & 31;
-        if (lane < nb) {
-            // stage one record per lane; the conic becomes base-2 power coefficients with
-            // the off-diagonal entries doubled (symmetric quadratic form in 9 operations)
-            const float4* rp = reinterpret_cast<const float4*>(recs + c[lane]);
-            const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1), r2 = __ldg(rp + 2), r3 = __ldg(rp + 3),
-                         r4 = __ldg(rp + 4);
-            batch[lane * 5 + 0] = r0;
-            batch[lane * 5 + 1] = make_float4(kHalfLog2e * r1.x, 2.f * kHalfLog2e * r1.y, 2.f * kHalfLog2e * r1.z,
-                                              kHalfLog2e * r1.w);
-            batch[lane * 5 + 2] = make_float4(2.f * kHalfLog2e * r2.x, kHalfLog2e * r2.y, r2.z, 0.f);
-            batch[lane * 5 + 3] = r3;
-            batch[lane * 5 + 4] = r4;
-        }
-        __syncwarp();
-        // Four Gaussians per step, branch-free inside the step: four independent
-        // dependency chains per lane; a step is skipped only when no lane of the warp is
-        // inside any of the four boxes.
-        for (int g0 = 0; g0 < nb; g0 += 4) {
-            bool in[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int g = g0 + j;
-                in[j] = false;
-                if (g < nb) {
-                    const float4 r3 = batch[g * 5 + 3], r4 = batch[g * 5 + 4];
-                    in[j] = valid && r3.x <= x && x <= r4.x && r3.y <= y && y <= r4.y && r3.z <= z && z <= r4.z;
-                }
-            }
-            if (!__any_sync(0xffffffffu, in[0] | in[1] | in[2] | in[3])) continue;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int g = min(g0 + j, nb - 1);
-                const float4 r0 = batch[g * 5 + 0], r1 = batch[g * 5 + 1], r2 = batch[g * 5 + 2];
-                const float dx = x - r0.x, dy = y - r0.y, dz = z - r0.z;
-                const float p2 = dx * fmaf(r1.x, dx, fmaf(r1.y, dy, r1.z * dz)) + dy * fmaf(r1.w, dy, r2.x * dz) +
-                                 dz * (r2.y * dz);
-                const bool c = in[j] && p2 >= kLog2Floor && p2 <= 0.0f;
-                const float wt = c ? r0.w * ex2_approx(p2) : 0.0f;
-                W += wt;
-                V = fmaf(wt, r2.z, V);
-                if (COUNT) {
-                    ncand += in[j] ? 1 : 0;
-                    ncontrib += c ? 1 : 0;
-                }
-            }
-        }
-        __syncwarp();
-    }
-};
-
-// Lane group of this lane in a tile with descriptor gd (see k_sample_tiles).
-__device__ __forceinline__ int lane_group(uint32_t gd, int lane) {
-    return (lane >= (int)(gd & 0xffu)) + (lane >= (int)((gd >> 8) & 0xffu)) + (lane >= (int)((gd >> 16) & 0xffu));
-}
-
-template <bool COUNT>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) k_forward(const float4* __restrict__ s_sorted,
-                                                                 const float4* __restrict__ group_boxes,
-                                                                 const uint32_t* __restrict__ gdesc, int n_tiles,
-                                                                 const BvhNode* __restrict__ nodes,
-                                                                 const GaussRec* __restrict__ recs,
-                                                                 float* __restrict__ out_cells,
-                                                                 float* __restrict__ out_weights, int* status,
-                                                                 unsigned long long* stats) {
-    __shared__ int s_stack[kWarpsPerBlock][kStackCap];
-    __shared__ int s_cand[kWarpsPerBlock][kCandCap];
-    __shared__ float4 s_batch[kWarpsPerBlock][32 * 5];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tile = blockIdx.x * kWarpsPerBlock + warp;
-    if (tile >= n_tiles) return;
-    const float4 sp = s_sorted[(int64_t)tile * 32 + lane];
-    const int orig = __float_as_int(sp.w);
-    const uint32_t gd = gdesc[tile];
-    const int ng = (int)(gd >> 24), mygroup = lane_group(gd, lane);
-    FwdVisitor<COUNT> vis{recs, s_batch[warp], sp.x, sp.y, sp.z, false, 0.f, 0.f, 0, 0};
-    TravCount tc;
-    int st = 0;
-    for (int g = 0; g < ng; g++) {
-        const int64_t slot = (int64_t)tile * kGroups + g;
-        const float4 tlo = group_boxes[2 * slot], thi = group_boxes[2 * slot + 1];
-        vis.valid = orig >= 0 && mygroup == g;
-        st |= warp_traverse(nodes, make_float3(tlo.x, tlo.y, tlo.z), make_float3(thi.x, thi.y, thi.z),
-                            s_stack[warp], s_cand[warp], vis, tc);
-    }
-    if (orig >= 0) {
-        float o, w;
-        if (vis.W <= kWeightCutoff) {
-            o = -1.0f;
-            w = 0.0f;
-        } else {
-            o = vis.V / vis.W;
-            w = vis.W;
-        }
-        out_cells[orig] = o;
-        out_weights[orig] = w;
-    }
-    if (st && lane == 0) atomicOr(status, st);
-    if (COUNT) {
-        unsigned long long a = (unsigned long long)vis.ncand, b = (unsigned long long)vis.ncontrib;
-        for (int off = 16; off > 0; off >>= 1) {
-            a += __shfl_xor_sync(0xffffffffu, a, off);
-            b += __shfl_xor_sync(0xffffffffu, b, off);
-        }
-        if (lane == 0) {
-            atomicAdd(&stats[0], a);
-            atomicAdd(&stats[1], b);
-            atomicMax(&stats[3], (unsigned long long)tc.max_sp);
-            atomicAdd(&stats[5], (unsigned long long)tc.leaves);
-            atomicAdd(&stats[6], (unsigned long long)tc.nodes);
-        }
-    }
-}
 
 // --------------------------------------------------------------------------------
 // Finalize: gacc [P][16] (caller order) -> dmeans, dvalues, dweights and the
@@ -299,21 +158,6 @@ __global__ void __launch_bounds__(256) k_finalize(int P, const float* __restrict
 // Launchers
 // --------------------------------------------------------------------------------
 static inline unsigned nblk(int64_t n, int per) { return (unsigned)((n + per - 1) / per); }
-
-cudaError_t launch_forward(const FwdArgs& a, cudaStream_t st) {
-    if (a.n_tiles <= 0) return cudaSuccess;
-    if (a.count) {
-        k_forward<true><<<nblk(a.n_tiles, kWarpsPerBlock), kWarpsPerBlock * 32, 0, st>>>(
-            a.s_sorted, a.tile_boxes, a.gdesc, (int)a.n_tiles, a.gnodes, a.recs, a.out_cells, a.out_weights, a.status,
-            a.stats);
-    } else {
-        k_forward<false><<<nblk(a.n_tiles, kWarpsPerBlock), kWarpsPerBlock * 32, 0, st>>>(
-            a.s_sorted, a.tile_boxes, a.gdesc, (int)a.n_tiles, a.gnodes, a.recs, a.out_cells, a.out_weights, a.status,
-            a.stats);
-    }
-    gvc::note_launch();
-    return cudaGetLastError();
-}
 
 cudaError_t launch_finalize(int64_t P, const float* gacc, const float* scales, const float* rots, const float* conics,
                             float sm, int ref_compat, float* dmeans, float* dscales, float* drots, float* dvalues,

@@ -1,23 +1,95 @@
 // render.cuh -- launch interfaces of the forward / backward evaluation kernels and
 // of the preprocessing kernels (prep.cu).
 #pragma once
-#include "gvc_internal.cuh"
+#include "wide_tree.cuh"
 
 namespace gvc {
 
+// Candidate log of the forwards, read by the tensor-core backward instead of walking the
+// LBVH again: the Gaussians whose boxes overlap a block's coarse groups in order in the
+// block's kCandLogPerBlock slots, coarse group g's ending at cend[blk * 8 + g], and with each
+// a byte whose bit b says that it meets the block's group b (box overlap and window test;
+// fwd_blocks.cu writes them, after the other forwards launch_log_masks does); a block
+// with more candidates than slots gets -1 for every group, and the backward walks.
+constexpr int kCandLogPerBlock = 4096;
+
+struct CandLog {
+    int32_t* ids = nullptr;  // this block's slots, or null (no log)
+    uint8_t* masks = nullptr;
+    int pos = 0;             // candidates appended (warp-uniform)
+    bool over = false;
+    int gend = 0;  // on lane g: end of group g
+
+    // appends lanes 0 .. n - 1
+    __device__ __forceinline__ void append(int n, int id, uint32_t mask) {
+        const int lane = threadIdx.x & 31;
+        if (pos + n > kCandLogPerBlock) {
+            over = true;
+        } else if (lane < n) {
+            ids[pos + lane] = id;
+            if (masks) masks[pos + lane] = (uint8_t)mask;
+        }
+        pos += n;
+    }
+    __device__ __forceinline__ void end_group(int g) {
+        if ((threadIdx.x & 31) == g) gend = pos;
+    }
+    __device__ __forceinline__ void finish(int32_t* cend_blk, int ng) {
+        if (ids && (int)(threadIdx.x & 31) < ng) cend_blk[threadIdx.x & 31] = over ? -1 : gend;
+    }
+};
+
 struct FwdArgs {
+    int64_t P;
     const float4* s_sorted;
-    const float4* tile_boxes;  // group boxes [n_tiles * kGroups]
-    const uint32_t* gdesc;     // [n_tiles]
-    int64_t n_tiles;
-    const BvhNode* gnodes;
-    const GaussRec* recs;
+    int64_t S;
+    const uint2* bdesc;    // [n_blocks] block-group descriptors
+    const float4* bboxes;  // [n_blocks * 8] block-group boxes (lo, hi)
+    WideTree tree;         // over the Gaussians in Morton order (level 0: their AABBs)
+    const BvhNode* nodes;  // the LBVH over the same order: walked instead when given
+    const GaussRec* recs;  // the same order
     float* out_cells;
     float* out_weights;
+    float2* out_sorted;    // (out, W) per sorted slot, read by the backward's rows; or null
+    int32_t* clog;         // candidate log, or null
+    uint8_t* cmask;        // its masks (FP32 forward)
+    int32_t* cend;
+    const uint2* fdesc;    // the block's finer groups (the bits of cmask)
+    const float4* fboxes;
     int* status;
     unsigned long long* stats;
     bool count;
 };
+// fwd_blocks.cu: FP32, one warp per block of 128 samples (or per part of it)
+cudaError_t launch_forward_blocks(const FwdArgs& a, cudaStream_t st);
+// Rows per warp of it by the LBVH, or 0 where launch_forward_cta's three warps per block are
+// faster.  us at 32 rows / three warps / 128 rows: 200k Gaussians x 60k samples
+// 797 / 895 / 1423, x 262k 901 / 632 / 833, x 524k 1122 / 729 / 698, x 4M 3971 / 2427 / 1741;
+// 300k clustered x 524k 779 / 528 / 605; 1M clustered x 130k 2377 / 2413 / 4006,
+// x 1M 3121 / 1869 / 2152, x 4M 6063 / 3689 / 3206; 20k x 60k 102 / 122 / 173.
+inline int forward_linked_rows(int64_t S, int64_t P) {
+    return S < 100000 ? 32 : S >= 500000 && S >= 2 * P ? 128 : 0;
+}
+// cta.cu: by the LBVH
+cudaError_t launch_forward_cta(const FwdArgs& a, cudaStream_t st);
+// fwd_points.cu: FP32, one warp per sample (no candidate log)
+cudaError_t launch_forward_points(const FwdArgs& a, cudaStream_t st);
+// fwd_tc.cu: the exponent on tcgen05, one CTA per block
+cudaError_t launch_forward_tc(const FwdArgs& a, cudaStream_t st);
+
+// Groups of the 128-sample blocks (cta.cu): a run of rows splits where both halves' boxes have
+// at most `ratio` of the whole's half-perimeter.  kBlockSplit for the FP32 forward and the
+// tensor-core backward; with the tensor-core kernels the forward's groups are coarser.
+// FP32 forward and tensor-core backward at 0.45 / 0.55 / 0.65 / 0.75, ms: 2M x 16M
+// 11.3 / 11.1 / 11.1 / 12.4 and 17.3 / 15.8 / 14.6 / 14.1; 1M x 4M clustered forward
+// 2.84 / 2.54 / 2.51 / 2.64; 256^3 grid x 500k forward 5.42 / 5.42 / 5.42 / 6.91.
+constexpr float kBlockSplit = 0.65f;
+constexpr float kBlockSplitCoarse = 0.45f;
+// Block groups with `ratio`; with bdesc2 also a second set with `ratio2` from the same
+// loaded rows (one launch).
+cudaError_t launch_sample_blocks(int64_t S, const float4* s_sorted, const uint32_t* skeys, uint2* bdesc,
+                                 float4* bboxes, float ratio, cudaStream_t st, uint2* bdesc2 = nullptr,
+                                 float4* bboxes2 = nullptr, float ratio2 = 0.f);
 
 struct BwdArgs {
     int64_t P;
@@ -29,124 +101,50 @@ struct BwdArgs {
     const float* values;
     const float* weights;
     // tensor-core sums
-    const int32_t* gperm;      // LBVH order -> caller idx
-    int64_t n_slots;           // sorted sample slots
+    const int32_t* gperm;      // Morton order -> caller idx
+    int64_t S;
+    const uint2* bdesc;        // block groups
+    const float4* bboxes;
     const float4* s_grad;      // (x, y, z, gx) per sorted slot
     const float* s_gyz;        // gyz per sorted slot
     const uint8_t* s_ok;       // W > 0.01 per sorted slot (pair statistics)
-    const BvhNode* gnodes;     // Gaussian LBVH
-    int64_t g_internal;        // its internal nodes
-    bool stackless;            // traverse by escape edges (warp_traverse_stackless)
-    const int32_t* clog;       // the forward's candidate log (null: traverse)
+    const BvhNode* nodes;      // LBVH over the Gaussians in Morton order
+    const int32_t* clog;       // the forward's candidate log (null: walk)
+    const uint8_t* cmask;      // its masks
     const int32_t* cend;
-    const uint2* cdesc;        // the forward's block groups (the log's groups)
-    const GaussRec* recs;      // LBVH order
+    const uint2* cdesc;        // the coarse groups of the log
+    const GaussRec* recs;      // Morton order
     float* gacc;               // [P][16] caller order
     int* status;
     unsigned long long* stats;
     bool count;
 };
 
-cudaError_t launch_forward(const FwdArgs& a, cudaStream_t st);
-
-// Candidate log of the block-group forwards, read by the tensor-core backward instead of
-// walking the Gaussian LBVH again: the forward's producer appends the candidates of a
-// block's groups in order to the block's kCandLogPerBlock slots, and group g's candidates
-// end at cend[blk * 8 + g]; a block with more candidates than slots gets -1 for every
-// group, and the backward walks the tree for it.
-constexpr int kCandLogPerBlock = 4096;
-
-struct CandLog {
-    int32_t* ids = nullptr;  // this block's slots, or null (no log)
-    int pos = 0;             // candidates appended (warp-uniform)
-    bool over = false;
-    int gend = 0;  // on lane g: end of group g
-
-    __device__ __forceinline__ void append(const int* c, int nb) {
-        if (!ids) return;
-        const int lane = threadIdx.x & 31;
-        if (pos + nb <= kCandLogPerBlock) {
-            if (lane < nb) ids[pos + lane] = c[lane];
-        } else {
-            over = true;
-        }
-        pos += nb;
-    }
-    __device__ __forceinline__ void end_group(int g) {
-        if ((threadIdx.x & 31) == g) gend = pos;
-    }
-    __device__ __forceinline__ void finish(int32_t* cend_blk, int ng) {
-        if (ids && (int)(threadIdx.x & 31) < ng) cend_blk[threadIdx.x & 31] = over ? -1 : gend;
-    }
-};
-
-// cta.cu: CTA-level forward on 128-sample blocks (tensor-core or SIMT exponent)
-struct CtaArgs {
-    const float4* s_sorted;
-    int64_t S;
-    const uint2* bdesc;    // [n_blocks] block-group descriptors
-    const float4* bboxes;  // [n_blocks * 8] block-group boxes (lo, hi)
-    const BvhNode* gnodes;
-    int64_t n_internal;    // internal nodes of gnodes
-    bool stackless;        // traverse by escape edges (warp_traverse_stackless)
-    int32_t* clog;         // candidate log [n_blocks * kCandLogPerBlock], or null
-    int32_t* cend;         // group ends of the log [n_blocks * 8]
-    const GaussRec* recs;
-    float* out_cells;
-    float* out_weights;
-    float2* out_sorted;    // (out, W) per sorted slot, read by the backward's sample records; or null
-    int* status;
-    unsigned long long* stats;
-    bool count;
-};
-// Block groups split where both halves' boxes have at most `ratio` of the whole's
-// half-perimeter: kBlockSplitForward for the forward, kBlockSplitBackward (finer) for the
-// tensor-core backward.
-constexpr float kBlockSplitForward = 0.45f;
-constexpr float kBlockSplitBackward = 0.65f;
-// Block groups with `ratio`; with bdesc2 also a second set with `ratio2` from the same
-// loaded rows (one launch).
-cudaError_t launch_sample_blocks(int64_t S, const float4* s_sorted, const uint32_t* skeys, uint2* bdesc,
-                                 float4* bboxes, float ratio, cudaStream_t st, uint2* bdesc2 = nullptr,
-                                 float4* bboxes2 = nullptr, float ratio2 = 0.f);
-cudaError_t launch_forward_cta(const CtaArgs& a, bool tc, cudaStream_t st);
-// fwd_tc.cu: the forward with the exponent on tcgen05 (launch_forward_cta(a, true) calls it)
-cudaError_t launch_forward_tc(const CtaArgs& a, cudaStream_t st);
 cudaError_t launch_tc_gemm_test(const void* A, const void* B, int N, float* D, int* status, cudaStream_t st);
 // One block waiting on an mbarrier nothing arrives on: the bounded wait runs out and
 // records kStatusTimeout (tests the host-side report of device timeouts).
 cudaError_t launch_wait_timeout_test(int* status, cudaStream_t st);
 
-// bwd_gauss.cu: gradient rows in chunks of 16, a tree of boxes over them (level 0: chunks,
-// level 1: 8 chunks, every further level: 32 children per node), and the Gaussian-owned
-// sums that walk it
+// bwd_gauss.cu: gradient rows in chunks of 16 under a wide tree (leaves: chunks), and the
+// Gaussian-owned sums that walk it
 constexpr int kChunkRows = 16;
 constexpr int kChunkFloats = 5 * kChunkRows;  // x, y, z, gx, gyz
-constexpr int kNodeChunks = 8;                // chunks of a level-1 node
-constexpr int kNodeRows = kNodeChunks * kChunkRows;
-constexpr int kTreeLevels = 6;
-struct SampleTree {
-    const float4* box[kTreeLevels];  // per level: (lo, hi) of each node
-    int n[kTreeLevels];
-    int top;
-};
-struct SampleTreeSize {
-    int64_t n[kTreeLevels];
-    int top;
-    int64_t boxes;      // all levels together
+constexpr int kRowsPerNode = kWideLeaves * kChunkRows;
+struct RowTreeSize {
+    WideTreeSize tree;
     size_t rows_bytes;  // gradient rows
 };
-SampleTreeSize sample_tree_size(int64_t S);
+RowTreeSize row_tree_size(int64_t S);
 // out_sorted: the forward's (out, W) per sorted slot when the caller's out_cells /
 // out_weights are that forward's outputs (else null: they are gathered).
-cudaError_t launch_backward_rows(int64_t S, const SampleTreeSize& z, const float4* s_sorted, const float2* out_sorted,
+cudaError_t launch_backward_rows(int64_t S, const RowTreeSize& z, const float4* s_sorted, const float2* out_sorted,
                                  const float* out_cells, const float* out_weights, const float* gout, const float* gw,
-                                 float* rows, float4* boxes, SampleTree* tree, cudaStream_t st);
-cudaError_t launch_backward_gauss(const BwdArgs& a, const SampleTree& tree, const float* rows, cudaStream_t st);
+                                 float* rows, float4* boxes, cudaStream_t st);
+cudaError_t launch_backward_gauss(const BwdArgs& a, const WideTree& tree, const float* rows, cudaStream_t st);
 
-// bwd_tc.cu: backward on 128-sample blocks with the reduction over samples on tcgen05
-cudaError_t launch_backward_cta(const BwdArgs& a, int64_t n_blocks, const uint2* bdesc, const float4* bboxes,
-                                cudaStream_t st);
+// bwd_tc.cu: reduction over samples on tcgen05, one CTA per 128 samples
+cudaError_t launch_backward_tc(const BwdArgs& a, cudaStream_t st);
+cudaError_t launch_log_masks(const BwdArgs& a, uint8_t* cmask, cudaStream_t st);
 cudaError_t launch_finalize(int64_t P, const float* gacc, const float* scales, const float* rots, const float* conics,
                             float sm, int ref_compat, float* dmeans, float* dscales, float* drots, float* dvalues,
                             float* dweights, cudaStream_t st);
@@ -154,12 +152,14 @@ cudaError_t launch_finalize(int64_t P, const float* gacc, const float* scales, c
 // prep.cu (compiled without FMA contraction so that its arithmetic matches the oracle)
 cudaError_t launch_preprocess(int64_t P, const float* means, const float* scales, const float* rots,
                               const float* weights, float sm, float* conics_out, float4* boxes_out, cudaStream_t st);
+// Records in Morton order, and their wide tree at `tree_boxes` (levels false: its two lowest
+// levels only).
 cudaError_t launch_gather_recs(int64_t P, const int32_t* perm, const float* means, const float* values,
                                const float* weights, const float* conics, const float4* boxes, GaussRec* recs,
-                               cudaStream_t st);
-cudaError_t launch_sample_tiles(int64_t S, int64_t n_tiles, const float* samples, const int32_t* perm,
-                                const uint32_t* skeys, float4* s_sorted, float4* group_boxes, uint32_t* gdesc,
-                                bool with_groups, cudaStream_t st);
+                               float4* tree_boxes, bool levels, cudaStream_t st);
+// Sorted sample slots: (x, y, z, bits of the caller's index or -1).
+cudaError_t launch_sample_slots(int64_t S, int64_t n_slots, const float* samples, const int32_t* perm,
+                                float4* s_sorted, cudaStream_t st);
 // out_sorted: the forward's (out, W) per sorted slot when the caller's out_cells /
 // out_weights are that forward's outputs (else null: they are gathered).
 cudaError_t launch_sample_grads(int64_t n_slots, const float4* s_sorted, const float2* out_sorted,

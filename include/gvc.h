@@ -50,53 +50,48 @@ typedef enum {
                                    over samples as a tcgen05 BF16 3-way split GEMM in TMEM,
                                    FP32 atomics (not bitwise reproducible)                  */
     GVC_OPT_EVAL_PATH = 3,  /* forward evaluation kernel (all compute the same field):
-                               0 = FP32 exponent, one CTA per 128-sample block: a producer warp
-                                   walks the Gaussian LBVH and stages batches, two consumer
-                                   warps evaluate two samples per thread (default, fastest),
-                               1 = tensor-core exponent: the same pipeline with the power as a
-                                   tcgen05 BF16 3-way split MMA into TMEM,
-                               2 = FP32 exponent, one warp per 32-sample tile               */
+                               0, 2 = FP32 exponent, one warp per 128-sample block (default,
+                                   fastest; 2 named a kernel by 32-sample tiles),
+                               1 = tensor-core exponent: one CTA per block, the power as a
+                                   tcgen05 BF16 3-way split MMA into TMEM.
+                               With neither tensor-core kernel selected, samples that are
+                               sparse among the Gaussians (S * S < 360000 P) take one warp
+                               each and the walks go by a wide tree; with one selected, by
+                               the Gaussian LBVH, in one order of the sums.                 */
     GVC_OPT_COUNT_PAIRS = 4,/* 1 = record per-call pair counts (gvc_get_stats)            */
     GVC_OPT_TIME_KERNELS = 5,/* 1 = time the evaluation kernels with CUDA events on the
                                 caller's stream (gvc_get_stats)                          */
-    GVC_OPT_TRAVERSAL = 6,  /* Gaussian-LBVH traversal of the block-group forwards (eval
-                               paths 0 and 1) and of the tensor-core backward (same
-                               candidates, same results up to summation order):
-                               0 = warp-cooperative with a shared-memory node stack (default),
-                               1 = stackless: level-synchronous descent while a level's
-                                   overlapping nodes fit the warp, then one subtree per lane
-                                   walked by escape edges stored in the nodes              */
+    GVC_OPT_TRAVERSAL = 6,  /* accepts 0 and 1; without effect (1 named a walk of the
+                               Gaussian LBVH without a stack, slower at every size)        */
     GVC_OPT_CAND_LOG = 7    /* 1 (default) = when the tensor-core backward is selected, the
-                               block-group forward records every block's candidate Gaussians
-                               (kCandLogPerBlock = 4096 per 128-sample block, 16 KB) and the
-                               backward reads them back instead of walking the Gaussian LBVH
-                               again (each of its finer block groups keeps the candidates of
-                               the enclosing forward group whose boxes overlap its own);
-                               blocks with more candidates are walked, and without device
-                               memory for the log the forward runs without it.
+                               forward records the candidates of each 128-sample block (4096
+                               slots, 20 KB with a byte each for the block's groups that they
+                               meet) and the backward reads them back instead of walking the
+                               tree of Gaussians again; blocks with more are walked, and
+                               without device memory for the log the forward runs without it.
                                0 = always walk.                                            */
 } gvc_option;
 
 typedef struct {
-    int64_t fwd_candidates;   /* (sample, Gaussian) pairs with the sample inside the AABB   */
+    int64_t fwd_candidates;   /* evaluated (sample, Gaussian) pairs with the sample inside the AABB */
     int64_t fwd_contributing; /* ... and -14 <= power <= 0                                  */
     int64_t bwd_contributing; /* contributing pairs of samples with W > 0.01 (Gaussian-owned
                                  backward: of samples with a non-zero gradient)            */
-    int32_t max_stack_fwd;    /* deepest traversal stack seen (entries)                     */
+    int32_t max_stack_fwd;    /* 0 (the walks have no stack that could overflow)            */
     int32_t max_stack_bwd;
     double fwd_kernel_ms;     /* summed duration of the forward evaluation kernel          */
     double bwd_kernel_ms;     /* summed duration of the backward evaluation kernel         */
     int64_t fwd_kernel_calls; /* launches timed since the option was set                   */
     int64_t bwd_kernel_calls;
-    int64_t fwd_leaf_hits;    /* (tile, Gaussian) pairs evaluated by the forward            */
-    int64_t fwd_node_visits;  /* internal LBVH nodes popped by the forward traversal        */
+    int64_t fwd_leaf_hits;    /* (group, Gaussian) pairs whose boxes overlap                */
+    int64_t fwd_node_visits;  /* boxes tested by the forward's walks                        */
     int64_t bwd_leaf_hits;    /* (group, Gaussian) or (16-row chunk, Gaussian) pairs evaluated */
-    int64_t bwd_node_visits;  /* LBVH nodes popped, or sample-tree boxes tested                */
-    int64_t fwd_lane_evals;   /* (sample, Gaussian) lane slots the forward evaluated (CTA paths) */
-    int64_t bwd_rows;         /* (sample, Gaussian) rows the deterministic backward evaluated   */
+    int64_t bwd_node_visits;  /* boxes tested by the backward's walks                       */
+    int64_t fwd_lane_evals;   /* (sample, Gaussian) lane slots the forward evaluated         */
+    int64_t bwd_rows;         /* (sample, Gaussian) rows the backward evaluated              */
 } gvc_stats;
 
-/* Context: owns the sample ordering, both LBVHs and all workspace (no per-call
+/* Context: owns the sample ordering, both trees and all workspace (no per-call
    cudaMalloc once sizes stop growing).  Replaces the module statics samples_bvh,
    gaussian_bvh and stored_samples of diff-gaussian-rasterization/ext.cu:8-10.
    A context belongs to the device current at creation; use one context per thread. */
