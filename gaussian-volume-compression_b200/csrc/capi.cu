@@ -201,7 +201,7 @@ void gvc_ctx_destroy(gvc_ctx* ctx) {
         for (DevBuf* b : bufs) b->release();
     }
     DevBuf* bufs[] = {&c->s_sorted, &c->fwd_sorted, &c->blk_desc, &c->blk_boxes, &c->blk_desc_c, &c->blk_boxes_c, &c->b_rows, &c->b_boxes, &c->gtree, &c->s_grad, &c->s_gyz, &c->s_ok, &c->grec, &c->gtmp,
-                      &c->m_out_sorted, &c->knn_boxes, &c->ts_points, &c->ts_words, &c->ts_gt64, &c->scratch.gacc, &c->scratch.tmp_boxes, &c->scratch.tmp_out,
+                      &c->m_out_sorted, &c->knn_boxes, &c->ts_points, &c->ts_words, &c->cell_tree, &c->cell_recs, &c->scratch.gacc, &c->scratch.tmp_boxes, &c->scratch.tmp_out,
                       &c->clog, &c->cmask, &c->cend};
     for (DevBuf* b : bufs) b->release();
     if (c->d_status) cudaFree(c->d_status);
@@ -651,6 +651,25 @@ int gvc_sample_uniform(gvc_ctx* ctx, const int64_t* dims, const float* origin, c
     return GVC_OK;
 }
 
+// Orders the C cells of scratch tmp_boxes, builds their tree and locates the samples (conn4: of
+// tetrahedra).
+static int locate(gvc_ctx* ctx, LocateArgs& la, int64_t C, const float* pts, const int32_t* conn4, cudaStream_t st) {
+    la.C = C;
+    if (C > 0) {
+        const float4* boxes = scratch_of(ctx)->tmp_boxes.as<float4>();
+        GVC_CUDA(morton_sort_boxes(ctx->cells, C, boxes, st), "cell order");
+        GVC_CUDA(ctx->cell_tree.ensure(sizeof(float4) * 2 * wide_tree_size(C).boxes), "alloc cell tree");
+        if (conn4) GVC_CUDA(ctx->cell_recs.ensure(sizeof(float4) * 8 * C), "alloc cell records");
+        float4* recs = conn4 ? ctx->cell_recs.as<float4>() : nullptr;
+        la.cperm = ctx->cells.perm.as<int32_t>();
+        la.tree_boxes = ctx->cell_tree.as<float4>();
+        la.recs = recs;
+        GVC_CUDA(launch_cell_tree(C, la.cperm, boxes, pts, conn4, recs, ctx->cell_tree.as<float4>(), st), "cell tree");
+    }
+    GVC_CUDA(launch_locate(la, st), "locate samples");
+    return GVC_OK;
+}
+
 int gvc_sample_tets(gvc_ctx* ctx, int64_t npts, const float* pts, int64_t C, const int32_t* conn4,
                     const double* values, int64_t N, const float* samples, double* out, int64_t* cell_ids,
                     void* stream) {
@@ -662,20 +681,19 @@ int gvc_sample_tets(gvc_ctx* ctx, int64_t npts, const float* pts, int64_t C, con
     cudaStream_t st = (cudaStream_t)stream;
     Scratch* sc = scratch_of(ctx);
     if (N == 0) return GVC_OK;
-    const int32_t* cperm = nullptr;
-    const BvhNode* cnodes = nullptr;
     if (C > 0) {
         GVC_CUDA(sc->tmp_boxes.ensure(sizeof(float4) * 2 * C), "alloc cell boxes");
         GVC_CUDA(launch_tet_boxes(C, pts, conn4, sc->tmp_boxes.as<float4>(), st), "tet boxes");
-        GVC_CUDA(lbvh_build_boxes(ctx->cells, C, sc->tmp_boxes.as<float4>(), st), "cell LBVH");
-        cperm = ctx->cells.perm.as<int32_t>();
-        cnodes = ctx->cells.nodes.as<BvhNode>();
     }
     GVC_CUDA(morton_sort_points(sc->msamp, N, samples, st), "sample order");
-    GVC_CUDA(launch_sample_tets(N, samples, sc->msamp.perm.as<int32_t>(), pts, conn4, values, cnodes, cperm, C, out,
-                                cell_ids, ctx->d_status, st),
-             "sample tets");
-    return GVC_OK;
+    LocateArgs la{};
+    la.N = N;
+    la.samples = samples;
+    la.sperm = sc->msamp.perm.as<int32_t>();
+    la.values = values;
+    la.out = out;
+    la.cell_ids = cell_ids;
+    return locate(ctx, la, C, pts, conn4, st);
 }
 
 int gvc_knn3_mean_dist2(gvc_ctx* ctx, int64_t n, const float* pts, float* out, void* stream) {
@@ -724,15 +742,13 @@ int gvc_training_samples(gvc_ctx* ctx, int64_t npts, const float* pts, int64_t C
     if (!gt_out) return GVC_OK;
     GVC_CUDA(sc->tmp_boxes.ensure(sizeof(float4) * 2 * C), "alloc cell boxes");
     GVC_CUDA(launch_tet_boxes(C, pts, conn4, sc->tmp_boxes.as<float4>(), st), "tet boxes");
-    GVC_CUDA(lbvh_build_boxes(ctx->cells, C, sc->tmp_boxes.as<float4>(), st), "cell LBVH");
-    GVC_CUDA(ctx->ts_gt64.ensure(sizeof(double) * N), "alloc values");
     // the samples are Morton-sorted per batch already: locate them in that order
-    GVC_CUDA(launch_sample_tets(N, samples_out, nullptr, pts, conn4, values, ctx->cells.nodes.as<BvhNode>(),
-                                ctx->cells.perm.as<int32_t>(), C, ctx->ts_gt64.as<double>(), nullptr,
-                                ctx->d_status, st),
-             "sample tets");
-    GVC_CUDA(launch_to_f32(N, ctx->ts_gt64.as<double>(), gt_out, st), "values to float32");
-    return GVC_OK;
+    LocateArgs la{};
+    la.N = N;
+    la.samples = samples_out;
+    la.values = values;
+    la.out32 = gt_out;
+    return locate(ctx, la, C, pts, conn4, st);
 }
 
 int gvc_sample_cells(gvc_ctx* ctx, int64_t npts, const float* pts, int64_t C, const uint8_t* cell_types,
@@ -747,21 +763,24 @@ int gvc_sample_cells(gvc_ctx* ctx, int64_t npts, const float* pts, int64_t C, co
     cudaStream_t st = (cudaStream_t)stream;
     Scratch* sc = scratch_of(ctx);
     if (N == 0) return GVC_OK;
-    const int32_t* cperm = nullptr;
-    const BvhNode* cnodes = nullptr;
     if (C > 0) {
         GVC_CUDA(sc->tmp_boxes.ensure(sizeof(float4) * 2 * C), "alloc cell boxes");
         GVC_CUDA(launch_cell_boxes(C, pts, cell_types, cell_offsets, conn, sc->tmp_boxes.as<float4>(), st),
                  "cell boxes");
-        GVC_CUDA(lbvh_build_boxes(ctx->cells, C, sc->tmp_boxes.as<float4>(), st), "cell LBVH");
-        cperm = ctx->cells.perm.as<int32_t>();
-        cnodes = ctx->cells.nodes.as<BvhNode>();
     }
     GVC_CUDA(morton_sort_points(sc->msamp, N, samples, st), "sample order");
-    GVC_CUDA(launch_sample_cells(N, samples, sc->msamp.perm.as<int32_t>(), pts, cell_types, cell_offsets, conn,
-                                 values, cnodes, cperm, C, out, cell_ids, ctx->d_status, st),
-             "sample cells");
-    return GVC_OK;
+    LocateArgs la{};
+    la.N = N;
+    la.samples = samples;
+    la.sperm = sc->msamp.perm.as<int32_t>();
+    la.values = values;
+    la.pts = pts;
+    la.types = cell_types;
+    la.offsets = cell_offsets;
+    la.conn = conn;
+    la.out = out;
+    la.cell_ids = cell_ids;
+    return locate(ctx, la, C, nullptr, nullptr, st);
 }
 
 int gvc_debug_lbvh(gvc_ctx* ctx, int64_t n, const float* boxes, uint32_t* keys_sorted, int32_t* perm,

@@ -160,7 +160,7 @@ struct gvc_ctx {
     gvc::DevBuf knn_boxes;
     // training sample batches: unsorted points, Morton / batch key words, FP64 values
     gvc::Lbvh ts_sort;
-    gvc::DevBuf ts_points, ts_words, ts_gt64;
+    gvc::DevBuf ts_points, ts_words, cell_tree, cell_recs;
     gvc::DevBuf m_out_sorted;
     // status and statistics
     int* d_status = nullptr;          // device status word

@@ -160,8 +160,9 @@ __global__ void __launch_bounds__(256) k_tet_boxes(int64_t C, const float* __res
 
 constexpr int kPointStack = 96;
 
-// One thread per (Morton-sorted) sample; point query of the cell LBVH with a
-// per-thread stack; every containing tet is tested and the lowest id kept.
+// One thread per sample, in the caller's order: point query of the cell LBVH with a
+// per-thread stack; every containing tet is tested and the lowest id kept (noalloc.cu; samples
+// in Morton order take k_locate).
 __global__ void __launch_bounds__(128) k_sample_tets(int64_t N, const float* __restrict__ samples,
                                                      const int32_t* __restrict__ sperm, const float* __restrict__ pts,
                                                      const int32_t* __restrict__ conn4,
@@ -335,71 +336,365 @@ __global__ void __launch_bounds__(256) k_cell_boxes(int64_t C, const float* __re
     boxes[2 * c + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
 }
 
-__global__ void __launch_bounds__(128) k_sample_cells(int64_t N, const float* __restrict__ samples,
-                                                      const int32_t* __restrict__ sperm, const float* __restrict__ pts,
-                                                      const uint8_t* __restrict__ types,
-                                                      const int64_t* __restrict__ offsets,
-                                                      const int32_t* __restrict__ conn,
-                                                      const double* __restrict__ values,
-                                                      const BvhNode* __restrict__ nodes,
-                                                      const int32_t* __restrict__ cperm, int64_t C,
-                                                      double* __restrict__ out, int64_t* __restrict__ cell_ids,
-                                                      int* status) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    const int64_t s = sperm ? sperm[i] : i;
-    const float p[3] = {samples[3 * s], samples[3 * s + 1], samples[3 * s + 2]};
-    int64_t best = -1;
-    double best_v = -1.0;
-    if (C > 0) {
-        int stack[kPointStack];
-        int sp = 0;
-        stack[sp++] = 0;
-        while (sp > 0) {
-            const int node = stack[--sp];
-            const float4* np = reinterpret_cast<const float4*>(nodes + node);
-            const float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2), d = __ldg(np + 3);
-            const uint32_t ch[2] = {__float_as_uint(a.w), __float_as_uint(b.w)};
-            const bool hit[2] = {a.x <= p[0] && p[0] <= b.x && a.y <= p[1] && p[1] <= b.y && a.z <= p[2] && p[2] <= b.z,
-                                 c.x <= p[0] && p[0] <= d.x && c.y <= p[1] && p[1] <= d.y && c.z <= p[2] && p[2] <= d.z};
-            for (int k = 0; k < 2; k++) {
-                if (!hit[k]) continue;
-                if (ch[k] & kLeafBit) {
-                    const int64_t cell = cperm[ch[k] & ~kLeafBit];
-                    if (best >= 0 && cell > best) continue;
-                    const int type = types[cell];
-                    const int32_t* cv = conn + offsets[cell];
-                    if (type == 10) {
-                        double lam[4];
-                        if (tet_contains(pts + 3 * (int64_t)cv[0], pts + 3 * (int64_t)cv[1],
-                                         pts + 3 * (int64_t)cv[2], pts + 3 * (int64_t)cv[3], p, lam)) {
-                            double v = lam[0] * values[cv[0]];
-                            v = v + lam[1] * values[cv[1]];
-                            v = v + lam[2] * values[cv[2]];
-                            v = v + lam[3] * values[cv[3]];
-                            best = cell;
-                            best_v = v;
-                        }
-                    } else if (type == 12 || type == 13 || type == 14) {
-                        double Nf[8];
-                        const int n = iso_contains(type, pts, cv, p, Nf);
-                        if (n) {
-                            double v = Nf[0] * values[cv[0]];
-                            for (int q = 1; q < n; q++) v = v + Nf[q] * values[cv[q]];
-                            best = cell;
-                            best_v = v;
-                        }
+// ---------------------------------------------------------------------------------
+// Point location by a wide tree (wide_tree.cuh) over the Morton-sorted cells.
+//
+// One warp owns up to 32 Morton-sorted samples.  It walks the tree once with their box and
+// keeps the level-1 nodes (8 cells) that it meets in shared memory.  Every sample is tested
+// against every node's box; the (sample, node) pairs that meet are queued and 32 at a time
+// tested against the node's eight cells, and the (sample, cell) pairs that meet are queued in
+// turn, 32 at a time, so that no lane idles where samples meet different cells.  Of a
+// tetrahedron's pairs, seven in eight are told to be outside by its four planes in FP32 (an
+// error bound decides: k_cell_leaves); what they leave takes the containment test in double.  The lowest containing cell of each sample is kept in shared
+// memory.  A run of samples that jumps across the mesh would meet a large part of it: a walk
+// that has met 8 nodes per sample of the run is given up and the run halved, down to single
+// samples.
+//
+// A thread per sample with a stack of its own took a chain of twenty dependent node loads and
+// three dependent gathers per cell (id, vertex numbers, vertices; here one 64-byte record), and
+// ran every containment test at the pace of the warp's slowest lane: 1.57M tetrahedra x 25M
+// samples 16.7 ms against 9.9.  Testing each sample against every cell met instead took
+// 11.3k instructions per warp there, 16.4 ms.
+// ---------------------------------------------------------------------------------
+struct LocateSmem {
+    float4 lo[64], hi[64];  // met nodes: at most 31 before a step of the walk adds up to 32; lo.w: node
+    int2 nodes[64];         // (node, sample): at most 31 before a node adds up to 32
+    int2 cells[64];         // (leaf, sample): at most 31 before a leaf adds up to 32
+    int2 close[64];         // those that the planes leave: at most 31 before 32 cells add to them
+    float px[32], py[32], pz[32];
+    unsigned best[32];
+    double val[32];
+    WideStack walk;
+};
+
+struct CellMesh {
+    const float4* recs;      // tetrahedra: four vertices per leaf, .w their numbers, four planes
+    const float* pts;        // other cells
+    const uint8_t* types;
+    const int64_t* offsets;
+    const int32_t* conn;
+    const int32_t* perm;     // leaf -> cell
+    const double* values;
+};
+
+constexpr int kNodesPerSample = 8;
+
+// A tetrahedron's plane k is the volume spanned by a point and its face k over the
+// tetrahedron's own, as an affine function of the point relative to the box's low corner,
+// scaled to at most one in size over the box.  Below minus this bound the double-precision
+// test finds the point outside too: rounding of the planes, of the relative point and of the
+// four products and sums is below 8 x 2^-24, the double-precision volumes' own errors are 1e-9
+// of the scale (a face below 1e-6 of the box's square gets no plane).
+constexpr float kPlaneBound = 4e-6f;
+
+// The pairs [off, off + n) of sm.close (tetrahedra) or sm.cells.  Not inlined, nor is the next: the containment test is
+// long, and a copy at every place that empties a queue thrashed the instruction cache.
+template <bool TETS>
+__device__ __noinline__ void contain(LocateSmem& sm, const CellMesh& mesh, int off, int n) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    bool c = false;
+    unsigned cell = 0;
+    int s = 0;
+    double v = 0.0;
+    if (lane < n) {
+        const int2 q = TETS ? sm.close[off + lane] : sm.cells[off + lane];
+        s = q.y;
+        cell = (unsigned)__ldg(mesh.perm + q.x);
+        if (cell < sm.best[s]) {
+            const float p[3] = {sm.px[s], sm.py[s], sm.pz[s]};
+            if (TETS) {
+                const float4* r = mesh.recs + 8 * (int64_t)q.x;
+                const float4 a4 = __ldg(r), b4 = __ldg(r + 1), c4 = __ldg(r + 2), d4 = __ldg(r + 3);
+                const float a[3] = {a4.x, a4.y, a4.z}, b[3] = {b4.x, b4.y, b4.z}, e[3] = {c4.x, c4.y, c4.z},
+                            d[3] = {d4.x, d4.y, d4.z};
+                double lam[4];
+                c = tet_contains(a, b, e, d, p, lam);
+                if (c) {
+                    v = lam[0] * mesh.values[__float_as_int(a4.w)];
+                    v = v + lam[1] * mesh.values[__float_as_int(b4.w)];
+                    v = v + lam[2] * mesh.values[__float_as_int(c4.w)];
+                    v = v + lam[3] * mesh.values[__float_as_int(d4.w)];
+                }
+            } else {
+                const int type = mesh.types[cell];
+                const int32_t* cv = mesh.conn + mesh.offsets[cell];
+                if (type == 10) {
+                    double lam[4];
+                    c = tet_contains(mesh.pts + 3 * (int64_t)cv[0], mesh.pts + 3 * (int64_t)cv[1],
+                                     mesh.pts + 3 * (int64_t)cv[2], mesh.pts + 3 * (int64_t)cv[3], p, lam);
+                    if (c) {
+                        v = lam[0] * mesh.values[cv[0]];
+                        v = v + lam[1] * mesh.values[cv[1]];
+                        v = v + lam[2] * mesh.values[cv[2]];
+                        v = v + lam[3] * mesh.values[cv[3]];
                     }
-                } else if (sp < kPointStack) {
-                    stack[sp++] = (int)ch[k];
-                } else {
-                    atomicOr(status, kStatusStackOverflow);
+                } else if (type == 12 || type == 13 || type == 14) {
+                    double Nf[8];
+                    const int k = iso_contains(type, mesh.pts, cv, p, Nf);
+                    c = k != 0;
+                    if (c) {
+                        v = Nf[0] * mesh.values[cv[0]];
+                        for (int i = 1; i < k; i++) v = v + Nf[i] * mesh.values[cv[i]];
+                    }
                 }
             }
+            if (c) atomicMin(&sm.best[s], cell);
         }
     }
-    out[s] = best >= 0 ? best_v : -1.0;
-    if (cell_ids) cell_ids[s] = best;
+    __syncwarp();
+    if (c && sm.best[s] == cell) sm.val[s] = v;
+    __syncwarp();
+}
+
+// The pairs [off, off + n) of sm.cells; n_close: the length of sm.close, returned.
+template <bool TETS>
+__device__ __forceinline__ int narrow(LocateSmem& sm, const WideTree& tree, const CellMesh& mesh, int off, int n,
+                                      int n_close) {
+    if (!TETS) {
+        contain<false>(sm, mesh, off, n);
+        return 0;
+    }
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    bool keep = false;
+    int2 q;
+    if (lane < n) {
+        q = sm.cells[off + lane];
+        const float4* r = mesh.recs + 8 * (int64_t)q.x + 4;
+        const float4 lo = __ldg(tree.box[0] + 2 * (int64_t)q.x);
+        const float4 p0 = __ldg(r), p1 = __ldg(r + 1), p2 = __ldg(r + 2), p3 = __ldg(r + 3);
+        const float dx = sm.px[q.y] - lo.x, dy = sm.py[q.y] - lo.y, dz = sm.pz[q.y] - lo.z;
+        const float g0 = fmaf(p0.x, dx, fmaf(p0.y, dy, fmaf(p0.z, dz, p0.w)));
+        const float g1 = fmaf(p1.x, dx, fmaf(p1.y, dy, fmaf(p1.z, dz, p1.w)));
+        const float g2 = fmaf(p2.x, dx, fmaf(p2.y, dy, fmaf(p2.z, dz, p2.w)));
+        const float g3 = fmaf(p3.x, dx, fmaf(p3.y, dy, fmaf(p3.z, dz, p3.w)));
+        keep = !(g0 < -kPlaneBound || g1 < -kPlaneBound || g2 < -kPlaneBound || g3 < -kPlaneBound);
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, keep);
+    if (keep) sm.close[n_close + __popc(m & lane_lt_mask())] = q;
+    n_close += __popc(m);
+    if (n_close >= 32) {
+        n_close -= 32;
+        contain<true>(sm, mesh, n_close, 32);
+    }
+    __syncwarp();
+    return n_close;
+}
+
+// The pairs [off, off + n) of sm.nodes: tests the cells of each node and queues the pairs that
+// meet; len: the lengths of sm.cells and sm.close, returned.
+template <bool TETS>
+__device__ __noinline__ int2 expand(LocateSmem& sm, const WideTree& tree, const CellMesh& mesh, int off, int n,
+                                    int2 len) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = lane_lt_mask();
+    __syncwarp();
+    const int2 q = lane < n ? sm.nodes[off + lane] : make_int2(0, 0);
+    const float x = sm.px[q.y], y = sm.py[q.y], z = sm.pz[q.y];
+#pragma unroll 1
+    for (int k = 0; k < kWideLeaves; k++) {
+        const int leaf = q.x * kWideLeaves + k;
+        bool h = false;
+        if (lane < n && leaf < tree.n[0]) {
+            const float4* p = tree.box[0] + 2 * (int64_t)leaf;
+            const float4 lo = __ldg(p), hi = __ldg(p + 1);
+            h = lo.x <= x && x <= hi.x && lo.y <= y && y <= hi.y && lo.z <= z && z <= hi.z;
+        }
+        const uint32_t m = __ballot_sync(0xffffffffu, h);
+        if (h) sm.cells[len.x + __popc(m & lt)] = make_int2(leaf, q.y);
+        len.x += __popc(m);
+        if (len.x >= 32) {
+            len.x -= 32;
+            len.y = narrow<TETS>(sm, tree, mesh, len.x, 32, len.y);
+        }
+    }
+    __syncwarp();
+    return len;
+}
+
+template <bool TETS>
+struct Locator {
+    LocateSmem& sm;
+    const CellMesh& mesh;
+    float x, y, z;
+    const WideTree& tree;
+    bool in;  // this lane's sample is in the current run
+    int n_nodes;
+    int2 n_cells;  // and n_close
+
+    // met nodes [off, off + n) against the run's samples
+    __device__ __forceinline__ void operator()(int off, int n) {
+        const int lane = threadIdx.x & 31;
+        const uint32_t lt = lane_lt_mask();
+        __syncwarp();
+        for (int j = off; j < off + n; j++) {
+            const float4 lo = sm.lo[j], hi = sm.hi[j];
+            const bool h = in && lo.x <= x && x <= hi.x && lo.y <= y && y <= hi.y && lo.z <= z && z <= hi.z;
+            const uint32_t m = __ballot_sync(0xffffffffu, h);
+            if (m == 0) continue;
+            if (h) sm.nodes[n_nodes + __popc(m & lt)] = make_int2(__float_as_int(lo.w), lane);
+            n_nodes += __popc(m);
+            if (n_nodes >= 32) {
+                n_nodes -= 32;
+                n_cells = expand<TETS>(sm, tree, mesh, n_nodes, 32, n_cells);
+            }
+        }
+        __syncwarp();
+    }
+};
+
+// `rows` samples per warp, a power of two up to 32.
+template <bool TETS, class Out>
+__global__ void __launch_bounds__(32, TETS ? 28 : 12)
+    k_locate(int64_t N, int rows, const float* __restrict__ samples, const int32_t* __restrict__ sperm,
+             const __grid_constant__ WideTree tree, const __grid_constant__ CellMesh mesh, Out* __restrict__ out,
+             int64_t* __restrict__ cell_ids) {
+    __shared__ LocateSmem sm;
+    const int lane = threadIdx.x;
+    const int64_t i = (int64_t)blockIdx.x * rows + lane;
+    const bool valid = lane < rows && i < N;
+    int64_t s = 0;
+    float x = NAN, y = NAN, z = NAN;
+    if (valid) {
+        s = sperm ? sperm[i] : i;
+        x = samples[3 * s];
+        y = samples[3 * s + 1];
+        z = samples[3 * s + 2];
+    }
+    sm.px[lane] = x;
+    sm.py[lane] = y;
+    sm.pz[lane] = z;
+    sm.best[lane] = 0xffffffffu;
+    __syncwarp();
+    const bool number = x == x && y == y && z == z;  // a NaN lies in no cell
+    Locator<TETS> loc{sm, mesh, x, y, z, tree, false, 0, make_int2(0, 0)};
+    int a = 0, len = rows;
+    while (a < rows) {
+        loc.in = number && lane >= a && lane < a + len;
+        const Box6 b = warp_point_box(loc.in, x, y, z);
+        const float3 lo = make_float3(b.lx, b.ly, b.lz), hi = make_float3(b.hx, b.hy, b.hz);
+        int n_wait = 0, n_met = 0, n_tested = 0;
+        bool given_up = false;
+        wide_walk_nodes<false>(tree, lo, hi, sm.walk, n_tested, [&](int first, uint32_t m) -> bool {
+            n_met += __popc(m);
+            if (len > 1 && n_met > kNodesPerSample * len) {
+                given_up = true;
+                return false;
+            }
+            if ((m >> lane) & 1u) {
+                const float4* q = tree.box[1] + 2 * (int64_t)(first + lane);
+                const int k = n_wait + __popc(m & lane_lt_mask());
+                float4 l = __ldg(q);
+                l.w = __int_as_float(first + lane);
+                sm.lo[k] = l;
+                sm.hi[k] = __ldg(q + 1);
+            }
+            n_wait += __popc(m);
+            __syncwarp();
+            if (n_wait >= 32) {
+                n_wait -= 32;
+                loc(n_wait, 32);
+            }
+            return true;
+        });
+        __syncwarp();
+        if (given_up) {
+            len >>= 1;
+            continue;
+        }
+        if (n_wait > 0) loc(0, n_wait);
+        a += len;
+        len = a & -a;
+    }
+    if (loc.n_nodes > 0) loc.n_cells = expand<TETS>(sm, tree, mesh, 0, loc.n_nodes, loc.n_cells);
+    if (loc.n_cells.x > 0) loc.n_cells.y = narrow<TETS>(sm, tree, mesh, 0, loc.n_cells.x, loc.n_cells.y);
+    if (TETS && loc.n_cells.y > 0) contain<TETS>(sm, mesh, 0, loc.n_cells.y);
+    if (valid) {
+        const bool found = sm.best[lane] != 0xffffffffu;
+        out[s] = (Out)(found ? sm.val[lane] : -1.0);
+        if (cell_ids) cell_ids[s] = found ? (int64_t)sm.best[lane] : -1;
+    }
+}
+
+// Plane of a face: sign * (p - at) . m over `scale`, as (coefficients, value at p = 0).
+__device__ __forceinline__ float4 face_plane(const double m[3], const double at[3], double sign, double L) {
+    const double n1 = fabs(m[0]) + fabs(m[1]) + fabs(m[2]);
+    if (n1 < 1e-6 * L * L) return make_float4(0.f, 0.f, 0.f, 0.f);
+    const double k = sign / (n1 * L);
+    return make_float4((float)(k * m[0]), (float)(k * m[1]), (float)(k * m[2]),
+                       (float)(-k * (m[0] * at[0] + m[1] * at[1] + m[2] * at[2])));
+}
+__device__ __forceinline__ void cross_d(const double u[3], const double v[3], double m[3]) {
+    m[0] = u[1] * v[2] - u[2] * v[1];
+    m[1] = u[2] * v[0] - u[0] * v[2];
+    m[2] = u[0] * v[1] - u[1] * v[0];
+}
+
+// The four planes of kPlaneBound's comment: tet_contains compares the signs of
+// (b - p) . ((c - b) x (d - b)), (p - a) . ((c - a) x (d - a)), (p - a) . ((d - a) x (b - a))
+// and (p - a) . ((b - a) x (c - a)) with the whole volume's.
+__device__ __forceinline__ void tet_planes(const float* a, const float* b, const float* c, const float* d, float4 lo,
+                                           float4 hi, float4* out) {
+    const double V = orient(a, b, c, d);
+    const double L = fmax(fmax((double)hi.x - lo.x, (double)hi.y - lo.y), (double)hi.z - lo.z);
+    if (V == 0.0 || !(L >= 1e-30 && L <= 1e30)) {
+        // a degenerate tetrahedron contains nothing; out of range, the planes say nothing
+        const float w = V == 0.0 ? -1.f : 0.f;
+        for (int k = 0; k < 4; k++) out[k] = make_float4(0.f, 0.f, 0.f, w);
+        return;
+    }
+    const double sign = V > 0.0 ? 1.0 : -1.0;
+    const float o[3] = {lo.x, lo.y, lo.z};
+    double A[3], B[3], ab[3], ac[3], ad[3], bc[3], bd[3], m[3];
+    for (int k = 0; k < 3; k++) {
+        A[k] = (double)a[k] - o[k];
+        B[k] = (double)b[k] - o[k];
+        ab[k] = (double)b[k] - a[k];
+        ac[k] = (double)c[k] - a[k];
+        ad[k] = (double)d[k] - a[k];
+        bc[k] = (double)c[k] - b[k];
+        bd[k] = (double)d[k] - b[k];
+    }
+    cross_d(bc, bd, m);
+    out[0] = face_plane(m, B, -sign, L);
+    cross_d(ac, ad, m);
+    out[1] = face_plane(m, A, sign, L);
+    cross_d(ad, ab, m);
+    out[2] = face_plane(m, A, sign, L);
+    cross_d(ab, ac, m);
+    out[3] = face_plane(m, A, sign, L);
+}
+
+// Leaves of the tree in Morton order (levels 0 and 1) and, of tetrahedra, their records.
+template <bool TETS>
+__global__ void __launch_bounds__(256) k_cell_leaves(int64_t C, const int32_t* __restrict__ perm,
+                                                     const float4* __restrict__ boxes, const float* __restrict__ pts,
+                                                     const int32_t* __restrict__ conn4, float4* __restrict__ recs,
+                                                     float4* __restrict__ leaf, float4* __restrict__ level1) {
+    const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    Box6 b = empty_box();
+    if (g < C) {
+        const int64_t o = perm[g];
+        const float4 lo = boxes[2 * o], hi = boxes[2 * o + 1];
+        if (TETS) {
+            float p[4][3];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int v = conn4[4 * o + k];
+#pragma unroll
+                for (int i = 0; i < 3; i++) p[k][i] = pts[3 * (int64_t)v + i];
+                recs[8 * g + k] = make_float4(p[k][0], p[k][1], p[k][2], __int_as_float(v));
+            }
+            tet_planes(p[0], p[1], p[2], p[3], lo, hi, recs + 8 * g + 4);
+        }
+        b = Box6{lo.x, lo.y, lo.z, hi.x, hi.y, hi.z};
+        store_box(leaf, g, b);
+    }
+    grow(b, shfl_xor_box(b, 1));
+    grow(b, shfl_xor_box(b, 2));
+    grow(b, shfl_xor_box(b, 4));
+    if (g < C && (g & (kWideLeaves - 1)) == 0) store_box(level1, g / kWideLeaves, b);
 }
 
 static inline unsigned nbk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -411,13 +706,40 @@ cudaError_t launch_cell_boxes(int64_t C, const float* pts, const uint8_t* types,
     return cudaGetLastError();
 }
 
-cudaError_t launch_sample_cells(int64_t N, const float* samples, const int32_t* sperm, const float* pts,
-                                const uint8_t* types, const int64_t* offsets, const int32_t* conn,
-                                const double* values, const BvhNode* cnodes, const int32_t* cperm, int64_t C,
-                                double* out, int64_t* cell_ids, int* status, cudaStream_t st) {
-    if (N <= 0) return cudaSuccess;
-    k_sample_cells<<<nbk(N, 128), 128, 0, st>>>(N, samples, sperm, pts, types, offsets, conn, values, cnodes, cperm,
-                                                C, out, cell_ids, status); gvc::note_launch();
+cudaError_t launch_cell_tree(int64_t C, const int32_t* perm, const float4* boxes, const float* pts,
+                             const int32_t* conn4, float4* recs, float4* tree_boxes, cudaStream_t st) {
+    if (C <= 0) return cudaSuccess;
+    const WideTreeSize z = wide_tree_size(C);
+    float4* level1 = tree_boxes + 2 * z.n[0];
+    if (conn4) {
+        k_cell_leaves<true><<<nbk(C, 256), 256, 0, st>>>(C, perm, boxes, pts, conn4, recs, tree_boxes, level1);
+    } else {
+        k_cell_leaves<false><<<nbk(C, 256), 256, 0, st>>>(C, perm, boxes, pts, nullptr, nullptr, tree_boxes, level1);
+    }
+    gvc::note_launch();
+    return launch_wide_levels(z, tree_boxes, st);
+}
+
+template <bool TETS>
+static void launch_locate_as(const LocateArgs& a, cudaStream_t st) {
+    const WideTree tree = wide_tree_at(wide_tree_size(a.C), a.tree_boxes);
+    const CellMesh mesh{a.recs, a.pts, a.types, a.offsets, a.conn, a.cperm, a.values};
+    // fewer samples per warp where 32 would leave the chip's 148 x 28 resident warps partly idle
+    int rows = 32;
+    while (rows > 1 && a.N < (int64_t)148 * 28 * rows) rows >>= 1;
+    const unsigned n = nbk(a.N, rows);
+    if (a.out32) {
+        k_locate<TETS><<<n, 32, 0, st>>>(a.N, rows, a.samples, a.sperm, tree, mesh, a.out32, a.cell_ids);
+    } else {
+        k_locate<TETS><<<n, 32, 0, st>>>(a.N, rows, a.samples, a.sperm, tree, mesh, a.out, a.cell_ids);
+    }
+    gvc::note_launch();
+}
+
+cudaError_t launch_locate(const LocateArgs& a, cudaStream_t st) {
+    if (a.N <= 0) return cudaSuccess;
+    if (a.recs) launch_locate_as<true>(a, st);
+    else launch_locate_as<false>(a, st);
     return cudaGetLastError();
 }
 

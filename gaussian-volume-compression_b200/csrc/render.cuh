@@ -174,10 +174,27 @@ cudaError_t launch_sample_uniform(const int64_t dims[3], const float origin[3], 
 cudaError_t launch_tet_boxes(int64_t C, const float* pts, const int32_t* conn4, float4* boxes, cudaStream_t st);
 cudaError_t launch_cell_boxes(int64_t C, const float* pts, const uint8_t* types, const int64_t* offsets,
                               const int32_t* conn, float4* boxes, cudaStream_t st);
-cudaError_t launch_sample_cells(int64_t N, const float* samples, const int32_t* sperm, const float* pts,
-                                const uint8_t* types, const int64_t* offsets, const int32_t* conn,
-                                const double* values, const BvhNode* cnodes, const int32_t* cperm, int64_t C,
-                                double* out, int64_t* cell_ids, int* status, cudaStream_t st);
+// Tree over the cells in Morton order and, of tetrahedra (conn4 given), their records (8 float4
+// per cell).
+cudaError_t launch_cell_tree(int64_t C, const int32_t* perm, const float4* boxes, const float* pts,
+                             const int32_t* conn4, float4* recs, float4* tree_boxes, cudaStream_t st);
+struct LocateArgs {
+    int64_t N, C;
+    const float* samples;
+    const int32_t* sperm;      // Morton order of the samples, or null: they are sorted
+    const float4* tree_boxes;
+    const int32_t* cperm;
+    const double* values;
+    const float4* recs;        // tetrahedra, or null and:
+    const float* pts;
+    const uint8_t* types;
+    const int64_t* offsets;
+    const int32_t* conn;
+    double* out;
+    float* out32;              // instead of out
+    int64_t* cell_ids;         // or null
+};
+cudaError_t launch_locate(const LocateArgs& a, cudaStream_t st);
 cudaError_t launch_sample_tets(int64_t N, const float* samples, const int32_t* sperm, const float* pts,
                                const int32_t* conn4, const double* values, const BvhNode* cnodes,
                                const int32_t* cperm, int64_t C, double* out, int64_t* cell_ids, int* status,
@@ -187,7 +204,6 @@ cudaError_t launch_sample_tets(int64_t N, const float* samples, const int32_t* s
 cudaError_t launch_tet_points(int64_t N, int64_t S, uint64_t seed, const float* pts, const int32_t* conn4, int64_t C,
                               float* out, uint32_t* w_lo, uint32_t* w_hi, uint32_t* w_batch, cudaStream_t st);
 cudaError_t launch_gather_points(int64_t N, const float* src, const int32_t* perm, float* dst, cudaStream_t st);
-cudaError_t launch_to_f32(int64_t N, const double* src, float* dst, cudaStream_t st);
 
 // knn.cu
 cudaError_t launch_point_boxes(int64_t n, const float* pts, float4* boxes, cudaStream_t st);

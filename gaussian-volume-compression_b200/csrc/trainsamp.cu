@@ -114,11 +114,6 @@ __global__ void __launch_bounds__(256) k_gather_points(int64_t N, const float* _
     dst[3 * i + 2] = src[3 * s + 2];
 }
 
-__global__ void __launch_bounds__(256) k_to_f32(int64_t N, const double* __restrict__ src, float* __restrict__ dst) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < N) dst[i] = (float)src[i];
-}
-
 inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
@@ -134,12 +129,6 @@ cudaError_t launch_tet_points(int64_t N, int64_t S, uint64_t seed, const float* 
 cudaError_t launch_gather_points(int64_t N, const float* src, const int32_t* perm, float* dst, cudaStream_t st) {
     if (N <= 0) return cudaSuccess;
     k_gather_points<<<nblk(N, 256), 256, 0, st>>>(N, src, perm, dst); gvc::note_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t launch_to_f32(int64_t N, const double* src, float* dst, cudaStream_t st) {
-    if (N <= 0) return cudaSuccess;
-    k_to_f32<<<nblk(N, 256), 256, 0, st>>>(N, src, dst); gvc::note_launch();
     return cudaGetLastError();
 }
 

@@ -75,33 +75,20 @@ __device__ __forceinline__ uint32_t wide_hits(const WideTree& tree, int level, i
     return __ballot_sync(0xffffffffu, h);
 }
 
-// Walks the tree with the box [lo, hi] and hands the leaves of the level-1 nodes it meets to
-// visit(leaf, valid), 32 per call: eight lanes for each of four nodes.  `mine` selects
-// level-1 nodes by their number modulo 32.  Warp-collective; visit returns false to stop.
-// The order of the leaves depends on the tree and the box alone.
+// Walks the tree with the box [lo, hi] and hands the level-1 nodes it meets to
+// visit(first, mask): nodes first + i for the bits i of the mask.  Warp-collective; visit
+// returns false to stop.  The order of the nodes depends on the tree and the box alone.
 template <bool COUNT, class Visit>
-__device__ __forceinline__ void wide_walk(const WideTree& tree, float3 lo, float3 hi, uint32_t mine, WideStack& st,
-                                          int& n_tested, Visit visit) {
+__device__ __forceinline__ void wide_walk_nodes(const WideTree& tree, float3 lo, float3 hi, WideStack& st,
+                                                int& n_tested, Visit visit) {
     const int lane = threadIdx.x & 31;
-    const uint32_t lt = lane_lt_mask();
-    int queued = 0;
     for (int f = 0; f < tree.n[tree.top]; f += 32) {
         int level = tree.top, first = f;
         uint32_t m = wide_hits(tree, level, f, lo, hi);
         if (COUNT) n_tested += 32;
         while (true) {
             if (level == 1) {
-                m &= mine;
-                if ((m >> lane) & 1u) st.list[queued + __popc(m & lt)] = first + lane;
-                queued += __popc(m);
-                __syncwarp();
-                while (queued >= 4) {
-                    queued -= 4;
-                    if (COUNT) n_tested += 32;
-                    const int leaf = st.list[queued + (lane >> 3)] * kWideLeaves + (lane & 7);
-                    if (!visit(leaf, leaf < tree.n[0])) return;
-                }
-                __syncwarp();
+                if (!visit(first, m)) return;
                 m = 0;
             }
             if (m == 0) {
@@ -123,7 +110,35 @@ __device__ __forceinline__ void wide_walk(const WideTree& tree, float3 lo, float
             if (COUNT) n_tested += 32;
         }
     }
-    if (queued > 0) {
+}
+
+// The same for the leaves of those nodes: visit(leaf, valid), 32 per call, eight lanes for each
+// of four nodes.  `mine` selects level-1 nodes by their number modulo 32.
+template <bool COUNT, class Visit>
+__device__ __forceinline__ void wide_walk(const WideTree& tree, float3 lo, float3 hi, uint32_t mine, WideStack& st,
+                                          int& n_tested, Visit visit) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = lane_lt_mask();
+    int queued = 0;
+    bool stopped = false;
+    wide_walk_nodes<COUNT>(tree, lo, hi, st, n_tested, [&](int first, uint32_t m) -> bool {
+        m &= mine;
+        if ((m >> lane) & 1u) st.list[queued + __popc(m & lt)] = first + lane;
+        queued += __popc(m);
+        __syncwarp();
+        while (queued >= 4) {
+            queued -= 4;
+            if (COUNT) n_tested += 32;
+            const int leaf = st.list[queued + (lane >> 3)] * kWideLeaves + (lane & 7);
+            if (!visit(leaf, leaf < tree.n[0])) {
+                stopped = true;
+                return false;
+            }
+        }
+        __syncwarp();
+        return true;
+    });
+    if (queued > 0 && !stopped) {
         if (COUNT) n_tested += 32;
         const int leaf = (lane >> 3) < queued ? st.list[lane >> 3] * kWideLeaves + (lane & 7) : tree.n[0];
         visit(leaf, leaf < tree.n[0]);
