@@ -35,6 +35,7 @@ SOURCES = {
     "bwd_gauss.cu": [],
     "knn.cu": [],
     "trainsamp.cu": [],
+    "host_io.cu": [],
 }
 
 

@@ -11,6 +11,7 @@
 #include <cstring>
 #include <new>
 
+#include "host_io.cuh"
 #include "lbvh.cuh"
 #include "render.cuh"
 
@@ -27,6 +28,7 @@ struct Scratch {
     DevBuf tmp_out;
     Lbvh dbg;          // debug LBVH
     Lbvh msamp;        // Morton order of mesh sample points
+    Stage stage;       // pinned chunks for host arrays
 };
 
 Scratch* scratch_of(gvc_ctx* c);
@@ -161,6 +163,32 @@ struct gvc_ctx_full : gvc_ctx {
 
 namespace {
 Scratch* scratch_of(gvc_ctx* c) { return &static_cast<gvc_ctx_full*>(c)->scratch; }
+
+// The buffers of training_samples and their sizes (ctx null: sizes only).
+template <class F>
+void training_buffers(gvc_ctx* ctx, int64_t C, int64_t N, bool gt, F f) {
+    auto at = [&](auto pick) -> DevBuf* { return ctx ? pick(static_cast<gvc_ctx_full*>(ctx)) : nullptr; };
+    f(at([](gvc_ctx_full* c) { return &c->ts_points; }), sizeof(float) * 3 * N);
+    f(at([](gvc_ctx_full* c) { return &c->ts_words; }), sizeof(uint32_t) * 3 * N);
+    f(at([](gvc_ctx_full* c) { return &c->ts_sort.keys; }), LbvhBytes::keys(N));
+    f(at([](gvc_ctx_full* c) { return &c->ts_sort.keys_alt; }), LbvhBytes::keys(N));
+    f(at([](gvc_ctx_full* c) { return &c->ts_sort.perm; }), LbvhBytes::keys(N));
+    f(at([](gvc_ctx_full* c) { return &c->ts_sort.perm_alt; }), LbvhBytes::keys(N));
+    f(at([](gvc_ctx_full* c) { return &c->ts_sort.hist; }), LbvhBytes::hist(N));
+    f(at([](gvc_ctx_full* c) { return &c->ts_sort.onesweep; }), LbvhBytes::onesweep(N));
+    if (!gt) return;
+    f(at([](gvc_ctx_full* c) { return &c->scratch.tmp_boxes; }), sizeof(float4) * 2 * C);
+    f(at([](gvc_ctx_full* c) { return &c->cells.keys; }), LbvhBytes::keys(C));
+    f(at([](gvc_ctx_full* c) { return &c->cells.keys_alt; }), LbvhBytes::keys(C));
+    f(at([](gvc_ctx_full* c) { return &c->cells.perm; }), LbvhBytes::keys(C));
+    f(at([](gvc_ctx_full* c) { return &c->cells.perm_alt; }), LbvhBytes::keys(C));
+    f(at([](gvc_ctx_full* c) { return &c->cells.bounds; }), LbvhBytes::bounds());
+    f(at([](gvc_ctx_full* c) { return &c->cells.onesweep; }), LbvhBytes::onesweep(C));
+    f(at([](gvc_ctx_full* c) { return &c->cell_tree; }), sizeof(float4) * 2 * (size_t)wide_tree_size(C).boxes);
+    f(at([](gvc_ctx_full* c) { return &c->cell_recs; }), sizeof(float4) * 8 * C);
+}
+
+size_t round256(size_t n) { return (n + 255) & ~size_t(255); }
 }  // namespace
 
 extern "C" {
@@ -204,6 +232,7 @@ void gvc_ctx_destroy(gvc_ctx* ctx) {
                       &c->m_out_sorted, &c->knn_boxes, &c->ts_points, &c->ts_words, &c->cell_tree, &c->cell_recs, &c->scratch.gacc, &c->scratch.tmp_boxes, &c->scratch.tmp_out,
                       &c->clog, &c->cmask, &c->cend};
     for (DevBuf* b : bufs) b->release();
+    c->scratch.stage.release();
     if (c->d_status) cudaFree(c->d_status);
     if (c->d_stats) cudaFree(c->d_stats);
     if (c->h_status) cudaFreeHost(c->h_status);
@@ -709,6 +738,69 @@ int gvc_knn3_mean_dist2(gvc_ctx* ctx, int64_t n, const float* pts, float* out, v
     GVC_CUDA(launch_knn3(n, ctx->knn.sorted_boxes.as<float4>(), ctx->knn.perm.as<int32_t>(),
                          ctx->knn.nodes.as<BvhNode>(), out, ctx->d_status, st),
              "knn3");
+    return GVC_OK;
+}
+
+int64_t gvc_training_workspace(int64_t C, int64_t num_batches, int64_t batch_size, int with_gt) {
+    if (C < 0 || num_batches < 0 || batch_size < 0 || C > kMaxElems) return 0;
+    if (batch_size > 0 && num_batches > kMaxElems / batch_size) return 0;
+    size_t total = 0;
+    training_buffers(nullptr, C, num_batches * batch_size, with_gt != 0,
+                     [&](DevBuf*, size_t n) { total += round256(n); });
+    return (int64_t)total;
+}
+
+int gvc_training_samples_in(gvc_ctx* ctx, int64_t npts, const float* pts, int64_t C, const int32_t* conn4,
+                            const double* values, int64_t num_batches, int64_t batch_size, uint64_t seed,
+                            float* samples_out, float* gt_out, void* workspace, int64_t workspace_bytes,
+                            void* stream) {
+    if (!ctx) return GVC_ERR_ARG;
+    if (workspace_bytes < 0 || (workspace_bytes > 0 && !workspace) || ((uintptr_t)workspace & 255u))
+        return fail(ctx, GVC_ERR_ARG, "workspace must be 256-byte aligned");
+    const bool sized = C > 0 && C <= kMaxElems && num_batches > 0 && batch_size > 0 &&
+                       num_batches <= kMaxElems / batch_size;
+    if (sized) {
+        char* p = (char*)workspace;
+        size_t left = (size_t)workspace_bytes;
+        training_buffers(ctx, C, num_batches * batch_size, gt_out != nullptr, [&](DevBuf* b, size_t n) {
+            if (round256(n) > left) return;  // the call allocates what does not fit
+            b->lend(p, round256(n));
+            p += round256(n);
+            left -= round256(n);
+        });
+    }
+    const int rc = gvc_training_samples(ctx, npts, pts, C, conn4, values, num_batches, batch_size, seed, samples_out,
+                                        gt_out, stream);
+    if (sized) training_buffers(ctx, C, num_batches * batch_size, true, [](DevBuf* b, size_t) { b->give_back(); });
+    return rc;
+}
+
+int gvc_upload(gvc_ctx* ctx, int n, void* const* dst, const void* const* src, const int64_t* bytes, void* stream) {
+    if (!ctx) return GVC_ERR_ARG;
+    if (n < 0 || (n > 0 && (!dst || !src || !bytes))) return fail(ctx, GVC_ERR_ARG, "null array list");
+    for (int i = 0; i < n; i++)
+        if (bytes[i] < 0 || (bytes[i] > 0 && (!dst[i] || !src[i]))) return fail(ctx, GVC_ERR_ARG, "null array");
+    GVC_CUDA(scratch_of(ctx)->stage.upload(ctx->device, n, dst, src, bytes, (cudaStream_t)stream), "upload");
+    return GVC_OK;
+}
+
+int gvc_download(gvc_ctx* ctx, void* dst, const void* src, int64_t bytes, void* stream) {
+    if (!ctx) return GVC_ERR_ARG;
+    if (bytes < 0 || (bytes > 0 && (!dst || !src))) return fail(ctx, GVC_ERR_ARG, "null array");
+    GVC_CUDA(scratch_of(ctx)->stage.download(ctx->device, dst, src, bytes, (cudaStream_t)stream), "download");
+    return GVC_OK;
+}
+
+int gvc_check_cells(gvc_ctx* ctx, int64_t C, const int64_t* cell_types, const int64_t* cell_offsets, int64_t n_conn,
+                    const int64_t* conn, int64_t npts, uint8_t* types_out, int32_t* conn_out, int64_t* result,
+                    void* stream) {
+    if (!ctx) return GVC_ERR_ARG;
+    if (C < 0 || n_conn < 0 || npts < 0) return fail(ctx, GVC_ERR_ARG, "negative size");
+    if (!result || (n_conn > 0 && (!conn || !conn_out)) || (cell_types && (!cell_offsets || !types_out)))
+        return fail(ctx, GVC_ERR_ARG, "null pointer");
+    GVC_CUDA(launch_check_cells(C, cell_types, cell_offsets, n_conn, conn, npts, types_out, conn_out, result,
+                                (cudaStream_t)stream),
+             "check cells");
     return GVC_OK;
 }
 

@@ -47,12 +47,14 @@ struct __align__(16) BvhNode {
 
 constexpr uint32_t kLeafBit = 0x80000000u;
 
-// Growable device buffer owned by the context.
+// Growable device buffer owned by the context, or a view of memory that the caller lends.
 struct DevBuf {
     void* ptr = nullptr;
     size_t bytes = 0;
+    bool lent = false;
     cudaError_t ensure(size_t need) {
         if (need <= bytes && ptr) return cudaSuccess;
+        if (lent) give_back();
         if (ptr) {
             cudaError_t e = cudaFree(ptr);
             if (e != cudaSuccess) return e;
@@ -68,9 +70,20 @@ struct DevBuf {
     template <class T>
     T* as() const { return reinterpret_cast<T*>(ptr); }
     void release() {
-        if (ptr) cudaFree(ptr);
+        if (ptr && !lent) cudaFree(ptr);
         ptr = nullptr;
         bytes = 0;
+        lent = false;
+    }
+    // takes a view in place of memory of its own
+    void lend(void* p, size_t n) {
+        release();
+        ptr = p;
+        bytes = n;
+        lent = true;
+    }
+    void give_back() {
+        if (lent) release();
     }
 };
 

@@ -18,6 +18,9 @@ struct LbvhBytes {
     static constexpr size_t hist(int64_t n) {
         return sizeof(uint32_t) * (256 * (size_t)((n + kRsTile - 1) / kRsTile) + 256);
     }
+    static constexpr size_t onesweep(int64_t n) {  // digit counts [4][256], tickets, a look-back word per tile and digit
+        return sizeof(uint32_t) * (4 * 256 + 64 + 4 * 256 * (size_t)((n + kRsTile - 1) / kRsTile));
+    }
     static constexpr size_t bounds() { return sizeof(uint32_t) * 8; }
     static constexpr size_t sorted_boxes(int64_t n) { return 2 * 16 * (size_t)n; }
     static constexpr size_t child(int64_t n) { return sizeof(int32_t) * (size_t)internal(n); }  // left, right, flags

@@ -171,6 +171,11 @@ cudaError_t launch_fill_zero_outputs(int64_t S, float* out_cells, float* out_wei
 cudaError_t launch_sample_uniform(const int64_t dims[3], const float origin[3], const float spacing[3],
                                   const void* values, int dtype, int64_t N, const float* samples, void* out,
                                   cudaStream_t st);
+// Cells as int64 arrays: types_out / conn_out (truncated to 32 bits) and the six words of
+// gvc_check_cells' result.
+cudaError_t launch_check_cells(int64_t C, const int64_t* types, const int64_t* offsets, int64_t n_conn,
+                               const int64_t* conn, int64_t npts, uint8_t* types_out, int32_t* conn_out,
+                               int64_t* result, cudaStream_t st);
 cudaError_t launch_tet_boxes(int64_t C, const float* pts, const int32_t* conn4, float4* boxes, cudaStream_t st);
 cudaError_t launch_cell_boxes(int64_t C, const float* pts, const uint8_t* types, const int64_t* offsets,
                               const int32_t* conn, float4* boxes, cudaStream_t st);

@@ -27,8 +27,6 @@ _lock = threading.Lock()
 _contexts = {}
 
 VTK_TETRA = 10
-# VTK cell types the reference maps to Viskores shapes (sample_mesh.cu:300-336)
-VTK_KNOWN = {1, 3, 5, 9, 10, 12, 13, 14}
 
 
 def _ctx():
@@ -50,6 +48,23 @@ def _dev(a, dtype):
     return torch.from_numpy(np.ascontiguousarray(a, dtype=dtype)).to(device="cuda:%d" % dev)
 
 
+def _upload(dev, c, *arrays):
+    """Device copies of contiguous host arrays, as flat byte tensors (never empty)."""
+    out = [torch.empty(max(a.nbytes, 1), dtype=torch.uint8, device="cuda:%d" % dev) for a in arrays]
+    n = len(arrays)
+    dst = (ctypes.c_void_p * n)(*[t.data_ptr() for t in out])
+    src = (ctypes.c_void_p * n)(*[a.ctypes.data for a in arrays])
+    size = (ctypes.c_int64 * n)(*[a.nbytes for a in arrays])
+    c.call("gvc_upload", n, dst, src, size, _stream(dev))
+    return out
+
+
+def _download(dev, c, t, n, dtype):
+    out = np.empty(n, dtype=dtype)
+    c.call("gvc_download", _n.ptr(out), _n.ptr(t), out.nbytes, _stream(dev))
+    return out
+
+
 def sample_mesh(dims_arr, origin_arr, spacing_arr, val_arr, samp_arr):
     """Uniform point field (x fastest) sampled by trilinear interpolation; outside -> -1
     in the values' dtype.  Output dtype follows the values (sample_mesh.cu:76-115)."""
@@ -68,23 +83,21 @@ def sample_mesh(dims_arr, origin_arr, spacing_arr, val_arr, samp_arr):
     samples = np.ascontiguousarray(samp_arr, dtype=np.float32)
     n = samples.shape[0] if samples.ndim > 0 else 0
     samples = samples.reshape(n, 3) if n else samples.reshape(0, 3)
-    out = np.empty(n, dtype=vals.dtype)
     if n == 0:
-        return out
+        return np.empty(0, dtype=vals.dtype)
     dev, c = _ctx()
-    d_vals = torch.from_numpy(vals.reshape(-1).view(np.uint8)).to("cuda:%d" % dev)
-    d_samp = _dev(samples, np.float32)
+    d_vals, d_samp = _upload(dev, c, vals, samples)
     d_out = torch.empty(n * vals.dtype.itemsize, dtype=torch.uint8, device="cuda:%d" % dev)
     # host arrays must stay referenced until the call returns
     h_dims, h_origin, h_spacing = dims[:3].copy(), origin[:3].copy(), spacing[:3].copy()
     c.call("gvc_sample_uniform", _n.ptr(h_dims), _n.ptr(h_origin), _n.ptr(h_spacing), _n.ptr(d_vals), code, n,
            _n.ptr(d_samp), _n.ptr(d_out), _stream(dev))
-    out[:] = d_out.cpu().numpy().view(vals.dtype)
-    return out
+    return _download(dev, c, d_out, n, vals.dtype)
 
 
 # points per cell for each VTK type the reference maps (sample_mesh.cu:300-336)
 VTK_NPTS = {1: 1, 3: 2, 5: 3, 9: 4, 10: 4, 12: 8, 13: 6, 14: 5}
+_NPTS_OF = np.array([VTK_NPTS.get(t, 0) for t in range(16)], dtype=np.int64)  # 0 and 15: none, and all beyond
 
 
 def _check_cells(conn, cell_types, cell_offsets):
@@ -99,23 +112,47 @@ def _check_cells(conn, cell_types, cell_offsets):
         return conn.astype(np.int32), types.astype(np.uint8), offs[:0].copy()
     if offs.size < C:
         raise RuntimeError("cell_offsets has fewer entries than cell_types")
-    unknown = types[~np.isin(types, list(VTK_KNOWN))]
-    if unknown.size:
-        raise RuntimeError("Unsupported VTK cell type: " + str(int(unknown[0])))
+    want = _NPTS_OF[np.clip(types, 0, _NPTS_OF.size - 1)]
+    if not want.all():
+        raise RuntimeError("Unsupported VTK cell type: " + str(int(types[np.argmin(want)])))
     start = offs[:C]
     end = np.empty(C, dtype=np.int64)
     end[:-1] = offs[1:C]
     end[-1] = conn.size
-    want = np.vectorize(VTK_NPTS.get, otypes=[np.int64])(types)
     if np.any(end - start != want) or np.any(start < 0) or np.any(end > conn.size):
         raise RuntimeError("cell point count does not match its VTK cell type")
     return conn.astype(np.int32), types.astype(np.uint8), start.copy()
 
 
-def _tets_from_cells(conn, types, offs):
-    """[C,4] int32 vertex ids of an all-tetrahedra mesh (already validated)."""
-    idx = offs[:, None] + np.arange(4, dtype=np.int64)[None, :]
-    return conn[idx].astype(np.int32)
+class _DeviceCells:
+    """_check_cells on the device: the cells' arrays there, validated when check() returns (the
+    transfers of other arrays can go on before it)."""
+
+    def __init__(self, dev, c, conn, cell_types, cell_offsets, npts):
+        self.conn = np.ascontiguousarray(conn, dtype=np.int64).reshape(-1)
+        self.types = np.ascontiguousarray(cell_types, dtype=np.int64).reshape(-1)
+        offs = np.ascontiguousarray(cell_offsets, dtype=np.int64).reshape(-1)
+        C = self.types.size
+        if offs.size < C:
+            raise RuntimeError("cell_offsets has fewer entries than cell_types")
+        self.offs = offs[:C]
+        up_conn, up_types, self.d_offs = _upload(dev, c, self.conn, self.types, self.offs)
+        d = "cuda:%d" % dev
+        self.d_conn = torch.empty(max(self.conn.size, 1), dtype=torch.int32, device=d)
+        self.d_types = torch.empty(max(C, 1), dtype=torch.uint8, device=d)
+        self.result = torch.empty(6, dtype=torch.int64, device=d)
+        c.call("gvc_check_cells", C, _n.ptr(up_types), _n.ptr(self.d_offs), self.conn.size, _n.ptr(up_conn), npts,
+               _n.ptr(self.d_types), _n.ptr(self.d_conn), _n.ptr(self.result), _stream(dev))
+
+    def check(self):
+        """Raises as _check_cells does; returns whether every cell is a tetrahedron and whether
+        their ids lie outside the point array."""
+        unknown, mismatch, other, bad, bad_tets, _ = self.result.tolist()
+        if unknown < self.types.size:
+            raise RuntimeError("Unsupported VTK cell type: " + str(int(self.types[unknown])))
+        if mismatch:
+            raise RuntimeError("cell point count does not match its VTK cell type")
+        return not other, bool(bad if other else bad_tets)
 
 
 def sample_meshu_cells(pts_arr, conn4, val_arr, samp_arr):
@@ -180,12 +217,32 @@ def sample_meshu_mixed(pts_arr, conn_arr, cell_types_arr, cell_offsets_arr, val_
 def sample_meshu(pts_arr, conn_arr, cell_types_arr, cell_offsets_arr, val_arr, samp_arr):
     """Explicit mesh point field sampled at points; outside every cell -> -1 (float64).
     All-tetrahedra meshes take the tetrahedral kernel; mixed meshes the general one."""
-    conn, types, offs = _check_cells(conn_arr, cell_types_arr, cell_offsets_arr)
-    if types.size and np.all(types == VTK_TETRA):
-        out, _ = sample_meshu_cells(pts_arr, _tets_from_cells(conn, types, offs), val_arr, samp_arr)
-        return out
-    out, _ = sample_meshu_mixed(pts_arr, conn_arr, cell_types_arr, cell_offsets_arr, val_arr, samp_arr)
-    return out
+    samples = np.ascontiguousarray(samp_arr, dtype=np.float32).reshape(-1, 3)
+    n, C = samples.shape[0], np.size(cell_types_arr)
+    if n == 0 or C == 0 or not torch.cuda.is_available():
+        # nothing to locate, or nothing to locate it with: the checks alone, on the host
+        return sample_meshu_mixed(pts_arr, conn_arr, cell_types_arr, cell_offsets_arr, val_arr, samp_arr)[0]
+    dev, c = _ctx()
+    pts = np.ascontiguousarray(pts_arr, dtype=np.float32).reshape(-1, 3)
+    vals = np.ascontiguousarray(val_arr, dtype=np.float64).reshape(-1)
+    cells = _DeviceCells(dev, c, conn_arr, cell_types_arr, cell_offsets_arr, pts.shape[0])
+    d_pts, d_vals, d_samp = _upload(dev, c, pts, vals, samples)
+    tets, outside = cells.check()
+    if outside:
+        raise RuntimeError("connectivity refers to a point outside the point array")
+    if vals.size < pts.shape[0]:
+        raise RuntimeError("values must hold one entry per point")
+    d_out = torch.empty(n, dtype=torch.float64, device="cuda:%d" % dev)
+    if tets:
+        # checked: four ids per cell, one cell after the other
+        conn4 = cells.d_conn[int(cells.offs[0]):]
+        c.call("gvc_sample_tets", pts.shape[0], _n.ptr(d_pts), C, _n.ptr(conn4), _n.ptr(d_vals), n, _n.ptr(d_samp),
+               _n.ptr(d_out), None, _stream(dev))
+    else:
+        c.call("gvc_sample_cells", pts.shape[0], _n.ptr(d_pts), C, _n.ptr(cells.d_types), _n.ptr(cells.d_offs),
+               _n.ptr(cells.d_conn), _n.ptr(d_vals), n, _n.ptr(d_samp), _n.ptr(d_out), None, _stream(dev))
+    c.sync_status(torch.cuda.current_stream(dev).cuda_stream)
+    return _download(dev, c, d_out, n, np.float64)
 
 
 def sample_training_batches(pts_arr, tets_arr, val_arr, num_batches, batch_size, seed=0, gt_cells=None):
@@ -200,7 +257,7 @@ def sample_training_batches(pts_arr, tets_arr, val_arr, num_batches, batch_size,
     from that (untriangulated) cell mesh instead, as the reference does when it samples
     the original mesh.  Returns CUDA tensors (samples [B,S,3] float32, gt [B,S] float32);
     nothing goes through host memory after the mesh upload.  The call's workspace (about
-    48 bytes per sample) belongs to a context of its own, released before returning.
+    40 bytes per sample) comes from torch's allocator and goes back to it on return.
     """
     pts = np.ascontiguousarray(pts_arr, dtype=np.float32).reshape(-1, 3)
     tets = np.ascontiguousarray(tets_arr, dtype=np.int64).reshape(-1, 4)
@@ -210,34 +267,51 @@ def sample_training_batches(pts_arr, tets_arr, val_arr, num_batches, batch_size,
         raise RuntimeError("num_batches and batch_size must be non-negative")
     if tets.shape[0] == 0 or pts.shape[0] == 0:
         raise RuntimeError("the mesh has no cells or no points")
-    if tets.min() < 0 or tets.max() >= pts.shape[0]:
+    have_gpu = torch.cuda.is_available()
+    if not have_gpu and (tets.min() < 0 or tets.max() >= pts.shape[0]):
         raise RuntimeError("connectivity refers to a point outside the point array")
+    dev = torch.cuda.current_device() if have_gpu else None
+    d = "cuda:%d" % dev if have_gpu else None
+    if have_gpu:
+        _, up = _ctx()
+        (raw,) = _upload(dev, up, tets)
+        d_tets = torch.empty(tets.size, dtype=torch.int32, device=d)
+        result = torch.empty(6, dtype=torch.int64, device=d)
+        up.call("gvc_check_cells", 0, None, None, tets.size, _n.ptr(raw), pts.shape[0], None, _n.ptr(d_tets),
+                _n.ptr(result), _stream(dev))
+        d_pts, d_vals = _upload(dev, up, pts, vals)
+        del raw
+        if result[5].item():
+            raise RuntimeError("connectivity refers to a point outside the point array")
     if vals.size < pts.shape[0]:
         raise RuntimeError("values must hold one entry per point")
     dev = torch.cuda.current_device()
-    c = _n.Context()   # one-off workspace, freed with the context at the end of the call
-    d = "cuda:%d" % dev
     samples = torch.empty((B, S, 3), dtype=torch.float32, device=d)
     gt = torch.empty((B, S), dtype=torch.float32, device=d)
     if B * S == 0:
         return samples, gt
-    d_pts = _dev(pts, np.float32)
-    d_tets = _dev(tets, np.int32)
-    d_vals = _dev(vals, np.float64)
-    c.call("gvc_training_samples", pts.shape[0], _n.ptr(d_pts), tets.shape[0], _n.ptr(d_tets), _n.ptr(d_vals),
-           B, S, ctypes.c_uint64(int(seed) & 0xFFFFFFFFFFFFFFFF), _n.ptr(samples),
-           None if gt_cells is not None else _n.ptr(gt), _stream(dev))
+    C = tets.shape[0]
+    size = _n.lib().gvc_training_workspace(C, B, S, 0 if gt_cells is not None else 1)
+    work = torch.empty(max(size, 1), dtype=torch.uint8, device=d)  # given back to the allocator on return
+    c = _n.Context()  # a state of its own for this call
+    c.call("gvc_training_samples_in", pts.shape[0], _n.ptr(d_pts), C, _n.ptr(d_tets), _n.ptr(d_vals), B, S,
+           ctypes.c_uint64(int(seed) & 0xFFFFFFFFFFFFFFFF), _n.ptr(samples),
+           None if gt_cells is not None else _n.ptr(gt), _n.ptr(work), size, _stream(dev))
     if gt_cells is not None:
-        conn, types, offs = _check_cells(*gt_cells)
-        if conn.size and (conn.min() < 0 or conn.max() >= pts.shape[0]):
-            raise RuntimeError("connectivity refers to a point outside the point array")
-        C = types.size
-        d_conn = _dev(conn if conn.size else np.zeros(1, np.int32), np.int32)
-        d_types = _dev(types if C else np.zeros(1, np.uint8), np.uint8)
-        d_offs = _dev(offs if C else np.zeros(1, np.int64), np.int64)
+        if np.size(gt_cells[1]):
+            cells = _DeviceCells(dev, up, *gt_cells, pts.shape[0])
+            tets_only, outside = cells.check()
+            if outside or (tets_only and cells.result[3].item()):
+                raise RuntimeError("connectivity refers to a point outside the point array")
+            C, d_conn, d_types, d_offs = cells.types.size, cells.d_conn, cells.d_types, cells.d_offs
+        else:
+            conn, types, offs = _check_cells(*gt_cells)
+            if conn.size and (conn.min() < 0 or conn.max() >= pts.shape[0]):
+                raise RuntimeError("connectivity refers to a point outside the point array")
+            C, d_conn, d_types, d_offs = 0, None, None, None
         g64 = torch.empty(B * S, dtype=torch.float64, device=d)
-        c.call("gvc_sample_cells", pts.shape[0], _n.ptr(d_pts), C, _n.ptr(d_types), _n.ptr(d_offs), _n.ptr(d_conn),
-               _n.ptr(d_vals), B * S, _n.ptr(samples), _n.ptr(g64), None, _stream(dev))
+        c.call("gvc_sample_cells", pts.shape[0], _n.ptr(d_pts), C, _n.ptr(d_types), _n.ptr(d_offs),
+               _n.ptr(d_conn), _n.ptr(d_vals), B * S, _n.ptr(samples), _n.ptr(g64), None, _stream(dev))
         gt.copy_(g64.view(B, S))
     c.sync_status(torch.cuda.current_stream(dev).cuda_stream)
     return samples, gt

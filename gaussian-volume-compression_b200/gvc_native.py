@@ -46,6 +46,11 @@ _SIGNATURES = {
     "gvc_sample_cells": [_vp, _i64, _vp, _i64, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp],
     "gvc_knn3_mean_dist2": [_vp, _i64, _vp, _vp, _vp],
     "gvc_training_samples": [_vp, _i64, _vp, _i64, _vp, _vp, _i64, _i64, ctypes.c_uint64, _vp, _vp, _vp],
+    "gvc_training_workspace": [_i64, _i64, _i64, _int],
+    "gvc_training_samples_in": [_vp, _i64, _vp, _i64, _vp, _vp, _i64, _i64, ctypes.c_uint64, _vp, _vp, _vp, _i64, _vp],
+    "gvc_upload": [_vp, _int, _vp, _vp, _vp, _vp],
+    "gvc_download": [_vp, _vp, _vp, _i64, _vp],
+    "gvc_check_cells": [_vp, _i64, _vp, _vp, _i64, _vp, _i64, _vp, _vp, _vp, _vp],
     "gvc_debug_lbvh": [_vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "gvc_debug_lbvh_escape": [_vp, _vp, _vp],
     "gvc_debug_preprocess": [_vp, _i64, _vp, _vp, _vp, _vp, _f32, _vp, _vp, _vp],
@@ -54,7 +59,8 @@ _SIGNATURES = {
     "gvc_debug_wait_timeout": [_vp, _vp],
     "gvc_sample_tets_static": [_i64, _vp, _i64, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _i64],
 }
-_RESTYPES = {"gvc_ctx_destroy": None, "gvc_last_error": ctypes.c_char_p, "gvc_launch_count": ctypes.c_int64}
+_RESTYPES = {"gvc_ctx_destroy": None, "gvc_last_error": ctypes.c_char_p, "gvc_launch_count": ctypes.c_int64,
+             "gvc_training_workspace": ctypes.c_int64}
 
 
 class GvcStats(ctypes.Structure):

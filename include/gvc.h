@@ -192,6 +192,33 @@ int gvc_training_samples(gvc_ctx* ctx, int64_t npts, const float* pts, int64_t C
                          const double* values, int64_t num_batches, int64_t batch_size, uint64_t seed,
                          float* samples_out, float* gt_out, void* stream);
 
+/* gvc_training_samples with its workspace lent by the caller (256-byte aligned device memory
+   of gvc_training_workspace bytes; what does not fit is allocated as above).  The workspace
+   is used until `stream` has finished the call's work; the context keeps no address of it. */
+int64_t gvc_training_workspace(int64_t C, int64_t num_batches, int64_t batch_size, int with_gt);
+int gvc_training_samples_in(gvc_ctx* ctx, int64_t npts, const float* pts, int64_t C, const int32_t* conn4,
+                            const double* values, int64_t num_batches, int64_t batch_size, uint64_t seed,
+                            float* samples_out, float* gt_out, void* workspace, int64_t workspace_bytes,
+                            void* stream);
+
+/* Copies between pageable host arrays and the device through the context's pinned chunks,
+   several threads copying.  gvc_upload queues n arrays (host lists of device pointers, host
+   pointers, byte counts) on `stream` and returns when the host arrays have been read;
+   gvc_download returns when the data has arrived.  Calls on one context take turns. */
+int gvc_upload(gvc_ctx* ctx, int n, void* const* dst, const void* const* src, const int64_t* bytes, void* stream);
+int gvc_download(gvc_ctx* ctx, void* dst, const void* src, int64_t bytes, void* stream);
+
+/* Validates an explicit mesh given as int64 device arrays and writes what gvc_sample_cells and
+   gvc_sample_tets take: types_out (uint8) and conn_out (the ids' low 32 bits).  cell_types
+   may be NULL (connectivity alone).  result (6 device words): the first cell of an unknown
+   VTK type (INT64_MAX: none); then nonzero where a cell's point count (the distance to the
+   next offset, of the last cell to n_conn) differs from its type's or its offsets leave
+   [0, n_conn]; where a cell is no tetrahedron; where a written id lies outside [0, npts);
+   where one from the first cell's offset on does; where an id as given does. */
+int gvc_check_cells(gvc_ctx* ctx, int64_t C, const int64_t* cell_types, const int64_t* cell_offsets, int64_t n_conn,
+                    const int64_t* conn, int64_t npts, uint8_t* types_out, int32_t* conn_out, int64_t* result,
+                    void* stream);
+
 /* No counterpart in the reference.  Tetrahedral sampling for callers that cannot
    allocate device memory (their memory belongs to another allocator, or cudaMalloc's
    device-wide synchronisation is unacceptable where they call).  Same inputs, outputs
