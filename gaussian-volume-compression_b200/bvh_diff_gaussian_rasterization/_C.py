@@ -113,11 +113,12 @@ def rasterize_gaussians(means3D, scales, rotations, values, weights, scale_modif
     samples = _stored(dev)
     S = samples.size(0)
     opts = dict(dtype=torch.float32, device=means3D.device)
-    out_cells = torch.zeros(S, **opts)
-    out_weights = torch.zeros(S, **opts)
-    conics = torch.zeros(P * 6, **opts)
     if P == 0:
-        return out_cells, out_weights, conics
+        return torch.zeros(S, **opts), torch.zeros(S, **opts), torch.zeros(0, **opts)
+    # every element is written by the call: no fill first
+    out_cells = torch.empty(S, **opts)
+    out_weights = torch.empty(S, **opts)
+    conics = torch.empty(P * 6, **opts)
     scales = _f32(scales, "scales", 3 * P)
     rotations = _f32(rotations, "rotations", 4 * P)
     values = _f32(values, "values", P)
@@ -143,11 +144,12 @@ def rasterize_gaussians_backward(means3D, scales, rotations, conics, values, wei
     samples = _stored(dev)
     S = samples.size(0)
     opts = dict(dtype=torch.float32, device=means3D.device)
-    dmeans = torch.zeros(P, 3, **opts)
-    dscales = torch.zeros(P, 3, **opts)
-    drots = torch.zeros(P, 4, **opts)
-    dvalues = torch.zeros(P, 1, **opts)
-    dweights = torch.zeros(P, 1, **opts)
+    # every element is written by the call: no fill first
+    dmeans = torch.empty(P, 3, **opts)
+    dscales = torch.empty(P, 3, **opts)
+    drots = torch.empty(P, 4, **opts)
+    dvalues = torch.empty(P, 1, **opts)
+    dweights = torch.empty(P, 1, **opts)
     if P == 0:
         return dmeans, dscales, drots, dvalues, dweights
     scales = _f32(scales, "scales", 3 * P)

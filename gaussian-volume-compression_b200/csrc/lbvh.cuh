@@ -29,17 +29,14 @@ struct LbvhBytes {
     static constexpr size_t nodes(int64_t n) { return sizeof(BvhNode) * (size_t)internal(n); }
 };
 
-// Stable radix sort of L.keys[0..n) (uint32); result in L.keys (sorted) and L.perm
-// (sorted position -> input index).
-cudaError_t radix_sort_pairs(Lbvh& L, int64_t n, cudaStream_t st);
-
 // Stable LSD sort of n indices by a key of several 32-bit words (words[0] least
 // significant); bits[w] = significant bits of word w (ceil(bits / 8) radix passes).
 // Result in L.perm (sorted position -> input index); L.keys / keys_alt are scratch.
 cudaError_t radix_sort_words(Lbvh& L, int64_t n, const uint32_t* const* words, const int* bits, int nwords,
                              cudaStream_t st);
 
-// 30-bit Morton keys of box centroids over the centroid bounds, then sort.
+// 30-bit Morton keys of box centroids over the centroid bounds, then a stable radix sort:
+// L.keys (sorted) and L.perm (sorted position -> input index).
 cudaError_t morton_sort_boxes(Lbvh& L, int64_t n, const float4* boxes, cudaStream_t st);
 // Same for points [n][3].
 cudaError_t morton_sort_points(Lbvh& L, int64_t n, const float* pts, cudaStream_t st);
