@@ -58,11 +58,34 @@ __global__ void k_boxes6_to_f4(int64_t n, const float* __restrict__ b6, float4* 
     out[2 * i + 1] = make_float4(b6[6 * i + 3], b6[6 * i + 4], b6[6 * i + 5], 0.f);
 }
 
-// escape edges (BvhNode c.w)
-__global__ void k_node_escape(int64_t n, const BvhNode* __restrict__ nodes, int32_t* __restrict__ out) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    out[i] = __float_as_int(nodes[i].c.w);
+// The tree in Karras' numbering: a node's index is the first or the last of its leaves, as it is
+// its parent's right or left child, the root's 0.
+__device__ int karras_index(const BvhNode* nodes, const uint32_t* keys, int n, int k) {
+    const int l = __float_as_int(nodes[k].b.w), r = __float_as_int(nodes[k].c.w);
+    if (l == 0 && r == n - 1) return 0;
+    return lbvh_is_left(keys, n, l, r) ? r : l;
+}
+
+// For node k = 1 + split: its children, its box, and its escape edge (2 p + 1 for the node p
+// whose left child's leaves end where this node's do, all ones on the root's right spine).
+__global__ void k_karras_tree(int n, const BvhNode* __restrict__ nodes, const uint32_t* __restrict__ keys,
+                              int32_t* __restrict__ left, int32_t* __restrict__ right, float* __restrict__ boxes6,
+                              int32_t* __restrict__ escape) {
+    const int k = 1 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const BvhNode nd = nodes[k];
+    const int at = karras_index(nodes, keys, n, k), l = __float_as_int(nd.b.w), r = __float_as_int(nd.c.w);
+    if (left) left[at] = l == k - 1 ? (int32_t)((uint32_t)l | kLeafBit) : k - 1;
+    if (right) right[at] = r == k ? (int32_t)((uint32_t)r | kLeafBit) : k;
+    if (boxes6) {
+        boxes6[6 * at] = fminf(nd.a.x, nd.c.x);
+        boxes6[6 * at + 1] = fminf(nd.a.y, nd.c.y);
+        boxes6[6 * at + 2] = fminf(nd.a.z, nd.c.z);
+        boxes6[6 * at + 3] = fmaxf(nd.b.x, nd.d.x);
+        boxes6[6 * at + 4] = fmaxf(nd.b.y, nd.d.y);
+        boxes6[6 * at + 5] = fmaxf(nd.b.z, nd.d.z);
+    }
+    if (escape) escape[at] = r == n - 1 ? -1 : 2 * karras_index(nodes, keys, n, r + 1) + 1;
 }
 
 __global__ void k_f4_to_boxes6(int64_t n, const float4* __restrict__ in, float* __restrict__ b6) {
@@ -223,13 +246,13 @@ void gvc_ctx_destroy(gvc_ctx* ctx) {
     Lbvh* lbvhs[] = {&c->s_sort,  &c->gsort,        &c->cells,       &c->knn,
                      &c->ts_sort, &c->scratch.dbg, &c->scratch.msamp};
     for (Lbvh* L : lbvhs) {
-        DevBuf* bufs[] = {&L->keys, &L->keys_alt, &L->perm, &L->perm_alt, &L->boxes, &L->sorted_boxes, &L->left,
-                          &L->right, &L->parent, &L->flags, &L->node_boxes, &L->nodes, &L->hist, &L->bounds,
+        DevBuf* bufs[] = {&L->keys, &L->keys_alt, &L->perm, &L->perm_alt, &L->boxes, &L->sorted_boxes,
+                          &L->flags, &L->nodes, &L->hist, &L->bounds,
                           &L->onesweep};
         for (DevBuf* b : bufs) b->release();
     }
     DevBuf* bufs[] = {&c->s_sorted, &c->fwd_sorted, &c->blk_desc, &c->blk_boxes, &c->blk_desc_c, &c->blk_boxes_c, &c->b_rows, &c->b_boxes, &c->gtree, &c->s_grad, &c->s_gyz, &c->s_ok, &c->grec, &c->gtmp,
-                      &c->m_out_sorted, &c->knn_boxes, &c->ts_points, &c->ts_words, &c->cell_tree, &c->cell_recs, &c->scratch.gacc, &c->scratch.tmp_boxes, &c->scratch.tmp_out,
+                      &c->m_out_sorted, &c->knn_points, &c->ts_points, &c->ts_words, &c->cell_tree, &c->cell_recs, &c->scratch.gacc, &c->scratch.tmp_boxes, &c->scratch.tmp_out,
                       &c->clog, &c->cmask, &c->cend};
     for (DevBuf* b : bufs) b->release();
     c->scratch.stage.release();
@@ -732,12 +755,12 @@ int gvc_knn3_mean_dist2(gvc_ctx* ctx, int64_t n, const float* pts, float* out, v
     if (n == 0) return GVC_OK;
     if (!pts || !out) return fail(ctx, GVC_ERR_ARG, "null pointer");
     cudaStream_t st = (cudaStream_t)stream;
-    GVC_CUDA(ctx->knn_boxes.ensure(sizeof(float4) * 2 * n), "alloc point boxes");
-    GVC_CUDA(launch_point_boxes(n, pts, ctx->knn_boxes.as<float4>(), st), "point boxes");
-    GVC_CUDA(lbvh_build_boxes(ctx->knn, n, ctx->knn_boxes.as<float4>(), st), "point LBVH");
-    GVC_CUDA(launch_knn3(n, ctx->knn.sorted_boxes.as<float4>(), ctx->knn.perm.as<int32_t>(),
-                         ctx->knn.nodes.as<BvhNode>(), out, ctx->d_status, st),
-             "knn3");
+    GVC_CUDA(morton_sort_points(ctx->knn, n, pts, st), "point order");
+    GVC_CUDA(ctx->knn_points.ensure(sizeof(float4) * n), "alloc points");
+    float4* sorted = ctx->knn_points.as<float4>();
+    GVC_CUDA(launch_knn_points(n, pts, ctx->knn.perm.as<int32_t>(), sorted, st), "sorted points");
+    GVC_CUDA(lbvh_hierarchy_points(ctx->knn, n, ctx->knn.keys.as<uint32_t>(), sorted, st), "point LBVH");
+    GVC_CUDA(launch_knn3(n, sorted, ctx->knn.nodes.as<BvhNode>(), out, ctx->d_status, st), "knn3");
     return GVC_OK;
 }
 
@@ -890,15 +913,9 @@ int gvc_debug_lbvh(gvc_ctx* ctx, int64_t n, const float* boxes, uint32_t* keys_s
     if (perm)
         GVC_CUDA(cudaMemcpyAsync(perm, sc->dbg.perm.ptr, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, st),
                  "copy perm");
-    if (n > 1) {
-        if (left)
-            GVC_CUDA(cudaMemcpyAsync(left, sc->dbg.left.ptr, sizeof(int32_t) * (n - 1), cudaMemcpyDeviceToDevice, st),
-                     "copy left");
-        if (right)
-            GVC_CUDA(
-                cudaMemcpyAsync(right, sc->dbg.right.ptr, sizeof(int32_t) * (n - 1), cudaMemcpyDeviceToDevice, st),
-                "copy right");
-        if (node_boxes) k_f4_to_boxes6<<<nb(n - 1, 256), 256, 0, st>>>(n - 1, sc->dbg.node_boxes.as<float4>(), node_boxes); gvc::note_launch();
+    if (n > 1 && (left || right || node_boxes)) {
+        k_karras_tree<<<nb(n - 1, 256), 256, 0, st>>>((int)n, sc->dbg.nodes.as<BvhNode>(), sc->dbg.keys.as<uint32_t>(),
+                                                      left, right, node_boxes, nullptr); gvc::note_launch();
     }
     GVC_CUDA(cudaGetLastError(), "debug lbvh");
     return GVC_OK;
@@ -909,9 +926,13 @@ int gvc_debug_lbvh_escape(gvc_ctx* ctx, int32_t* escape, void* stream) {
     Scratch* sc = scratch_of(ctx);
     const int64_t n = sc->dbg.n;
     if (n <= 0) return fail(ctx, GVC_ERR_STATE, "gvc_debug_lbvh has not built a tree");
-    const int64_t ni = n > 1 ? n - 1 : 1;
     cudaStream_t st = (cudaStream_t)stream;
-    k_node_escape<<<nb(ni, 256), 256, 0, st>>>(ni, sc->dbg.nodes.as<BvhNode>(), escape); gvc::note_launch();
+    if (n == 1) {
+        GVC_CUDA(cudaMemsetAsync(escape, 0xff, sizeof(int32_t), st), "debug lbvh escape");
+        return GVC_OK;
+    }
+    k_karras_tree<<<nb(n - 1, 256), 256, 0, st>>>((int)n, sc->dbg.nodes.as<BvhNode>(), sc->dbg.keys.as<uint32_t>(),
+                                                  nullptr, nullptr, nullptr, escape); gvc::note_launch();
     GVC_CUDA(cudaGetLastError(), "debug lbvh escape");
     return GVC_OK;
 }

@@ -36,11 +36,10 @@ struct __align__(16) GaussRec {
 };
 
 // LBVH internal node with both children's boxes: 64 bytes.
-//   a = (L.lo.xyz, left child bits), b = (L.hi.xyz, right child bits),
-//   c = (R.lo.xyz, escape edge),     d = (R.hi.xyz, right child bits)
-// Child encoding: internal node k >= 0; leaf i stored as (i | 0x80000000).  The escape
-// edge (2p + s: child s of node p, 0xffffffff for none) is the edge that follows this
-// node's subtree in pre-order: a walk by it needs no stack.
+//   a = (L.lo.xyz, left child),  b = (L.hi.xyz, first leaf),
+//   c = (R.lo.xyz, last leaf),   d = (R.hi.xyz, right child)
+// Child: internal node k > 0, or leaf i as (i | 0x80000000).  Node k > 0 holds the leaves from
+// its first to k - 1 on its left and from k to its last on its right; node 0 is the root's copy.
 struct __align__(16) BvhNode {
     float4 a, b, c, d;
 };
@@ -93,9 +92,8 @@ struct Lbvh {
     DevBuf keys, keys_alt, perm, perm_alt;  // sorted keys / permutation (sorted pos -> input idx)
     DevBuf boxes;                           // input boxes [n] as 2 x float4 (lo, hi)
     DevBuf sorted_boxes;                    // leaf boxes in sorted order, 2 x float4
-    DevBuf left, right, parent, flags;      // Karras hierarchy + refit counters
-    DevBuf node_boxes;                      // [n-1] internal node boxes, 2 x float4
-    DevBuf nodes;                           // [n-1] BvhNode
+    DevBuf flags;                           // children that have reached a node
+    DevBuf nodes;                           // [n] BvhNode
     DevBuf hist, bounds;                    // sort histograms, centroid bounds
     DevBuf onesweep;                        // one-kernel-per-pass sort: digit counts, tickets, look-back words
     int* status = nullptr;                  // device status word; null keeps the three-kernel sort passes
@@ -170,7 +168,7 @@ struct gvc_ctx {
     gvc::Lbvh cells;
     // three-nearest-neighbour distances (point LBVH and its leaf boxes)
     gvc::Lbvh knn;
-    gvc::DevBuf knn_boxes;
+    gvc::DevBuf knn_points;
     // training sample batches: unsorted points, Morton / batch key words, FP64 values
     gvc::Lbvh ts_sort;
     gvc::DevBuf ts_points, ts_words, cell_tree, cell_recs;

@@ -23,10 +23,8 @@ struct LbvhBytes {
     }
     static constexpr size_t bounds() { return sizeof(uint32_t) * 8; }
     static constexpr size_t sorted_boxes(int64_t n) { return 2 * 16 * (size_t)n; }
-    static constexpr size_t child(int64_t n) { return sizeof(int32_t) * (size_t)internal(n); }  // left, right, flags
-    static constexpr size_t parent(int64_t n) { return sizeof(int32_t) * 2 * (size_t)n; }
-    static constexpr size_t node_boxes(int64_t n) { return 2 * 16 * (size_t)internal(n); }
-    static constexpr size_t nodes(int64_t n) { return sizeof(BvhNode) * (size_t)internal(n); }
+    static constexpr size_t flags(int64_t n) { return sizeof(uint32_t) * (size_t)internal(n); }
+    static constexpr size_t nodes(int64_t n) { return sizeof(BvhNode) * (size_t)n; }
 };
 
 // Stable LSD sort of n indices by a key of several 32-bit words (words[0] least
@@ -41,9 +39,25 @@ cudaError_t morton_sort_boxes(Lbvh& L, int64_t n, const float4* boxes, cudaStrea
 // Same for points [n][3].
 cudaError_t morton_sort_points(Lbvh& L, int64_t n, const float* pts, cudaStream_t st);
 
-// Karras hierarchy + refit + node packing over keys/leaf boxes already in sorted order.
+// Common prefix of the keys at i and j of the sorted order, equal keys told apart by position.
+__device__ __forceinline__ int lbvh_delta(const uint32_t* __restrict__ keys, int i, int j) {
+    const uint32_t a = keys[i], b = keys[j];
+    return a == b ? 32 + __clz((uint32_t)(i ^ j)) : __clz(a ^ b);
+}
+// Whether the subtree over the leaves [l, r], not all n, is its parent's left child.
+__device__ __forceinline__ bool lbvh_is_left(const uint32_t* __restrict__ keys, int n, int l, int r) {
+    if (l == 0) return true;
+    if (r == n - 1) return false;
+    return lbvh_delta(keys, r, r + 1) > lbvh_delta(keys, l - 1, l);
+}
+
+// The tree (L.nodes) over keys and leaf boxes already in sorted order.
 cudaError_t lbvh_hierarchy(Lbvh& L, int64_t n, const uint32_t* sorted_keys, const float4* sorted_leaf_boxes,
                            cudaStream_t st);
+
+// The same over points (x, y, z, any).
+cudaError_t lbvh_hierarchy_points(Lbvh& L, int64_t n, const uint32_t* sorted_keys, const float4* sorted_points,
+                                  cudaStream_t st);
 
 // Full build from boxes in input order: keys, sort, gather, hierarchy.
 cudaError_t lbvh_build_boxes(Lbvh& L, int64_t n, const float4* boxes, cudaStream_t st);

@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(128) k_sample_tets(int64_t N, const float* __r
             const int node = stack[--sp];
             const float4* np = reinterpret_cast<const float4*>(nodes + node);
             const float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2), d = __ldg(np + 3);
-            const uint32_t ch[2] = {__float_as_uint(a.w), __float_as_uint(b.w)};
+            const uint32_t ch[2] = {__float_as_uint(a.w), __float_as_uint(d.w)};
             const bool hit[2] = {a.x <= p[0] && p[0] <= b.x && a.y <= p[1] && p[1] <= b.y && a.z <= p[2] && p[2] <= b.z,
                                  c.x <= p[0] && p[0] <= d.x && c.y <= p[1] && p[1] <= d.y && c.z <= p[2] && p[2] <= d.z};
             for (int k = 0; k < 2; k++) {

@@ -52,12 +52,8 @@ constexpr size_t kOffPermAlt = kOffPerm + up(LbvhBytes::keys(kC));
 constexpr size_t kOffHist = kOffPermAlt + up(LbvhBytes::keys(kC));
 constexpr size_t kOffBounds = kOffHist + up(LbvhBytes::hist(kC));
 constexpr size_t kOffSorted = kOffBounds + up(LbvhBytes::bounds());
-constexpr size_t kOffLeft = kOffSorted + up(LbvhBytes::sorted_boxes(kC));
-constexpr size_t kOffRight = kOffLeft + up(LbvhBytes::child(kC));
-constexpr size_t kOffParent = kOffRight + up(LbvhBytes::child(kC));
-constexpr size_t kOffFlags = kOffParent + up(LbvhBytes::parent(kC));
-constexpr size_t kOffNodeBoxes = kOffFlags + up(LbvhBytes::child(kC));
-constexpr size_t kOffNodes = kOffNodeBoxes + up(LbvhBytes::node_boxes(kC));
+constexpr size_t kOffFlags = kOffSorted + up(LbvhBytes::sorted_boxes(kC));
+constexpr size_t kOffNodes = kOffFlags + up(LbvhBytes::flags(kC));
 constexpr size_t kScratchBytes = kOffNodes + up(LbvhBytes::nodes(kC));  // about 6.4 MB
 static_assert(kScratchBytes < (size_t(8) << 20), "the static scratch array is meant to stay modest");
 static_assert(kOffBoxes % 16 == 0 && kOffSorted % 16 == 0 && kOffNodes % 64 == 0, "region alignment");
@@ -153,11 +149,7 @@ extern "C" int gvc_sample_tets_static(int64_t npts, const float* pts, int64_t C,
         L.hist = view(base, kOffHist, LbvhBytes::hist(kC));
         L.bounds = view(base, kOffBounds, LbvhBytes::bounds());
         L.sorted_boxes = view(base, kOffSorted, LbvhBytes::sorted_boxes(kC));
-        L.left = view(base, kOffLeft, LbvhBytes::child(kC));
-        L.right = view(base, kOffRight, LbvhBytes::child(kC));
-        L.parent = view(base, kOffParent, LbvhBytes::parent(kC));
-        L.flags = view(base, kOffFlags, LbvhBytes::child(kC));
-        L.node_boxes = view(base, kOffNodeBoxes, LbvhBytes::node_boxes(kC));
+        L.flags = view(base, kOffFlags, LbvhBytes::flags(kC));
         L.nodes = view(base, kOffNodes, LbvhBytes::nodes(kC));
         // every view must hold what the builder asks for C boxes; then none of its
         // ensure() calls reallocates (an undersized view would be freed as if it were
@@ -168,9 +160,7 @@ extern "C" int gvc_sample_tets_static(int64_t npts, const float* pts, int64_t C,
         } need[] = {{L.keys, LbvhBytes::keys(C)},          {L.keys_alt, LbvhBytes::keys(C)},
                     {L.perm, LbvhBytes::keys(C)},          {L.perm_alt, LbvhBytes::keys(C)},
                     {L.hist, LbvhBytes::hist(C)},          {L.bounds, LbvhBytes::bounds()},
-                    {L.sorted_boxes, LbvhBytes::sorted_boxes(C)}, {L.left, LbvhBytes::child(C)},
-                    {L.right, LbvhBytes::child(C)},        {L.parent, LbvhBytes::parent(C)},
-                    {L.flags, LbvhBytes::child(C)},        {L.node_boxes, LbvhBytes::node_boxes(C)},
+                    {L.sorted_boxes, LbvhBytes::sorted_boxes(C)}, {L.flags, LbvhBytes::flags(C)},
                     {L.nodes, LbvhBytes::nodes(C)}};
         for (const auto& r : need) {
             if (r.b.bytes < r.need) {
@@ -179,8 +169,7 @@ extern "C" int gvc_sample_tets_static(int64_t npts, const float* pts, int64_t C,
             }
         }
         const void* before[] = {L.keys.ptr, L.keys_alt.ptr, L.perm.ptr, L.perm_alt.ptr, L.hist.ptr, L.bounds.ptr,
-                                L.sorted_boxes.ptr, L.left.ptr, L.right.ptr, L.parent.ptr, L.flags.ptr,
-                                L.node_boxes.ptr, L.nodes.ptr};
+                                L.sorted_boxes.ptr, L.flags.ptr, L.nodes.ptr};
         float4* boxes = reinterpret_cast<float4*>(base + kOffBoxes);
         if ((e = gvc::launch_tet_boxes(C, pts, conn4, boxes, st)) != cudaSuccess ||
             (e = gvc::lbvh_build_boxes(L, C, boxes, st)) != cudaSuccess) {
@@ -188,8 +177,7 @@ extern "C" int gvc_sample_tets_static(int64_t npts, const float* pts, int64_t C,
             return GVC_ERR_CUDA;
         }
         const void* after[] = {L.keys.ptr, L.keys_alt.ptr, L.perm.ptr, L.perm_alt.ptr, L.hist.ptr, L.bounds.ptr,
-                               L.sorted_boxes.ptr, L.left.ptr, L.right.ptr, L.parent.ptr, L.flags.ptr,
-                               L.node_boxes.ptr, L.nodes.ptr};
+                               L.sorted_boxes.ptr, L.flags.ptr, L.nodes.ptr};
         if (std::memcmp(before, after, sizeof(before)) != 0) {  // a region was too small: never expected
             set_msg(errbuf, errbuf_len, "gvc_sample_tets_static: scratch layout too small");
             return GVC_ERR_CAPACITY;

@@ -210,9 +210,9 @@ cudaError_t launch_tet_points(int64_t N, int64_t S, uint64_t seed, const float* 
                               float* out, uint32_t* w_lo, uint32_t* w_hi, uint32_t* w_batch, cudaStream_t st);
 cudaError_t launch_gather_points(int64_t N, const float* src, const int32_t* perm, float* dst, cudaStream_t st);
 
-// knn.cu
-cudaError_t launch_point_boxes(int64_t n, const float* pts, float4* boxes, cudaStream_t st);
-cudaError_t launch_knn3(int64_t n, const float4* sorted_boxes, const int32_t* perm, const BvhNode* nodes, float* out,
-                        int* status, cudaStream_t st);
+// knn.cu: the points in Morton order with their index in .w, and the LBVH over them
+cudaError_t launch_knn_points(int64_t n, const float* pts, const int32_t* perm, float4* sorted, cudaStream_t st);
+cudaError_t launch_knn3(int64_t n, const float4* sorted, const BvhNode* nodes, float* out, int* status,
+                        cudaStream_t st);
 
 }  // namespace gvc

@@ -67,7 +67,7 @@ __device__ __forceinline__ int warp_traverse(const BvhNode* __restrict__ nodes, 
             const float4* np = reinterpret_cast<const float4*>(nodes + node);
             const float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2), d = __ldg(np + 3);
             cl = __float_as_uint(a.w);
-            cr = __float_as_uint(b.w);
+            cr = __float_as_uint(d.w);
             hl = box_overlap(a, b, qlo, qhi);
             hr = box_overlap(c, d, qlo, qhi);
         }
