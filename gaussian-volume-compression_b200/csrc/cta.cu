@@ -537,11 +537,13 @@ __global__ void __launch_bounds__(kConsumerWarps * 32 + 32, kCtaMinBlocks)
                     const float x = xr[k], y = yr[k], z = zr[k];
                     const bool in = inr[k];
                     const float dx = x - r0.x, dy = y - r0.y, dz = z - r0.z;
-                    const float p2 = dx * fmaf(r1.x, dx, fmaf(r1.y, dy, r1.z * dz)) + dy * fmaf(r1.w, dy, r2.x * dz) +
-                                     dz * (r2.y * dz);
+                    // roundings spelled out as in fwd_blocks.cu, whose sums these must equal bit for bit
+                    float p2 = __fmul_rn(dx, fmaf(r1.x, dx, fmaf(r1.y, dy, __fmul_rn(r1.z, dz))));
+                    p2 = fmaf(dy, fmaf(r1.w, dy, __fmul_rn(r2.x, dz)), p2);
+                    p2 = fmaf(dz, __fmul_rn(r2.y, dz), p2);
                     const bool cc = in && p2 >= kLog2Floor && p2 <= 0.0f;
-                    const float wt = cc ? r0.w * ex2_approx(p2) : 0.f;
-                    Wr[k] += wt;
+                    const float wt = cc ? __fmul_rn(r0.w, ex2_approx(p2)) : 0.f;
+                    Wr[k] = __fadd_rn(Wr[k], wt);
                     Vr[k] = fmaf(wt, r2.z, Vr[k]);
                     if (COUNT) {
                         ncand += in ? 1 : 0;

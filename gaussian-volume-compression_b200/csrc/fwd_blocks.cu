@@ -75,12 +75,16 @@ struct BlockEval {
         const bool inside = bl.x <= x[k] && x[k] <= bh.x && bl.y <= y[k] && y[k] <= bh.y && bl.z <= z[k] &&
                             z[k] <= bh.z;
         const float dx = x[k] - a.x, dy = y[k] - a.y, dz = z[k] - a.z;
-        const float t = dx * fmaf(s.x, dx, fmaf(s.y, dy, s.z * dz)) + dy * fmaf(s.w, dy, bl.w * dz) + dz * (bh.w * dz);
+        // every rounding spelled out: the compiler's choice of what to fuse would differ from one
+        // instantiation to the next, and with it the last bit (see the top)
+        float t = __fmul_rn(dx, fmaf(s.x, dx, fmaf(s.y, dy, __fmul_rn(s.z, dz))));
+        t = fmaf(dy, fmaf(s.w, dy, __fmul_rn(bl.w, dz)), t);
+        t = fmaf(dz, __fmul_rn(bh.w, dz), t);
         // t = -p2 is in the window [0, -kLog2Floor] iff its bits, as an unsigned number, are at
         // most the floor's (a negative t or a NaN has larger ones; t is never -0: the squares
         // enter it as +0)
         const bool c = inside && __float_as_uint(t) <= __float_as_uint(-kLog2Floor);
-        wt = a.w * ex2_approx(-t);
+        wt = __fmul_rn(a.w, ex2_approx(-t));
         if (COUNT) {
             n_cand += inside;
             n_contrib += c;
@@ -156,14 +160,14 @@ struct BlockEval {
                 }
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    W[0] += wt[i];
+                    W[0] = __fadd_rn(W[0], wt[i]);
                     V[0] = fmaf(wt[i], v4[i], V[0]);
                 }
             }
             for (; j < np; j++) {
                 float vj;
                 const float wt = pair(j, 0, vj);
-                W[0] += wt;
+                W[0] = __fadd_rn(W[0], wt);
                 V[0] = fmaf(wt, vj, V[0]);
             }
         } else {
@@ -177,7 +181,7 @@ struct BlockEval {
                     if (!(chains & (1u << k))) continue;  // warp-uniform
                     float wt;
                     if (weight(a, s, bl, bh, k, wt)) {
-                        W[k] += wt;
+                        W[k] = __fadd_rn(W[k], wt);
                         V[k] = fmaf(wt, vm.x, V[k]);
                     }
                 }

@@ -44,3 +44,31 @@ def test_sizes_match_oracle(ctx, cuda, orc, mode, P, S):
     ro, rw = orc.forward(means, values, weights, gc.astype(np.float64), gb, pts)
     compare_forward(out.cpu().numpy(), outw.cpu().numpy(), ro, rw, 2e-5, 2e-5)
     assert (ro != -1).any()
+
+
+@pytest.mark.parametrize("path", ["plain", "tensor_core"])
+def test_one_order_of_sums(cuda, orc, path):
+    """With the tensor-core backward selected a sample's sums are the same bits whatever kernel
+    the number of samples selects: 38400 samples alone (32 rows per warp), and followed by
+    copies of the last corner, which sort behind them and leave their blocks as they are, up to
+    a CTA per block and up to a warp per block."""
+    from bvh_diff_gaussian_rasterization import _C
+    means, scales, rots, values, weights = orc.mixture_small(seed=3, P=3000)
+    n = 128 * 300
+    pts = np.random.default_rng(5).random((n, 3)).astype(np.float32)
+    pts[0], pts[1] = 0.0, 1.0
+    got = []
+    _C.set_backward_mode("tensor_core")
+    _C.set_eval_path(path)
+    try:
+        for more in (0, 70_000, 480_000):
+            all_pts = np.concatenate([pts, np.ones((more, 3), np.float32)])
+            out, outw, _ = run_forward(cuda, means, scales, rots, values, weights, all_pts)
+            got.append((out[:n].cpu().numpy(), outw[:n].cpu().numpy()))
+    finally:
+        _C.set_backward_mode("auto")
+        _C.set_eval_path("plain")
+    assert (got[0][1] > 0).any()
+    for out, outw in got[1:]:
+        np.testing.assert_array_equal(out, got[0][0])
+        np.testing.assert_array_equal(outw, got[0][1])
