@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(256) k_cell_boxes(int64_t C, const float* __re
 // A thread per sample with a stack of its own took a chain of twenty dependent node loads and
 // three dependent gathers per cell (id, vertex numbers, vertices; here one 64-byte record), and
 // ran every containment test at the pace of the warp's slowest lane: 1.57M tetrahedra x 25M
-// samples 16.7 ms against 9.9.  Testing each sample against every cell met instead took
+// samples 16.7 ms against 9.1.  Testing each sample against every cell met instead took
 // 11.3k instructions per warp there, 16.4 ms.
 // ---------------------------------------------------------------------------------
 struct LocateSmem {
@@ -492,15 +492,21 @@ __device__ __noinline__ int2 expand(LocateSmem& sm, const WideTree& tree, const 
     __syncwarp();
     const int2 q = lane < n ? sm.nodes[off + lane] : make_int2(0, 0);
     const float x = sm.px[q.y], y = sm.py[q.y], z = sm.pz[q.y];
+    // the eight loads together, then the pairs
+    uint32_t hits = 0;
+    const float4* p = tree.box[0] + 2 * (int64_t)(q.x * kWideLeaves);
+    const int leaves = lane < n ? min(tree.n[0] - q.x * kWideLeaves, kWideLeaves) : 0;
+#pragma unroll
+    for (int k = 0; k < kWideLeaves; k++) {
+        if (k < leaves) {
+            const float4 lo = __ldg(p + 2 * k), hi = __ldg(p + 2 * k + 1);
+            if (lo.x <= x && x <= hi.x && lo.y <= y && y <= hi.y && lo.z <= z && z <= hi.z) hits |= 1u << k;
+        }
+    }
 #pragma unroll 1
     for (int k = 0; k < kWideLeaves; k++) {
         const int leaf = q.x * kWideLeaves + k;
-        bool h = false;
-        if (lane < n && leaf < tree.n[0]) {
-            const float4* p = tree.box[0] + 2 * (int64_t)leaf;
-            const float4 lo = __ldg(p), hi = __ldg(p + 1);
-            h = lo.x <= x && x <= hi.x && lo.y <= y && y <= hi.y && lo.z <= z && z <= hi.z;
-        }
+        const bool h = (hits >> k) & 1u;
         const uint32_t m = __ballot_sync(0xffffffffu, h);
         if (h) sm.cells[len.x + __popc(m & lt)] = make_int2(leaf, q.y);
         len.x += __popc(m);
