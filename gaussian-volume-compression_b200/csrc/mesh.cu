@@ -552,7 +552,7 @@ struct Locator {
 
 // `rows` samples per warp, a power of two up to 32.
 template <bool TETS, class Out>
-__global__ void __launch_bounds__(32, TETS ? 28 : 12)
+__global__ void __launch_bounds__(32, TETS ? 28 : 16)
     k_locate(int64_t N, int rows, const float* __restrict__ samples, const int32_t* __restrict__ sperm,
              const __grid_constant__ WideTree tree, const __grid_constant__ CellMesh mesh, Out* __restrict__ out,
              int64_t* __restrict__ cell_ids) {
