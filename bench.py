@@ -61,14 +61,14 @@ FP32_NOMINAL_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the dominant
 # kernels at the 2M x 16M workload, from one single-pass capture of
 # `ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none
-#  -k regex:"k_backward_cta|k_forward_cta" -s 2 -c 2 python bench.py --profile --steps 1 --warmup 1`
+#  -k regex:"k_backward_cta|k_forward_blocks" -s 2 -c 2 python bench.py --profile --steps 1 --warmup 1`
 # (and of k_backward_gauss with --bwd-mode deterministic); other workloads report null.
 # Tensor-pipe activity (sm__pipe_tc_cycles_active, share of peak) of the tensor-core kernels
 # in their committed --set full captures of the 2M x 4M profiling case (profiles/).
 TENSOR_PIPE_ACTIVE = {"k_backward_cta": 0.358, "k_forward_tc": 0.189}
-MEASURED_TRAFFIC = {("large", "k_backward_cta"): 1.291e9 + 0.142e9,
-                    ("large", "k_backward_gauss"): 1.475e9 + 0.125e9,
-                    ("large", "k_forward_cta"): 1.585e9 + 1.774e9}
+MEASURED_TRAFFIC = {("large", "k_backward_cta"): 1.425e9 + 0.143e9,
+                    ("large", "k_backward_gauss"): 1.327e9 + 0.124e9,
+                    ("large", "k_forward_blocks"): 1.938e9 + 1.873e9}
 
 
 def parse():
@@ -84,7 +84,7 @@ def parse():
     p.add_argument("--bwd-mode", default="tensor_core", choices=["auto", "deterministic", "atomic", "tensor_core"])
     p.add_argument("--eval-path", default="plain", choices=["plain", "tensor_core", "plain_tile"])
     p.add_argument("--traversal", default="stack", choices=["stack", "stackless"],
-                   help="Gaussian-LBVH traversal of the block-group kernels (both are timed in tc_vs_plain)")
+                   help="accepted, without effect (GVC_OPT_TRAVERSAL)")
     p.add_argument("--use-gaussian-bvh", action="store_true")
     p.add_argument("--no-e2e", action="store_true")
     p.add_argument("--no-cpu-baseline", action="store_true")
@@ -475,7 +475,7 @@ def mesh_bench(dev, steps, warmup, with_cpu):
                                 gvc_native.ptr(d_tets), gvc_native.ptr(d_vals), n_pts, gvc_native.ptr(d_q),
                                 gvc_native.ptr(d_out), gvc_native.ptr(d_cell), sp))
     tet = {"cells": int(tets.shape[0]), "points": n_pts, "ms_per_call": ms, "points_per_s": n_pts / (ms * 1e-3),
-           "includes": "cell LBVH build (keys, sort, Karras, refit) + point sort + locate + interpolate",
+           "includes": "cell tree build (keys, sort, boxes, records) + point sort + locate + interpolate",
            "found": float((d_cell >= 0).float().mean().item())}
     if with_cpu:
         sys.path.insert(0, os.path.join(ROOT, "oracle"))
@@ -733,7 +733,7 @@ def knn_bench(dev, means, steps, warmup, with_cpu):
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1) / steps
     res = {"points": n, "ms_per_call": ms, "points_per_s": n / (ms * 1e-3),
-           "includes": "point LBVH build (keys, sort, Karras, refit) + exact 3-NN traversal",
+           "includes": "point LBVH build (keys, sort, tree) + exact 3-NN traversal",
            "points_desc": "Gaussian means of the headline workload (256 clusters)"}
     if with_cpu:
         sys.path.insert(0, os.path.join(ROOT, "oracle"))
@@ -832,7 +832,7 @@ def run_ours(args):
     hbm, bf16, bf16s, src = measured_peaks()
     bwd_kernel = "k_backward_cta" if args.bwd_mode == "tensor_core" or (
         args.eval_path == "tensor_core" and args.bwd_mode == "auto") else "k_backward_gauss"
-    fwd_kernel = "k_forward" if args.eval_path == "plain_tile" else "k_forward_cta"
+    fwd_kernel = "k_forward_tc" if args.eval_path == "tensor_core" else "k_forward_blocks"
     if t_bwd >= t_fwd:
         name, flops, t_k = bwd_kernel, f_bwd, t_bwd
     else:
@@ -1018,9 +1018,9 @@ def run_ours(args):
         tc_vs_plain = {"plain_ms_per_step": paths["plain"]["ms_per_step"],
                        "tensor_core_ms_per_step": paths["tensor_core"]["ms_per_step"],
                        "speedup_tc_over_plain": paths["plain"]["ms_per_step"] / paths["tensor_core"]["ms_per_step"],
-                       "paths": {"plain": "FP32 CTA forward + FP32 deterministic Gaussian-owned backward",
+                       "paths": {"plain": "FP32 forward + FP32 deterministic Gaussian-owned backward",
                                  "tensor_core": "tcgen05 split-BF16 exponent forward + tcgen05 moment backward",
-                                 "plain_fwd_tc_bwd": "FP32 CTA forward + tcgen05 moment backward",
+                                 "plain_fwd_tc_bwd": "FP32 forward + tcgen05 moment backward",
                                  "plain_fwd_tc_bwd_walk": "the same with the backward walking the Gaussian "
                                                           "LBVH again instead of reading the forward's "
                                                           "candidate log"},

@@ -521,7 +521,8 @@ static bool dense_samples(const BwdArgs& a) { return a.S >= a.P; }
 __global__ void __launch_bounds__(128) k_log_masks(const uint2* __restrict__ cdesc, const uint2* __restrict__ bdesc,
                                                    const float4* __restrict__ bboxes,
                                                    const GaussRec* __restrict__ recs, const int32_t* __restrict__ clog,
-                                                   const int32_t* __restrict__ cend, bool window, uint8_t* __restrict__ cmask) {
+                                                   const int32_t* __restrict__ cend, bool window,
+                                                   uint8_t* __restrict__ cmask) {
     const int64_t blk = blockIdx.x;
     const uint2 cd = cdesc[blk], bd = bdesc[blk];
     const int cng = (int)(cd.y >> 24), ng = (int)(bd.y >> 24);

@@ -25,7 +25,6 @@ namespace {
 struct Scratch {
     DevBuf gacc;       // [P][16] per-Gaussian gradient accumulators
     DevBuf tmp_boxes;  // debug hooks / tet boxes
-    DevBuf tmp_out;
     Lbvh dbg;          // debug LBVH
     Lbvh msamp;        // Morton order of mesh sample points
     Stage stage;       // pinned chunks for host arrays
@@ -246,14 +245,15 @@ void gvc_ctx_destroy(gvc_ctx* ctx) {
     Lbvh* lbvhs[] = {&c->s_sort,  &c->gsort,        &c->cells,       &c->knn,
                      &c->ts_sort, &c->scratch.dbg, &c->scratch.msamp};
     for (Lbvh* L : lbvhs) {
-        DevBuf* bufs[] = {&L->keys, &L->keys_alt, &L->perm, &L->perm_alt, &L->boxes, &L->sorted_boxes,
+        DevBuf* bufs[] = {&L->keys, &L->keys_alt, &L->perm, &L->perm_alt, &L->sorted_boxes,
                           &L->flags, &L->nodes, &L->hist, &L->bounds,
                           &L->onesweep};
         for (DevBuf* b : bufs) b->release();
     }
-    DevBuf* bufs[] = {&c->s_sorted, &c->fwd_sorted, &c->blk_desc, &c->blk_boxes, &c->blk_desc_c, &c->blk_boxes_c, &c->b_rows, &c->b_boxes, &c->gtree, &c->s_grad, &c->s_gyz, &c->s_ok, &c->grec, &c->gtmp,
-                      &c->m_out_sorted, &c->knn_points, &c->ts_points, &c->ts_words, &c->cell_tree, &c->cell_recs, &c->scratch.gacc, &c->scratch.tmp_boxes, &c->scratch.tmp_out,
-                      &c->clog, &c->cmask, &c->cend};
+    DevBuf* bufs[] = {&c->s_sorted, &c->fwd_sorted, &c->blk_desc, &c->blk_boxes, &c->blk_desc_c, &c->blk_boxes_c,
+                      &c->b_rows, &c->b_boxes, &c->gtree, &c->s_grad, &c->s_gyz, &c->s_ok, &c->grec, &c->gtmp,
+                      &c->knn_points, &c->ts_points, &c->ts_words, &c->cell_tree, &c->cell_recs, &c->clog, &c->cmask,
+                      &c->cend, &c->scratch.gacc, &c->scratch.tmp_boxes};
     for (DevBuf* b : bufs) b->release();
     c->scratch.stage.release();
     if (c->d_status) cudaFree(c->d_status);
@@ -649,7 +649,8 @@ int gvc_rasterize_gaussians_backward(gvc_ctx* ctx, int64_t P, const float* means
                 ba.cmask = ctx->cmask.as<uint8_t>();
                 ba.cend = ctx->cend.as<int32_t>();
                 ba.cdesc = ctx->blk_desc_c.as<uint2>();
-                if (!ctx->clog_masks || !same_gauss) GVC_CUDA(launch_log_masks(ba, ctx->cmask.as<uint8_t>(), st), "log masks");
+                if (!ctx->clog_masks || !same_gauss)
+                    GVC_CUDA(launch_log_masks(ba, ctx->cmask.as<uint8_t>(), st), "log masks");
                 ctx->clog_masks = true;
             }
             const int tk = timer_begin(ctx, st, 1);

@@ -260,7 +260,8 @@ __global__ void __launch_bounds__(192, kMinBlocks)
     k_forward_tc(const float4* __restrict__ s_sorted, int64_t S, const uint2* __restrict__ bdesc,
                  const float4* __restrict__ bboxes, const BvhNode* __restrict__ nodes,
                  const GaussRec* __restrict__ recs, float* __restrict__ out_cells, float* __restrict__ out_weights,
-                 float2* __restrict__ out_sorted, int32_t* __restrict__ clog, int32_t* __restrict__ cend, int* status, unsigned long long* stats) {
+                 float2* __restrict__ out_sorted, int32_t* __restrict__ clog, int32_t* __restrict__ cend, int* status,
+                 unsigned long long* stats) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     FwdTcSmem& sm = *reinterpret_cast<FwdTcSmem*>(
         smem_raw + ((1024 - (static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw)) & 1023)) & 1023));

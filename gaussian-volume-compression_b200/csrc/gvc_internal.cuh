@@ -10,9 +10,7 @@ namespace gvc {
 
 // diff-gaussian-rasterization/cuda_rasterizer/config.h:9
 constexpr float kWeightCutoff = 1e-2f;
-// forward.cu:166 / forward.cu:235: power window [-14, 0]
-constexpr float kPowerFloor = -14.0f;
-// Tile of Morton-sorted samples handled by one warp.
+// Sample slots are padded to a multiple of it.
 constexpr int kTile = 32;
 // Per-warp traversal stack (entries of int32) in shared memory.
 constexpr int kStackCap = 512;
@@ -90,7 +88,6 @@ struct DevBuf {
 struct Lbvh {
     int64_t n = 0;
     DevBuf keys, keys_alt, perm, perm_alt;  // sorted keys / permutation (sorted pos -> input idx)
-    DevBuf boxes;                           // input boxes [n] as 2 x float4 (lo, hi)
     DevBuf sorted_boxes;                    // leaf boxes in sorted order, 2 x float4
     DevBuf flags;                           // children that have reached a node
     DevBuf nodes;                           // [n] BvhNode
@@ -164,15 +161,15 @@ struct gvc_ctx {
     gvc::DevBuf gtree;      // leaf boxes in that order, and the wide tree's levels over them
     gvc::DevBuf grec;       // [P] GaussRec in Morton order
     gvc::DevBuf gtmp;       // preprocess scratch: AABBs in caller order
-    // mesh sampler
+    // mesh samplers: the cells' Morton order, the wide tree and the tetrahedra's records in it
     gvc::Lbvh cells;
-    // three-nearest-neighbour distances (point LBVH and its leaf boxes)
+    gvc::DevBuf cell_tree, cell_recs;
+    // three-nearest-neighbour distances (points in Morton order and the LBVH over them)
     gvc::Lbvh knn;
     gvc::DevBuf knn_points;
-    // training sample batches: unsorted points, Morton / batch key words, FP64 values
+    // training sample batches: unsorted points, Morton / batch key words
     gvc::Lbvh ts_sort;
-    gvc::DevBuf ts_points, ts_words, cell_tree, cell_recs;
-    gvc::DevBuf m_out_sorted;
+    gvc::DevBuf ts_points, ts_words;
     // status and statistics
     int* d_status = nullptr;          // device status word
     unsigned long long* d_stats = nullptr;  // [16] device counters

@@ -92,7 +92,8 @@ cudaError_t Stage::upload(int device, int n, void* const* dst, const void* const
             // the slot's last transfer, this call's or an earlier one's
             if ((r = cudaEventSynchronize(event_[slot])) != cudaSuccess) break;
             std::memcpy(pin, (const char*)src[i] + off, (size_t)len);
-            if ((r = cudaMemcpyAsync((char*)dst[i] + off, pin, (size_t)len, cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
+            if ((r = cudaMemcpyAsync((char*)dst[i] + off, pin, (size_t)len, cudaMemcpyHostToDevice, st)) != cudaSuccess)
+                break;
             r = cudaEventRecord(event_[slot], st);
         }
         if (r != cudaSuccess) failed.store((int)r, std::memory_order_relaxed);

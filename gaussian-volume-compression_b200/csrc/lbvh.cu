@@ -536,7 +536,8 @@ __global__ void __launch_bounds__(256, 3) k_os_scatter(const uint32_t* __restric
         while (true) {
             uint32_t v[kOsWindow], every = ~0u, any = 0u, add = 0u;
 #pragma unroll
-            for (int i = 0; i < kOsWindow; i++) v[i] = k >= i ? ld_relaxed_gpu(lp + (int64_t)(k - i) * 256) : kOsInclusive;
+            for (int i = 0; i < kOsWindow; i++)
+                v[i] = k >= i ? ld_relaxed_gpu(lp + (int64_t)(k - i) * 256) : kOsInclusive;
 #pragma unroll
             for (int i = 0; i < kOsWindow; i++) {
                 every &= v[i];
@@ -946,7 +947,8 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_morton_sort_small(Src src,
 #pragma unroll
         for (int it = 0; it < kSmallRounds; it++) {
             if (it < rounds && first + 32 * it < n) {
-                const uint32_t p = sm.cnt[warp][(kreg[it] >> shift) & 255u] + ((rreg[it / 2] >> (16 * (it & 1))) & 0xffffu);
+                const uint32_t rank = (rreg[it / 2] >> (16 * (it & 1))) & 0xffffu;
+                const uint32_t p = sm.cnt[warp][(kreg[it] >> shift) & 255u] + rank;
                 sm.key[p] = kreg[it];
                 sm.val[p] = vreg[it];
             }
@@ -1003,7 +1005,8 @@ static cudaError_t morton_sort(Lbvh& L, int64_t n, Src src, cudaStream_t st) {
     const unsigned nbk = blocks_for(n, 256);
     k_bounds<Src><<<nbk < 148u * 8u ? nbk : 148u * 8u, 256, 0, st>>>(src, n, bounds); gvc::note_launch();
     if (os) {
-        k_keys<Src, true><<<nbk < 148u * 4u ? nbk : 148u * 4u, 256, 0, st>>>(src, n, bounds, L.keys.as<uint32_t>(), ghist);
+        k_keys<Src, true><<<nbk < 148u * 4u ? nbk : 148u * 4u, 256, 0, st>>>(src, n, bounds, L.keys.as<uint32_t>(),
+                                                                             ghist);
         gvc::note_launch();
         return radix_sort_onesweep(L, n, st);
     }

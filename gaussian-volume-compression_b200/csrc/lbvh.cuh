@@ -1,4 +1,4 @@
-// lbvh.cuh -- LBVH builder interface shared by the Gaussian, sample-tile and cell BVHs.
+// lbvh.cuh -- LBVH builder interface of the Gaussians, points and cells.
 #pragma once
 #include "gvc_internal.cuh"
 

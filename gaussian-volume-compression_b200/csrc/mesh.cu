@@ -345,10 +345,10 @@ __global__ void __launch_bounds__(256) k_cell_boxes(int64_t C, const float* __re
 // tested against the node's eight cells, and the (sample, cell) pairs that meet are queued in
 // turn, 32 at a time, so that no lane idles where samples meet different cells.  Of a
 // tetrahedron's pairs, seven in eight are told to be outside by its four planes in FP32 (an
-// error bound decides: k_cell_leaves); what they leave takes the containment test in double.  The lowest containing cell of each sample is kept in shared
-// memory.  A run of samples that jumps across the mesh would meet a large part of it: a walk
-// that has met 8 nodes per sample of the run is given up and the run halved, down to single
-// samples.
+// error bound decides: k_cell_leaves); what they leave takes the containment test in double.
+// The lowest containing cell of each sample is kept in shared memory.  A run of samples that
+// jumps across the mesh would meet a large part of it: a walk that has met 8 nodes per sample
+// of the run is given up and the run halved, down to single samples.
 //
 // A thread per sample with a stack of its own took a chain of twenty dependent node loads and
 // three dependent gathers per cell (id, vertex numbers, vertices; here one 64-byte record), and
@@ -550,7 +550,9 @@ struct Locator {
     }
 };
 
-// `rows` samples per warp, a power of two up to 32.
+// `rows` samples per warp, a power of two up to 32.  Blocks per SM asked for: tetrahedra 28 (72
+// registers; 32 and 24: 1 % and 6 % slower), other cells 16 (128 registers, for Newton's method;
+// 12 or 10 5 % and 8 36 % slower).
 template <bool TETS, class Out>
 __global__ void __launch_bounds__(32, TETS ? 28 : 16)
     k_locate(int64_t N, int rows, const float* __restrict__ samples, const int32_t* __restrict__ sperm,

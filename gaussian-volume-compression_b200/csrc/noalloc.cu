@@ -54,7 +54,7 @@ constexpr size_t kOffBounds = kOffHist + up(LbvhBytes::hist(kC));
 constexpr size_t kOffSorted = kOffBounds + up(LbvhBytes::bounds());
 constexpr size_t kOffFlags = kOffSorted + up(LbvhBytes::sorted_boxes(kC));
 constexpr size_t kOffNodes = kOffFlags + up(LbvhBytes::flags(kC));
-constexpr size_t kScratchBytes = kOffNodes + up(LbvhBytes::nodes(kC));  // about 6.4 MB
+constexpr size_t kScratchBytes = kOffNodes + up(LbvhBytes::nodes(kC));  // about 4.9 MB
 static_assert(kScratchBytes < (size_t(8) << 20), "the static scratch array is meant to stay modest");
 static_assert(kOffBoxes % 16 == 0 && kOffSorted % 16 == 0 && kOffNodes % 64 == 0, "region alignment");
 

@@ -1,6 +1,6 @@
 // pair.cuh -- the arithmetic of one (sample, Gaussian) pair shared by the forward and the
-// backward kernels: the base-2 power with staged coefficients, its window, and the
-// backward's moment accumulation.
+// backward kernels: the staged coefficients of the base-2 power, its window, and the terms that
+// the backward's moments make.
 #pragma once
 #include "gvc_internal.cuh"
 
@@ -47,31 +47,6 @@ __device__ __forceinline__ GaussB gauss_b(float mx, float my, float mz, float v,
     g.lx = lo.x; g.ly = lo.y; g.lz = lo.z;
     g.hx = hi.x; g.hy = hi.y; g.hz = hi.z;
     return g;
-}
-
-// p = (x, y, z, gx) with finite coordinates; gx = gyz = 0 makes every term exactly 0.
-// Branch-free: a pair outside the box or the power window gets e = 0.  Returns whether
-// the pair is inside the box and the window.
-__device__ __forceinline__ bool pair_moments(const GaussB& g, float4 p, float gyz, float (&m)[11]) {
-    const bool in = g.lx <= p.x && p.x <= g.hx && g.ly <= p.y && p.y <= g.hy && g.lz <= p.z && p.z <= g.hz;
-    const float dx = p.x - g.mx, dy = p.y - g.my, dz = p.z - g.mz;
-    const float p2 = dx * fmaf(g.q0, dx, fmaf(g.q1, dy, g.q2 * dz)) + dy * fmaf(g.q3, dy, g.q4 * dz) + dz * (g.q5 * dz);
-    const bool c = in && p2 >= kLog2Floor && p2 <= 0.0f;
-    const float e = c ? ex2_approx(p2) : 0.0f;
-    m[0] = fmaf(p.w, e, m[0]);
-    const float gs = fmaf(g.v, p.w, gyz) * e;
-    m[1] += gs;
-    const float gx = gs * dx, gy = gs * dy, gz = gs * dz;
-    m[2] += gx;
-    m[3] += gy;
-    m[4] += gz;
-    m[5] = fmaf(gx, dx, m[5]);
-    m[6] = fmaf(gx, dy, m[6]);
-    m[7] = fmaf(gx, dz, m[7]);
-    m[8] = fmaf(gy, dy, m[8]);
-    m[9] = fmaf(gy, dz, m[9]);
-    m[10] = fmaf(gz, dz, m[10]);
-    return c;
 }
 
 // After warp_transpose_reduce16 lanes 2k, 2k+1 hold moment k; returns gradient field k

@@ -160,19 +160,6 @@ __device__ __forceinline__ void store_row_k16(unsigned char* tile, int r, const 
     *reinterpret_cast<uint4*>(base + 128) = hi;
 }
 
-// Splits 16 fp32 values into `terms` bf16 parts (hi, mid, lo): v = sum of parts to ~8*terms bits.
-__device__ __forceinline__ void split_bf16(const float (&v)[16], __nv_bfloat16 (&h)[16], __nv_bfloat16 (&m)[16],
-                                           __nv_bfloat16 (&l)[16]) {
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-        h[i] = __float2bfloat16_rn(v[i]);
-        const float r1 = v[i] - __bfloat162float(h[i]);
-        m[i] = __float2bfloat16_rn(r1);
-        const float r2 = r1 - __bfloat162float(m[i]);
-        l[i] = __float2bfloat16_rn(r2);
-    }
-}
-
 // ---- split-BF16 operand rows and narrower TMEM reads ------------------------------------
 __device__ __forceinline__ uint32_t bf2_bits(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
 

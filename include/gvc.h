@@ -77,7 +77,7 @@ typedef struct {
     int64_t fwd_contributing; /* ... and -14 <= power <= 0                                  */
     int64_t bwd_contributing; /* contributing pairs of samples with W > 0.01 (Gaussian-owned
                                  backward: of samples with a non-zero gradient)            */
-    int32_t max_stack_fwd;    /* 0 (the walks have no stack that could overflow)            */
+    int32_t max_stack_fwd;    /* deepest stack of the CTA kernels' LBVH walks (0: none)     */
     int32_t max_stack_bwd;
     double fwd_kernel_ms;     /* summed duration of the forward evaluation kernel          */
     double bwd_kernel_ms;     /* summed duration of the backward evaluation kernel         */
@@ -223,7 +223,7 @@ int gvc_check_cells(gvc_ctx* ctx, int64_t C, const int64_t* cell_types, const in
    allocate device memory (their memory belongs to another allocator, or cudaMalloc's
    device-wide synchronisation is unacceptable where they call).  Same inputs, outputs
    and results as gvc_sample_tets, but no context and no allocation: the scratch is one
-   static device array of about 6.4 MB in every device that loads the library, which
+   static device array of about 4.9 MB in every device that loads the library, which
    limits the mesh to C <= 32768 cells (larger meshes are rejected with
    GVC_ERR_CAPACITY and a message in errbuf).  The first call on a device looks up the
    array's device address; under CUDA's default lazy module loading that is also when
@@ -246,7 +246,7 @@ int gvc_sample_tets_static(int64_t npts, const float* pts, int64_t C, const int3
 int gvc_debug_lbvh(gvc_ctx* ctx, int64_t n, const float* boxes, uint32_t* keys_sorted, int32_t* perm,
                    int32_t* left, int32_t* right, float* node_boxes, void* stream);
 
-/* Test hook: the escape edges of the stackless traversal in the tree of the last
+/* Test hook: the escape edges (for a walk without a stack) of the tree of the last
    gvc_debug_lbvh call: escape [max(n-1, 1)] int32 (device), per internal node the edge
    2p + s (child s of node p) that follows its subtree in pre-order, -1 for none.  No
    counterpart in the reference. */
