@@ -73,8 +73,16 @@ void Stage::release() {
 cudaError_t Stage::upload(int device, int n, void* const* dst, const void* const* src, const int64_t* bytes,
                           cudaStream_t st) {
     std::lock_guard<std::mutex> lock(mutex_);
-    cudaError_t e = prepare();
-    if (e != cudaSuccess) return e;
+    if (prepare() != cudaSuccess) {
+        // no pinned memory to be had: the driver's own staging, which reads the arrays before it returns
+        (void)cudaGetLastError();
+        for (int i = 0; i < n; i++) {
+            if (bytes[i] == 0) continue;
+            const cudaError_t e = cudaMemcpyAsync(dst[i], src[i], (size_t)bytes[i], cudaMemcpyHostToDevice, st);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaStreamSynchronize(st);
+    }
     int64_t total = 0;
     for (int i = 0; i < n; i++) total += (bytes[i] + kChunk - 1) / kChunk;
     std::atomic<int64_t> next{0};
@@ -104,8 +112,12 @@ cudaError_t Stage::upload(int device, int n, void* const* dst, const void* const
 
 cudaError_t Stage::download(int device, void* dst, const void* src, int64_t bytes, cudaStream_t st) {
     std::lock_guard<std::mutex> lock(mutex_);
-    cudaError_t e = prepare();
-    if (e != cudaSuccess) return e;
+    cudaError_t e;
+    if (prepare() != cudaSuccess) {
+        (void)cudaGetLastError();
+        e = bytes ? cudaMemcpyAsync(dst, src, (size_t)bytes, cudaMemcpyDeviceToHost, st) : cudaSuccess;
+        return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+    }
     // one thread waits for the work before the copies
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
     const int64_t total = (bytes + kChunk - 1) / kChunk;
