@@ -358,7 +358,9 @@ constexpr uint32_t kOsAggregate = 1u << 30;
 constexpr uint32_t kOsInclusive = 2u << 30;
 constexpr uint32_t kOsCount = (1u << 30) - 1u;
 constexpr long long kOsSpinCycles = 200000000LL;  // ~0.1 s at 2 GHz
-constexpr int kOsWindow = 16;                    // look-back words loaded together
+// look-back words loaded together: 16M keys 122 us per pass with 4, 125 with 8, 130 with 16, 143
+// with 32; 4M 38.8 / 39.3 / 41.8 / -
+constexpr int kOsWindow = 4;
 
 __device__ __forceinline__ uint32_t ld_relaxed_gpu(const uint32_t* p) {
     uint32_t v;
@@ -428,11 +430,11 @@ __device__ __forceinline__ uint32_t digit_rank(bool valid, uint32_t d, uint32_t*
 }
 
 // What bounds a pass: the instructions of the ranking and the look-back, at few warps per
-// scheduler (43 KB of shared memory and 80 registers: three blocks per SM; four spill), and with
+// scheduler (43 KB of shared memory and 80 registers: three blocks per SM; four at 64 registers are as fast), and with
 // a handful of tiles their latency.  Loads all issued before the first key is ranked, votes and
 // pipelined shared-memory additions in place of match.any between warp barriers, 32-bit bounds,
-// and a window of aggregates added whole: per pass 12.7 -> 7.3 us for 4096 keys, 17.2 -> 9.2
-// for 200k, 33 -> 26 for 2M, 60 -> 42 for 4M, 190 -> 128 for 16M.
+// and a window of aggregates added whole: per pass 12.7 -> 7.3 us for 4096 keys, 17.2 -> 9.1
+// for 200k, 33 -> 25 for 2M, 60 -> 39 for 4M, 190 -> 122 for 16M.
 __global__ void __launch_bounds__(256, 3) k_os_scatter(const uint32_t* __restrict__ keys_in,
                                                        const int32_t* __restrict__ vals_in,
                                                        uint32_t* __restrict__ keys_out, int32_t* __restrict__ vals_out,
@@ -545,7 +547,7 @@ __global__ void __launch_bounds__(256, 3) k_os_scatter(const uint32_t* __restric
                 add += v[i];
             }
             if ((every & kOsAggregate) && !(any & kOsInclusive)) {
-                // aggregates throughout: sixteen states of 2^30 vanish from the sum
+                // aggregates throughout: their states, 2^30 each, vanish from the sum
                 static_assert((uint64_t)kOsWindow * kOsAggregate % (uint64_t(1) << 32) == 0, "states vanish");
                 excl += add;
                 k -= kOsWindow;
