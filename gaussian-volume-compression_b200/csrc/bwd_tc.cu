@@ -515,15 +515,19 @@ __global__ void __launch_bounds__(kBRows + 64, 4) k_backward_cta(
 // 262k 1.45 / 1.30, 524k 1.58 / 1.56, 1M 1.88 / 2.04.
 static bool dense_samples(const BwdArgs& a) { return a.S >= a.P; }
 
-// The masks of a log whose forward wrote none: one CTA per block, one candidate per
-// thread and step.  (Tested by the producer warp instead, candidate after candidate for every
+// The masks of a log whose forward wrote none, or of Gaussians that were handed in anew: one CTA
+// per block, one candidate per thread and step.  (Tested by the producer warp instead, candidate after candidate for every
 // group, they held up the kernel: 500k x 1.5M 2.77 against 2.18 ms and 0.1 ms here.)
 __global__ void __launch_bounds__(128) k_log_masks(const uint2* __restrict__ cdesc, const uint2* __restrict__ bdesc,
                                                    const float4* __restrict__ bboxes,
                                                    const GaussRec* __restrict__ recs, const int32_t* __restrict__ clog,
-                                                   const int32_t* __restrict__ cend, bool window,
-                                                   uint8_t* __restrict__ cmask) {
+                                                   int32_t* __restrict__ cend, const int* __restrict__ moved,
+                                                   bool window, uint8_t* __restrict__ cmask) {
     const int64_t blk = blockIdx.x;
+    if (moved && *moved) {
+        if (threadIdx.x < kBGroups) cend[blk * kBGroups + threadIdx.x] = -1;
+        return;
+    }
     const uint2 cd = cdesc[blk], bd = bdesc[blk];
     const int cng = (int)(cd.y >> 24), ng = (int)(bd.y >> 24);
     const int n = cend[blk * kBGroups + cng - 1];
@@ -543,10 +547,10 @@ __global__ void __launch_bounds__(128) k_log_masks(const uint2* __restrict__ cde
     }
 }
 
-cudaError_t launch_log_masks(const BwdArgs& a, uint8_t* cmask, cudaStream_t st) {
+cudaError_t launch_log_masks(const BwdArgs& a, uint8_t* cmask, int32_t* cend, const int* moved, cudaStream_t st) {
     if (a.S <= 0) return cudaSuccess;
     k_log_masks<<<(unsigned)((a.S + kBRows - 1) / kBRows), 128, 0, st>>>(a.cdesc, a.bdesc, a.bboxes, a.recs, a.clog,
-                                                                         a.cend, dense_samples(a), cmask);
+                                                                         cend, moved, dense_samples(a), cmask);
     gvc::note_launch();
     return cudaGetLastError();
 }

@@ -253,7 +253,7 @@ void gvc_ctx_destroy(gvc_ctx* ctx) {
     DevBuf* bufs[] = {&c->s_sorted, &c->fwd_sorted, &c->blk_desc, &c->blk_boxes, &c->blk_desc_c, &c->blk_boxes_c,
                       &c->b_rows, &c->b_boxes, &c->gtree, &c->s_grad, &c->s_gyz, &c->s_ok, &c->grec, &c->gtmp,
                       &c->knn_points, &c->ts_points, &c->ts_words, &c->cell_tree, &c->cell_recs, &c->clog, &c->cmask,
-                      &c->cend, &c->scratch.gacc, &c->scratch.tmp_boxes};
+                      &c->cend, &c->moved, &c->scratch.gacc, &c->scratch.tmp_boxes};
     for (DevBuf* b : bufs) b->release();
     c->scratch.stage.release();
     if (c->d_status) cudaFree(c->d_status);
@@ -349,15 +349,15 @@ static bool tensor_core_backward(const gvc_ctx* ctx) {
 
 // Morton order of the Gaussians' AABBs, their records in that order and the tree over them:
 // the LBVH for the tensor-core kernels, else the wide tree (new_order false: the order of the
-// last forward still holds).
+// last forward still holds).  `moved`: as launch_gather_recs.
 static int prepare_gaussians(gvc_ctx* ctx, int64_t P, const float* means, const float* values, const float* weights,
-                             const float* conics, bool new_order, bool linked, cudaStream_t st) {
+                             const float* conics, bool new_order, bool linked, int* moved, cudaStream_t st) {
     const float4* boxes = ctx->gtmp.as<float4>();
     if (new_order) GVC_CUDA(morton_sort_boxes(ctx->gsort, P, boxes, st), "Gaussian order");
     GVC_CUDA(ctx->grec.ensure(sizeof(GaussRec) * P), "alloc records");
     GVC_CUDA(ctx->gtree.ensure(sizeof(float4) * 2 * wide_tree_size(P).boxes), "alloc Gaussian tree");
     GVC_CUDA(launch_gather_recs(P, ctx->gsort.perm.as<int32_t>(), means, values, weights, conics, boxes,
-                                ctx->grec.as<GaussRec>(), ctx->gtree.as<float4>(), !linked, st),
+                                ctx->grec.as<GaussRec>(), ctx->gtree.as<float4>(), !linked, moved, st),
              "gather records");
     ctx->glinks_ready = false;
     if (linked) {
@@ -466,7 +466,7 @@ int gvc_rasterize_gaussians(gvc_ctx* ctx, int64_t P, const float* means3D, const
     // with the tensor-core kernels selected, the forward walks the LBVH by the coarser groups
     const bool tc_bwd = tensor_core_backward(ctx);
     const bool linked = tc_bwd || ctx->eval_path == 1;
-    int rc = prepare_gaussians(ctx, P, means3D, values, weights, conics, true, linked, st);
+    int rc = prepare_gaussians(ctx, P, means3D, values, weights, conics, true, linked, nullptr, st);
     if (rc == GVC_OK && linked) rc = ensure_coarse_groups(ctx, st);
     if (rc != GVC_OK) return rc;
     tm.mark();
@@ -623,9 +623,19 @@ int gvc_rasterize_gaussians_backward(gvc_ctx* ctx, int64_t P, const float* means
                                          ctx->s_gyz.as<float>(), ctx->s_ok.as<uint8_t>(), st),
                      "sample grads");
             tm.mark();
+            // the forward's candidate log serves the Gaussians whose boxes it holds: the forward's
+            // own arrays, or others with the same boxes (copies), which the device finds out
+            const bool use_log = have_order && ctx->clog_ready;
+            int* moved = nullptr;
             if (!same_gauss) {
                 if (!have_order) ctx->gauss_ready = false;  // the order below is not the forward's
-                const int rc = prepare_gaussians(ctx, P, means3D, values, weights, conics, !have_order, true, st);
+                if (use_log) {
+                    GVC_CUDA(ctx->moved.ensure(sizeof(int)), "alloc flag");
+                    moved = ctx->moved.as<int>();
+                    GVC_CUDA(cudaMemsetAsync(moved, 0, sizeof(int), st), "clear flag");
+                }
+                const int rc =
+                    prepare_gaussians(ctx, P, means3D, values, weights, conics, !have_order, true, moved, st);
                 if (rc != GVC_OK) return rc;
             } else if (!ctx->glinks_ready) {
                 GVC_CUDA(lbvh_hierarchy(ctx->gsort, P, ctx->gsort.keys.as<uint32_t>(), ctx->gtree.as<float4>(), st),
@@ -642,15 +652,15 @@ int gvc_rasterize_gaussians_backward(gvc_ctx* ctx, int64_t P, const float* means
             ba.s_ok = ctx->s_ok.as<uint8_t>();
             ba.nodes = ctx->gsort.nodes.as<BvhNode>();
             ba.recs = ctx->grec.as<GaussRec>();
-            // the forward's candidate log, when it belongs to these Gaussians and samples,
-            // replaces the backward's own walk of the tree
-            if (have_order && ctx->clog_ready) {
+            // it replaces the backward's own walk of the tree
+            if (use_log) {
                 ba.clog = ctx->clog.as<int32_t>();
                 ba.cmask = ctx->cmask.as<uint8_t>();
                 ba.cend = ctx->cend.as<int32_t>();
                 ba.cdesc = ctx->blk_desc_c.as<uint2>();
                 if (!ctx->clog_masks || !same_gauss)
-                    GVC_CUDA(launch_log_masks(ba, ctx->cmask.as<uint8_t>(), st), "log masks");
+                    GVC_CUDA(launch_log_masks(ba, ctx->cmask.as<uint8_t>(), ctx->cend.as<int32_t>(), moved, st),
+                             "log masks");
                 ctx->clog_masks = true;
             }
             const int tk = timer_begin(ctx, st, 1);

@@ -159,14 +159,20 @@ __device__ __forceinline__ bool window_covers(const GaussRec& r) {
     return q <= 27.9f;
 }
 
+__device__ __forceinline__ bool same_bits(float4 a, float4 b) {
+    return __float_as_uint(a.x) == __float_as_uint(b.x) && __float_as_uint(a.y) == __float_as_uint(b.y) &&
+           __float_as_uint(a.z) == __float_as_uint(b.z);
+}
+
 // One thread per Gaussian in Morton order: its record, its box as a leaf of the wide tree,
-// and (eight neighbouring lanes together) the box of its level-1 node.
+// and (eight neighbouring lanes together) the box of its level-1 node.  Given `moved`, it is
+// set where a leaf that the tree held before is replaced by another box.
 __global__ void __launch_bounds__(256) k_gather_recs(int64_t P, const int32_t* __restrict__ perm,
                                                      const float* __restrict__ means, const float* __restrict__ values,
                                                      const float* __restrict__ weights,
                                                      const float* __restrict__ conics, const float4* __restrict__ boxes,
                                                      GaussRec* __restrict__ recs, float4* __restrict__ leaf,
-                                                     float4* __restrict__ level1) {
+                                                     float4* __restrict__ level1, int* __restrict__ moved) {
     const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     Box6 b = empty_box();
     if (g < P) {
@@ -180,6 +186,7 @@ __global__ void __launch_bounds__(256) k_gather_recs(int64_t P, const int32_t* _
         r.r2.w = window_covers(r) ? 1.f : 0.f;
         recs[g] = r;
         b = Box6{r.r3.x, r.r3.y, r.r3.z, r.r4.x, r.r4.y, r.r4.z};
+        if (moved && !(same_bits(leaf[2 * g], r.r3) && same_bits(leaf[2 * g + 1], r.r4))) *moved = 1;
         store_box(leaf, g, b);
     }
     grow(b, shfl_xor_box(b, 1));
@@ -255,11 +262,11 @@ cudaError_t launch_preprocess(int64_t P, const float* means, const float* scales
 
 cudaError_t launch_gather_recs(int64_t P, const int32_t* perm, const float* means, const float* values,
                                const float* weights, const float* conics, const float4* boxes, GaussRec* recs,
-                               float4* tree_boxes, bool levels, cudaStream_t st) {
+                               float4* tree_boxes, bool levels, int* moved, cudaStream_t st) {
     if (P <= 0) return cudaSuccess;
     const WideTreeSize z = wide_tree_size(P);
     k_gather_recs<<<nb256(P), 256, 0, st>>>(P, perm, means, values, weights, conics, boxes, recs, tree_boxes,
-                                            tree_boxes + 2 * z.n[0]); gvc::note_launch();
+                                            tree_boxes + 2 * z.n[0], moved); gvc::note_launch();
     if (!levels) return cudaGetLastError();
     return launch_wide_levels(z, tree_boxes, st);
 }

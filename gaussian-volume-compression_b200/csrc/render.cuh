@@ -144,7 +144,9 @@ cudaError_t launch_backward_gauss(const BwdArgs& a, const WideTree& tree, const 
 
 // bwd_tc.cu: reduction over samples on tcgen05, one CTA per 128 samples
 cudaError_t launch_backward_tc(const BwdArgs& a, cudaStream_t st);
-cudaError_t launch_log_masks(const BwdArgs& a, uint8_t* cmask, cudaStream_t st);
+// `moved` (device, or null) nonzero: the log is of other boxes than `recs`', and every block's is
+// struck out instead.
+cudaError_t launch_log_masks(const BwdArgs& a, uint8_t* cmask, int32_t* cend, const int* moved, cudaStream_t st);
 cudaError_t launch_finalize(int64_t P, const float* gacc, const float* scales, const float* rots, const float* conics,
                             float sm, int ref_compat, float* dmeans, float* dscales, float* drots, float* dvalues,
                             float* dweights, cudaStream_t st);
@@ -153,10 +155,10 @@ cudaError_t launch_finalize(int64_t P, const float* gacc, const float* scales, c
 cudaError_t launch_preprocess(int64_t P, const float* means, const float* scales, const float* rots,
                               const float* weights, float sm, float* conics_out, float4* boxes_out, cudaStream_t st);
 // Records in Morton order, and their wide tree at `tree_boxes` (levels false: its two lowest
-// levels only).
+// levels only).  `moved` (device, or null): set if a leaf differs from what tree_boxes held.
 cudaError_t launch_gather_recs(int64_t P, const int32_t* perm, const float* means, const float* values,
                                const float* weights, const float* conics, const float4* boxes, GaussRec* recs,
-                               float4* tree_boxes, bool levels, cudaStream_t st);
+                               float4* tree_boxes, bool levels, int* moved, cudaStream_t st);
 // Sorted sample slots: (x, y, z, bits of the caller's index or -1).
 cudaError_t launch_sample_slots(int64_t S, int64_t n_slots, const float* samples, const int32_t* perm,
                                 float4* s_sorted, cudaStream_t st);
