@@ -6,8 +6,9 @@
 // chunks of 16: 16 x, 16 y, 16 z, 16 gx, 16 gyz (320 bytes), so that a lane reads two
 // neighbouring rows of each field as one float2.  The same kernel reduces the boxes of the
 // chunks and of runs of 8 chunks, the lower levels of a wide tree (wide_tree.cuh).  A row
-// without a gradient (W below the cutoff, or an upstream gradient of zero) adds nothing to any sum
-// and is left out of the boxes.
+// without a gradient (W below the cutoff, an upstream gradient of zero, or a sample that is no point)
+// adds nothing to any sum and is left out of the boxes; its coordinates are stored as zeros, since
+// a zero times a NaN or an infinity would not be one.
 //
 // Sums.  A warp walks that tree with its Gaussian's AABB, 32 children per step:
 // neighbouring children lie in neighbouring memory, and five levels cover 16M samples,
@@ -66,7 +67,7 @@ __global__ void __launch_bounds__(kRowThreads) k_backward_rows(
         y[k] = sp[k].y;
         z[k] = sp[k].z;
         gx[k] = gyz[k] = 0.f;
-        if (o >= 0) {
+        if (o >= 0 && x[k] == x[k]) {
             const float2 ow = out_sorted ? out_sorted[r0 + k] : make_float2(out_cells[o], out_weights[o]);
             if (ow.y > kWeightCutoff) {
                 const float g = gout[o];
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(kRowThreads) k_backward_rows(
             }
         }
         if (!(gx[k] == 0.f && gyz[k] == 0.f)) grow(b, Box6{x[k], y[k], z[k], x[k], y[k], z[k]});
+        else x[k] = y[k] = z[k] = 0.f;
     }
     float4* dst = reinterpret_cast<float4*>(rows + (r0 / kChunkRows) * kChunkFloats) + (lane & 3);
     dst[0] = make_float4(x[0], x[1], x[2], x[3]);

@@ -70,12 +70,15 @@ struct BoxSrc {
 };
 struct PointSrc {
     const float* pts;  // [n][3]
+    // an infinite coordinate counts as none (NaN): in the bounds it would leave every point with
+    // key 0, in no order at all
+    static __device__ __forceinline__ float finite(float c) { return isfinite(c) ? c : NAN; }
     __device__ __forceinline__ void centroid(int64_t i, float c[3]) const {
         // (p + p) * 0.5f == p exactly for finite p, as for a degenerate box
         float x = pts[3 * i], y = pts[3 * i + 1], z = pts[3 * i + 2];
-        c[0] = __fmul_rn(__fadd_rn(x, x), 0.5f);
-        c[1] = __fmul_rn(__fadd_rn(y, y), 0.5f);
-        c[2] = __fmul_rn(__fadd_rn(z, z), 0.5f);
+        c[0] = finite(__fmul_rn(__fadd_rn(x, x), 0.5f));
+        c[1] = finite(__fmul_rn(__fadd_rn(y, y), 0.5f));
+        c[2] = finite(__fmul_rn(__fadd_rn(z, z), 0.5f));
     }
 };
 

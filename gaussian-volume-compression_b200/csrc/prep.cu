@@ -196,7 +196,10 @@ __global__ void __launch_bounds__(256) k_gather_recs(int64_t P, const int32_t* _
 }
 
 // Sorted sample slots: (x, y, z, caller index as int bits); padding slots carry NaN
-// coordinates and index -1.
+// coordinates and index -1.  So does, but for its index, a sample with any coordinate that is
+// not finite: it contributes to nothing (its distance from any mean has no power in the
+// window), and NaN keeps it out of every box, where an infinity would stretch a group's box
+// and centre over the ordinary samples beside it.
 __global__ void __launch_bounds__(256) k_sample_slots(int64_t S, int64_t n_slots, const float* __restrict__ samples,
                                                       const int32_t* __restrict__ perm,
                                                       float4* __restrict__ s_sorted) {
@@ -209,6 +212,7 @@ __global__ void __launch_bounds__(256) k_sample_slots(int64_t S, int64_t n_slots
         x = samples[3 * (int64_t)o];
         y = samples[3 * (int64_t)o + 1];
         z = samples[3 * (int64_t)o + 2];
+        if (!(isfinite(x) && isfinite(y) && isfinite(z))) x = y = z = NAN;
     }
     s_sorted[i] = make_float4(x, y, z, __int_as_float(o));
 }
@@ -218,7 +222,8 @@ __global__ void __launch_bounds__(256) k_sample_slots(int64_t S, int64_t n_slots
 // Backward sample records in sorted order: (x, y, z, gx) with gx = dL/dout / W, gyz =
 // -dL/dout * out / W + dL/dW (backward.cu:252-298 folds the same factors per pair), and
 // ok = W > 0.01.  Samples below the cutoff get gx = gyz = 0, so their pairs add exactly
-// nothing; tile padding gets finite coordinates (0) and zero gradients for the same reason.
+// nothing; padding and samples that are no points get finite coordinates (0) and zero gradients for
+// the same reason.
 // With out_sorted (the forward's (out, W) per sorted slot) only dL/dout and dL/dW are
 // gathered from the caller's order.
 __global__ void __launch_bounds__(256) k_sample_grads(int64_t n_slots, const float4* __restrict__ s_sorted,
@@ -235,7 +240,7 @@ __global__ void __launch_bounds__(256) k_sample_grads(int64_t n_slots, const flo
     float gx = 0.f, gyz = 0.f;
     uint8_t ok = 0;
     float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (o >= 0) {
+    if (o >= 0 && sp.x == sp.x) {
         const float2 ow = out_sorted ? out_sorted[i] : make_float2(0.f, out_weights[o]);
         const float W = ow.y;
         if (W > kWeightCutoff) {

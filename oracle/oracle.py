@@ -170,8 +170,9 @@ def lbvh_build(boxes):
 
 
 def morton30_points(pts):
-    """Declared 30-bit Morton keys of points over their own bounds, and the stable order."""
-    pts = _c(pts, np.float32)
+    """Declared 30-bit Morton keys of points over their own bounds (an infinite coordinate counts as
+    none), and the stable order."""
+    pts = _c(np.where(np.isfinite(pts), pts, np.nan), np.float32)
     boxes = np.concatenate([pts, pts], axis=1)
     lo = np.zeros(3, np.float32); hi = np.zeros(3, np.float32)
     lib().orc_centroid_bounds(pts.shape[0], _p(boxes), _p(lo), _p(hi))
