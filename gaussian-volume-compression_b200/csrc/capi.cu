@@ -504,8 +504,9 @@ int gvc_rasterize_gaussians(gvc_ctx* ctx, int64_t P, const float* means3D, const
             ctx->cend.release();
         }
     }
-    // (out, W) in sorted order as well, for the backward's rows
-    if (S > 0) {
+    // (out, W) in sorted order as well, for the backward's rows (FP32 only: after a tensor-core
+    // evaluation the backward has always read the caller's arrays, changed or not)
+    if (S > 0 && ctx->eval_path == 0) {
         if (ctx->fwd_sorted.ensure(sizeof(float2) * ctx->n_tiles * kTile) == cudaSuccess) {
             fa.out_sorted = ctx->fwd_sorted.as<float2>();
         } else {

@@ -260,8 +260,7 @@ __global__ void __launch_bounds__(192, kMinBlocks)
     k_forward_tc(const float4* __restrict__ s_sorted, int64_t S, const uint2* __restrict__ bdesc,
                  const float4* __restrict__ bboxes, const BvhNode* __restrict__ nodes,
                  const GaussRec* __restrict__ recs, float* __restrict__ out_cells, float* __restrict__ out_weights,
-                 float2* __restrict__ out_sorted, int32_t* __restrict__ clog, int32_t* __restrict__ cend, int* status,
-                 unsigned long long* stats) {
+                 int32_t* __restrict__ clog, int32_t* __restrict__ cend, int* status, unsigned long long* stats) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     FwdTcSmem& sm = *reinterpret_cast<FwdTcSmem*>(
         smem_raw + ((1024 - (static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw)) & 1023)) & 1023));
@@ -456,7 +455,6 @@ __global__ void __launch_bounds__(192, kMinBlocks)
             }
             out_cells[orig] = o;
             out_weights[orig] = ww;
-            if (out_sorted) out_sorted[row] = make_float2(o, ww);
         }
         if (COUNT) {
             unsigned long long a = (unsigned long long)ncand, b = (unsigned long long)ncontrib;
@@ -484,7 +482,7 @@ static cudaError_t launch_fwd_tc_impl(const FwdArgs& a, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     const unsigned nb = (unsigned)((a.S + kBlockRows - 1) / kBlockRows);
     k_forward_tc<COUNT><<<nb, 192, smem, st>>>(a.s_sorted, a.S, a.bdesc, a.bboxes, a.nodes, a.recs, a.out_cells,
-                                               a.out_weights, a.out_sorted, a.clog, a.cend, a.status, a.stats);
+                                               a.out_weights, a.clog, a.cend, a.status, a.stats);
     gvc::note_launch();
     return cudaGetLastError();
 }

@@ -125,7 +125,7 @@ struct gvc_ctx {
     bool clog_ready = false;
     bool clog_masks = false;  // its masks are written
     gvc::DevBuf moved;        // whether a backward's Gaussians have other boxes than the log's
-    // (out, W) per sorted slot as the last forward wrote them, and the
+    // (out, W) per sorted slot as the last FP32 forward wrote them, and the
     // output arrays it wrote them to (the backward uses the copy for those arrays only)
     gvc::DevBuf fwd_sorted;
     const float* fwd_out_cells = nullptr;

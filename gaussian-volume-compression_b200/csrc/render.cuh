@@ -50,7 +50,7 @@ struct FwdArgs {
     const GaussRec* recs;  // the same order
     float* out_cells;
     float* out_weights;
-    float2* out_sorted;    // (out, W) per sorted slot, read by the backward's rows; or null
+    float2* out_sorted;    // (out, W) per sorted slot, read by the backward's rows (FP32 only); or null
     int32_t* clog;         // candidate log, or null
     uint8_t* cmask;        // its masks (FP32 forward)
     int32_t* cend;

@@ -130,7 +130,11 @@ int gvc_rasterize_gaussians(gvc_ctx* ctx, int64_t P, const float* means3D, const
 /* Replaces RasterizeGaussiansBackwardCUDAWrapper / RasterizeGaussiansBackwardCUDA
    (diff-gaussian-rasterization/ext.cu:107-147, rasterize_points.cu:75-137).
    Outputs (caller-allocated, overwritten): dmeans [P,3], dscales [P,3], drots [P,4],
-   dvalues [P], dweights [P]. */
+   dvalues [P], dweights [P].
+   Handed the very arrays of the context's last forward (its Gaussians and conics; with
+   GVC_OPT_EVAL_PATH 0 its out_cells and out_weights), it uses what that forward derived
+   from them: change them in place only before a forward.  Others, copies among them, are read
+   as they are. */
 int gvc_rasterize_gaussians_backward(gvc_ctx* ctx, int64_t P, const float* means3D, const float* scales,
                                      const float* rotations, const float* conics, const float* values,
                                      const float* weights, const float* out_cells, const float* out_weights,
