@@ -37,7 +37,10 @@ int fail(gvc_ctx* c, int code, const char* msg) {
     return code;
 }
 
+// The error is reported here: it must not stay behind as the thread's last one, where the next
+// launch's check, this library's or another's, takes it for its own.
 int cuda_fail(gvc_ctx* c, cudaError_t e, const char* where) {
+    (void)cudaGetLastError();
     if (c) {
         c->err = std::string(where) + ": " + cudaGetErrorString(e);
     }
