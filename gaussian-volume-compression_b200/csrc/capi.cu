@@ -455,7 +455,11 @@ int gvc_rasterize_gaussians(gvc_ctx* ctx, int64_t P, const float* means3D, const
     }
     if (!means3D || !scales || !rotations || !values || !weights || !conics)
         return fail(ctx, GVC_ERR_ARG, "null Gaussian parameter pointer");
-    // this call rewrites the AABBs, records and sorted outputs: valid again only once it ends
+    // this call rewrites the order, AABBs, records, log and sorted outputs: valid again only once
+    // it ends (left by a call that fails, an order of more Gaussians would index past the last
+    // forward's)
+    ctx->gauss_ready = false;
+    ctx->clog_ready = false;
     ctx->fwd_recs_ready = false;
     ctx->fwd_sorted_ready = false;
     DebugTimer tm(debug != 0, st);

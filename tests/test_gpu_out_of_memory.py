@@ -1,12 +1,14 @@
 """A forward that finds no device memory half way: it reports GVC_ERR_CUDA, once, and the context
 works on."""
 import ctypes
+import gc
 
+import numpy as np
 import pytest
 import torch
 
 import gvc_native
-from test_gpu_rasterizer import T
+from test_gpu_rasterizer import T, assert_grads_close, oracle_backward
 
 pytestmark = pytest.mark.gpu
 
@@ -47,6 +49,7 @@ class Calls:
         n = 4_000_000
         t = [torch.rand((n, k), device=self.dev) * 0.01 + 0.01 for k in (3, 3, 4, 1, 1)]
         outs = self.outputs(n)
+        gc.collect()  # contexts of earlier tests: what they free later would be found by the call
         torch.cuda.synchronize()
         torch.cuda.empty_cache()
         # the boxes (128 MB) and the sort's arrays fit, the records (320 MB) do not
@@ -66,3 +69,21 @@ def test_forward_after_a_failed_one(cuda, orc, mode):
     again = c.forward(c.ta)
     c.ctx.sync_status(c.st.value)
     assert all(torch.equal(x, y) for x, y in zip(again, c.outs))
+
+
+@pytest.mark.parametrize("mode", MODES)
+def test_backward_after_a_failed_forward(cuda, orc, mode):
+    """Of the forward before it: what the failed one left (the order of more Gaussians) is not used."""
+    c = Calls(cuda, orc, mode)
+    rng = np.random.default_rng(91)
+    up = [rng.normal(size=c.S).astype(np.float32) for _ in range(2)]
+    d_up = [T(u, cuda) for u in up]
+    means, scales, rots, values, weights = c.ta
+    out, outw, conics = c.outs
+    grads = [torch.empty((3000, k), device=cuda) for k in (3, 3, 4, 1, 1)]
+    c.ctx.call("gvc_rasterize_gaussians_backward", 3000, p(means), p(scales), p(rots), p(conics), p(values),
+               p(weights), p(out), p(outw), ONE, None, BG, p(d_up[0]), p(d_up[1]), 0, 0, *[p(g) for g in grads], c.st)
+    c.ctx.sync_status(c.st.value)
+    ref = oracle_backward(orc, tuple(c.a) + (c.samples,), out.cpu().numpy(), outw.cpu().numpy(),
+                          conics.cpu().numpy().reshape(-1, 6), *up)
+    assert_grads_close([g.cpu().numpy() for g in grads], ref)
