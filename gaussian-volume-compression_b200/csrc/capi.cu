@@ -735,7 +735,7 @@ static int locate(gvc_ctx* ctx, LocateArgs& la, int64_t C, const float* pts, con
         la.cperm = ctx->cells.perm.as<int32_t>();
         la.tree_boxes = ctx->cell_tree.as<float4>();
         la.recs = recs;
-        GVC_CUDA(launch_cell_tree(C, la.cperm, boxes, pts, conn4, recs, ctx->cell_tree.as<float4>(), st), "cell tree");
+        GVC_CUDA(launch_cell_tree(C, ctx->cells.perm.as<int32_t>(), boxes, pts, conn4, recs, ctx->cell_tree.as<float4>(), st), "cell tree");
     }
     GVC_CUDA(launch_locate(la, st), "locate samples");
     return GVC_OK;
@@ -982,6 +982,19 @@ int gvc_debug_tc_gemm(gvc_ctx* ctx, const void* A, const void* B, int N, float* 
 int gvc_debug_wait_timeout(gvc_ctx* ctx, void* stream) {
     if (!ctx) return GVC_ERR_ARG;
     GVC_CUDA(launch_wait_timeout_test(ctx->d_status, (cudaStream_t)stream), "wait timeout");
+    return GVC_OK;
+}
+
+int gvc_debug_sort_timeout(gvc_ctx* ctx, int64_t n, const float* pts, int32_t* perm, float* slots, void* stream) {
+    if (!ctx) return GVC_ERR_ARG;
+    if (n <= kRsTile || n > (1 << 20)) return fail(ctx, GVC_ERR_ARG, "n out of range");
+    if (!pts || !perm || !slots) return fail(ctx, GVC_ERR_ARG, "null pointer");
+    cudaStream_t st = (cudaStream_t)stream;
+    Lbvh& L = scratch_of(ctx)->dbg;
+    L.n = 0;
+    GVC_CUDA(morton_sort_points_withheld(L, n, pts, st), "withheld sort");
+    GVC_CUDA(launch_sample_slots(n, n, pts, L.perm.as<int32_t>(), reinterpret_cast<float4*>(slots), st), "slots");
+    GVC_CUDA(cudaMemcpyAsync(perm, L.perm.ptr, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, st), "copy perm");
     return GVC_OK;
 }
 

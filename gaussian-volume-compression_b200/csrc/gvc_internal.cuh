@@ -24,6 +24,16 @@ void note_launch(int n = 1);
 constexpr int kStatusStackOverflow = 1;
 constexpr int kStatusTimeout = 2;  // a bounded wait gave up (mbarrier, radix-sort look-back)
 
+// Entry i of a sorted order of n elements, for the kernel that reads the order first.  Where a
+// look-back of the sort gave up (kStatusTimeout), slots of the order may never have been written:
+// what is no index becomes 0, in the order itself too, for the kernels that read it later.
+__device__ __forceinline__ int32_t order_at(int32_t* __restrict__ order, int64_t i, int64_t n) {
+    const int32_t o = order[i];
+    if ((uint32_t)o < (uint32_t)n) return o;
+    order[i] = 0;
+    return 0;
+}
+
 // Gaussian evaluation record, one per Gaussian in Morton order: 80 bytes.
 //   r0 = (mu.x, mu.y, mu.z, w)
 //   r1 = (c0, c1, c2, c3)  -- conic xx, xy, xz, yy as written to the conics output

@@ -32,10 +32,10 @@ namespace {
 constexpr int kKnnStack = 64;  // the tree's depth is bounded by the 62 key + index bits
 
 __global__ void __launch_bounds__(256) k_knn_points(int64_t n, const float* __restrict__ pts,
-                                                    const int32_t* __restrict__ perm, float4* __restrict__ sorted) {
+                                                    int32_t* __restrict__ perm, float4* __restrict__ sorted) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int64_t o = perm[i];
+    const int64_t o = order_at(perm, i, n);
     sorted[i] = make_float4(pts[3 * o], pts[3 * o + 1], pts[3 * o + 2], __int_as_float((int)o));
 }
 
@@ -124,7 +124,7 @@ inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
 
-cudaError_t launch_knn_points(int64_t n, const float* pts, const int32_t* perm, float4* sorted, cudaStream_t st) {
+cudaError_t launch_knn_points(int64_t n, const float* pts, int32_t* perm, float4* sorted, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     k_knn_points<<<nblk(n, 256), 256, 0, st>>>(n, pts, perm, sorted); gvc::note_launch();
     return cudaGetLastError();

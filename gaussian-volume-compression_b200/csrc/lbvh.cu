@@ -353,7 +353,8 @@ __global__ void __launch_bounds__(256) k_rs_scatter(const uint32_t* __restrict__
 // A word packs a 2-bit state (not ready / aggregate / inclusive) with a 30-bit count, so
 // n < 2^30.  A tile only waits on tiles with smaller tickets, whose blocks are already
 // running and wait only on tiles before their own, so the look-back ends; its spin is
-// bounded all the same (kStatusTimeout, results invalid).  Same stable order as the
+// bounded all the same (kStatusTimeout; the order is invalid then, and may hold what its
+// buffers held before: order_at).  Same stable order as the
 // three-kernel passes: tile t holds keys [t * kRsTile, (t + 1) * kRsTile) of the pass's
 // input whatever block takes ticket t.
 // ----------------------------------------------------------------------------------
@@ -594,7 +595,8 @@ __global__ void __launch_bounds__(256, 3) k_os_scatter(const uint32_t* __restric
     for (int sp = threadIdx.x; sp < cnt; sp += 256) {
         const uint32_t key = skey[sp];
         const uint32_t pos = gpos[(key >> shift) & 255u] + (uint32_t)sp;
-        // pos < n always (a timed-out look-back only undercounts); the test costs nothing
+        // false only after a look-back gave up: the keys of a pass that lost some to the slots it
+        // left unwritten no longer match the digit counts taken before the first pass
         if (pos < (uint32_t)n) {
             keys_out[pos] = key;
             vals_out[pos] = sval[sp];
@@ -607,8 +609,9 @@ __global__ void __launch_bounds__(256, 3) k_os_scatter(const uint32_t* __restric
 constexpr int kOsHead = 4 * 256 + 64;
 constexpr int kOsBounds = 4 * 256 + 8;
 
-// Passes over L.keys; the words are zeroed and the digit counts filled in.
-static cudaError_t radix_sort_onesweep(Lbvh& L, int64_t n, cudaStream_t st) {
+// Passes over L.keys; the words are zeroed and the digit counts filled in, the tickets start at
+// `withheld` (test hook: the tiles before it never run, and those after wait for them in vain).
+static cudaError_t radix_sort_onesweep(Lbvh& L, int64_t n, int withheld, cudaStream_t st) {
     const int64_t T = (n + kRsTile - 1) / kRsTile;
     cudaError_t e;
     if ((e = L.keys_alt.ensure(LbvhBytes::keys(n))) != cudaSuccess) return e;
@@ -622,7 +625,7 @@ static cudaError_t radix_sort_onesweep(Lbvh& L, int64_t n, cudaStream_t st) {
     int32_t* vin = nullptr;
     int32_t* vout = L.perm_alt.as<int32_t>();
     for (int pass = 0; pass < 4; pass++) {
-        k_os_scatter<<<(unsigned)T, 256, 0, st>>>(kin, vin, kout, vout, n, pass, ghist,
+        k_os_scatter<<<(unsigned)(T - withheld), 256, 0, st>>>(kin, vin, kout, vout, n, pass, ghist,
                                                   look0 + (size_t)pass * 256 * (size_t)T, tickets + pass,
                                                   L.status); gvc::note_launch();
         // ping-pong as in radix_sort_pairs: the result ends in L.keys / L.perm
@@ -664,9 +667,9 @@ static cudaError_t radix_sort_pairs(Lbvh& L, int64_t n, cudaStream_t st) {
 }
 
 __global__ void __launch_bounds__(256) k_gather_u32(int64_t n, const uint32_t* __restrict__ src,
-                                                    const int32_t* __restrict__ perm, uint32_t* __restrict__ dst) {
+                                                    int32_t* __restrict__ perm, uint32_t* __restrict__ dst) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = src[perm[i]];
+    if (i < n) dst[i] = src[order_at(perm, i, n)];
 }
 
 cudaError_t radix_sort_words(Lbvh& L, int64_t n, const uint32_t* const* words, const int* bits, int nwords,
@@ -807,11 +810,11 @@ __global__ void __launch_bounds__(256) k_lbvh_build(int n, const uint32_t* __res
     }
 }
 
-__global__ void __launch_bounds__(256) k_gather_boxes(int64_t n, const int32_t* __restrict__ perm,
+__global__ void __launch_bounds__(256) k_gather_boxes(int64_t n, int32_t* __restrict__ perm,
                                                       const float4* __restrict__ boxes, float4* __restrict__ out) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    int64_t p = perm[i];
+    int64_t p = order_at(perm, i, n);
     out[2 * i] = boxes[2 * p];
     out[2 * i + 1] = boxes[2 * p + 1];
 }
@@ -1013,7 +1016,7 @@ static cudaError_t morton_sort(Lbvh& L, int64_t n, Src src, cudaStream_t st) {
         k_keys<Src, true><<<nbk < 148u * 4u ? nbk : 148u * 4u, 256, 0, st>>>(src, n, bounds, L.keys.as<uint32_t>(),
                                                                              ghist);
         gvc::note_launch();
-        return radix_sort_onesweep(L, n, st);
+        return radix_sort_onesweep(L, n, 0, st);
     }
     k_keys<Src, false><<<nbk < 148u * 8u ? nbk : 148u * 8u, 256, 0, st>>>(src, n, bounds, L.keys.as<uint32_t>(), nullptr);
     gvc::note_launch();
@@ -1026,6 +1029,25 @@ cudaError_t morton_sort_boxes(Lbvh& L, int64_t n, const float4* boxes, cudaStrea
 
 cudaError_t morton_sort_points(Lbvh& L, int64_t n, const float* pts, cudaStream_t st) {
     return morton_sort(L, n, PointSrc{pts}, st);
+}
+
+cudaError_t morton_sort_points_withheld(Lbvh& L, int64_t n, const float* pts, cudaStream_t st) {
+    if (n <= kRsTile || n > (int64_t)kOsCount || !L.status) return cudaErrorInvalidValue;
+    cudaError_t e;
+    if ((e = L.keys.ensure(LbvhBytes::keys(n))) != cudaSuccess) return e;
+    if ((e = L.perm.ensure(LbvhBytes::keys(n))) != cudaSuccess) return e;
+    if ((e = L.perm_alt.ensure(LbvhBytes::keys(n))) != cudaSuccess) return e;
+    if ((e = L.onesweep.ensure(LbvhBytes::onesweep(n))) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(L.onesweep.ptr, 0, LbvhBytes::onesweep(n), st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(L.perm.ptr, 0x7f, LbvhBytes::keys(n), st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(L.perm_alt.ptr, 0x7f, LbvhBytes::keys(n), st)) != cudaSuccess) return e;
+    uint32_t* ghist = L.onesweep.as<uint32_t>();
+    const uint32_t first[4] = {1, 1, 1, 1};
+    if ((e = cudaMemcpyAsync(ghist + 4 * 256, first, sizeof(first), cudaMemcpyHostToDevice, st)) != cudaSuccess) return e;
+    k_bounds<PointSrc><<<8, 256, 0, st>>>(PointSrc{pts}, n, ghist + kOsBounds); gvc::note_launch();
+    k_keys<PointSrc, true><<<8, 256, 0, st>>>(PointSrc{pts}, n, ghist + kOsBounds, L.keys.as<uint32_t>(), ghist);
+    gvc::note_launch();
+    return radix_sort_onesweep(L, n, 1, st);
 }
 
 cudaError_t lbvh_build_boxes(Lbvh& L, int64_t n, const float4* boxes, cudaStream_t st) {

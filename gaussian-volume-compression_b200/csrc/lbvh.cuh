@@ -39,6 +39,10 @@ cudaError_t morton_sort_boxes(Lbvh& L, int64_t n, const float4* boxes, cudaStrea
 // Same for points [n][3].
 cudaError_t morton_sort_points(Lbvh& L, int64_t n, const float* pts, cudaStream_t st);
 
+// Test hook: morton_sort_points (over more than one tile) with the first tile of every pass
+// withheld and an order that held no index, so that each look-back runs out.
+cudaError_t morton_sort_points_withheld(Lbvh& L, int64_t n, const float* pts, cudaStream_t st);
+
 // Common prefix of the keys at i and j of the sorted order, equal keys told apart by position.
 __device__ __forceinline__ int lbvh_delta(const uint32_t* __restrict__ keys, int i, int j) {
     const uint32_t a = keys[i], b = keys[j];

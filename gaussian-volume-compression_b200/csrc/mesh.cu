@@ -555,7 +555,7 @@ struct Locator {
 // 12 or 10 5 % and 8 36 % slower).
 template <bool TETS, class Out>
 __global__ void __launch_bounds__(32, TETS ? 28 : 16)
-    k_locate(int64_t N, int rows, const float* __restrict__ samples, const int32_t* __restrict__ sperm,
+    k_locate(int64_t N, int rows, const float* __restrict__ samples, int32_t* __restrict__ sperm,
              const __grid_constant__ WideTree tree, const __grid_constant__ CellMesh mesh, Out* __restrict__ out,
              int64_t* __restrict__ cell_ids) {
     __shared__ LocateSmem sm;
@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(32, TETS ? 28 : 16)
     int64_t s = 0;
     float x = NAN, y = NAN, z = NAN;
     if (valid) {
-        s = sperm ? sperm[i] : i;
+        s = sperm ? order_at(sperm, i, N) : i;
         x = samples[3 * s];
         y = samples[3 * s + 1];
         z = samples[3 * s + 2];
@@ -676,14 +676,14 @@ __device__ __forceinline__ void tet_planes(const float* a, const float* b, const
 
 // Leaves of the tree in Morton order (levels 0 and 1) and, of tetrahedra, their records.
 template <bool TETS>
-__global__ void __launch_bounds__(256) k_cell_leaves(int64_t C, const int32_t* __restrict__ perm,
+__global__ void __launch_bounds__(256) k_cell_leaves(int64_t C, int32_t* __restrict__ perm,
                                                      const float4* __restrict__ boxes, const float* __restrict__ pts,
                                                      const int32_t* __restrict__ conn4, float4* __restrict__ recs,
                                                      float4* __restrict__ leaf, float4* __restrict__ level1) {
     const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     Box6 b = empty_box();
     if (g < C) {
-        const int64_t o = perm[g];
+        const int64_t o = order_at(perm, g, C);
         const float4 lo = boxes[2 * o], hi = boxes[2 * o + 1];
         if (TETS) {
             float p[4][3];
@@ -781,7 +781,7 @@ cudaError_t launch_cell_boxes(int64_t C, const float* pts, const uint8_t* types,
     return cudaGetLastError();
 }
 
-cudaError_t launch_cell_tree(int64_t C, const int32_t* perm, const float4* boxes, const float* pts,
+cudaError_t launch_cell_tree(int64_t C, int32_t* perm, const float4* boxes, const float* pts,
                              const int32_t* conn4, float4* recs, float4* tree_boxes, cudaStream_t st) {
     if (C <= 0) return cudaSuccess;
     const WideTreeSize z = wide_tree_size(C);

@@ -167,7 +167,7 @@ __device__ __forceinline__ bool same_bits(float4 a, float4 b) {
 // One thread per Gaussian in Morton order: its record, its box as a leaf of the wide tree,
 // and (eight neighbouring lanes together) the box of its level-1 node.  Given `moved`, it is
 // set where a leaf that the tree held before is replaced by another box.
-__global__ void __launch_bounds__(256) k_gather_recs(int64_t P, const int32_t* __restrict__ perm,
+__global__ void __launch_bounds__(256) k_gather_recs(int64_t P, int32_t* __restrict__ perm,
                                                      const float* __restrict__ means, const float* __restrict__ values,
                                                      const float* __restrict__ weights,
                                                      const float* __restrict__ conics, const float4* __restrict__ boxes,
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(256) k_gather_recs(int64_t P, const int32_t* _
     const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     Box6 b = empty_box();
     if (g < P) {
-        const int64_t o = perm[g];
+        const int64_t o = order_at(perm, g, P);
         GaussRec r;
         r.r0 = make_float4(means[3 * o], means[3 * o + 1], means[3 * o + 2], weights[o]);
         r.r1 = make_float4(conics[6 * o], conics[6 * o + 1], conics[6 * o + 2], conics[6 * o + 3]);
@@ -201,14 +201,14 @@ __global__ void __launch_bounds__(256) k_gather_recs(int64_t P, const int32_t* _
 // window), and NaN keeps it out of every box, where an infinity would stretch a group's box
 // and centre over the ordinary samples beside it.
 __global__ void __launch_bounds__(256) k_sample_slots(int64_t S, int64_t n_slots, const float* __restrict__ samples,
-                                                      const int32_t* __restrict__ perm,
+                                                      int32_t* __restrict__ perm,
                                                       float4* __restrict__ s_sorted) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n_slots) return;
     float x = NAN, y = NAN, z = NAN;
     int o = -1;
     if (i < S) {
-        o = perm[i];
+        o = order_at(perm, i, S);
         x = samples[3 * (int64_t)o];
         y = samples[3 * (int64_t)o + 1];
         z = samples[3 * (int64_t)o + 2];
@@ -265,7 +265,7 @@ cudaError_t launch_preprocess(int64_t P, const float* means, const float* scales
     return cudaGetLastError();
 }
 
-cudaError_t launch_gather_recs(int64_t P, const int32_t* perm, const float* means, const float* values,
+cudaError_t launch_gather_recs(int64_t P, int32_t* perm, const float* means, const float* values,
                                const float* weights, const float* conics, const float4* boxes, GaussRec* recs,
                                float4* tree_boxes, bool levels, int* moved, cudaStream_t st) {
     if (P <= 0) return cudaSuccess;
@@ -276,7 +276,7 @@ cudaError_t launch_gather_recs(int64_t P, const int32_t* perm, const float* mean
     return launch_wide_levels(z, tree_boxes, st);
 }
 
-cudaError_t launch_sample_slots(int64_t S, int64_t n_slots, const float* samples, const int32_t* perm,
+cudaError_t launch_sample_slots(int64_t S, int64_t n_slots, const float* samples, int32_t* perm,
                                 float4* s_sorted, cudaStream_t st) {
     if (n_slots <= 0) return cudaSuccess;
     k_sample_slots<<<nb256(n_slots), 256, 0, st>>>(S, n_slots, samples, perm, s_sorted); gvc::note_launch();

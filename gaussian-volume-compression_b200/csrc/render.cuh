@@ -156,11 +156,11 @@ cudaError_t launch_preprocess(int64_t P, const float* means, const float* scales
                               const float* weights, float sm, float* conics_out, float4* boxes_out, cudaStream_t st);
 // Records in Morton order, and their wide tree at `tree_boxes` (levels false: its two lowest
 // levels only).  `moved` (device, or null): set if a leaf differs from what tree_boxes held.
-cudaError_t launch_gather_recs(int64_t P, const int32_t* perm, const float* means, const float* values,
+cudaError_t launch_gather_recs(int64_t P, int32_t* perm, const float* means, const float* values,
                                const float* weights, const float* conics, const float4* boxes, GaussRec* recs,
                                float4* tree_boxes, bool levels, int* moved, cudaStream_t st);
 // Sorted sample slots: (x, y, z, bits of the caller's index or -1).
-cudaError_t launch_sample_slots(int64_t S, int64_t n_slots, const float* samples, const int32_t* perm,
+cudaError_t launch_sample_slots(int64_t S, int64_t n_slots, const float* samples, int32_t* perm,
                                 float4* s_sorted, cudaStream_t st);
 // out_sorted: the forward's (out, W) per sorted slot when the caller's out_cells /
 // out_weights are that forward's outputs (else null: they are gathered).
@@ -183,12 +183,12 @@ cudaError_t launch_cell_boxes(int64_t C, const float* pts, const uint8_t* types,
                               const int32_t* conn, float4* boxes, cudaStream_t st);
 // Tree over the cells in Morton order and, of tetrahedra (conn4 given), their records (8 float4
 // per cell).
-cudaError_t launch_cell_tree(int64_t C, const int32_t* perm, const float4* boxes, const float* pts,
+cudaError_t launch_cell_tree(int64_t C, int32_t* perm, const float4* boxes, const float* pts,
                              const int32_t* conn4, float4* recs, float4* tree_boxes, cudaStream_t st);
 struct LocateArgs {
     int64_t N, C;
     const float* samples;
-    const int32_t* sperm;      // Morton order of the samples, or null: they are sorted
+    int32_t* sperm;            // Morton order of the samples, or null: they are sorted
     const float4* tree_boxes;
     const int32_t* cperm;
     const double* values;
@@ -210,10 +210,10 @@ cudaError_t launch_sample_tets(int64_t N, const float* samples, const int32_t* s
 // trainsamp.cu
 cudaError_t launch_tet_points(int64_t N, int64_t S, uint64_t seed, const float* pts, const int32_t* conn4, int64_t C,
                               float* out, uint32_t* w_lo, uint32_t* w_hi, uint32_t* w_batch, cudaStream_t st);
-cudaError_t launch_gather_points(int64_t N, const float* src, const int32_t* perm, float* dst, cudaStream_t st);
+cudaError_t launch_gather_points(int64_t N, const float* src, int32_t* perm, float* dst, cudaStream_t st);
 
 // knn.cu: the points in Morton order with their index in .w, and the LBVH over them
-cudaError_t launch_knn_points(int64_t n, const float* pts, const int32_t* perm, float4* sorted, cudaStream_t st);
+cudaError_t launch_knn_points(int64_t n, const float* pts, int32_t* perm, float4* sorted, cudaStream_t st);
 cudaError_t launch_knn3(int64_t n, const float4* sorted, const BvhNode* nodes, float* out, int* status,
                         cudaStream_t st);
 

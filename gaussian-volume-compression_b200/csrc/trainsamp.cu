@@ -105,10 +105,10 @@ __global__ void __launch_bounds__(256) k_tet_points(int64_t N, int64_t S, uint64
 }
 
 __global__ void __launch_bounds__(256) k_gather_points(int64_t N, const float* __restrict__ src,
-                                                       const int32_t* __restrict__ perm, float* __restrict__ dst) {
+                                                       int32_t* __restrict__ perm, float* __restrict__ dst) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= N) return;
-    const int64_t s = perm[i];
+    const int64_t s = order_at(perm, i, N);
     dst[3 * i] = src[3 * s];
     dst[3 * i + 1] = src[3 * s + 1];
     dst[3 * i + 2] = src[3 * s + 2];
@@ -126,7 +126,7 @@ cudaError_t launch_tet_points(int64_t N, int64_t S, uint64_t seed, const float* 
     return cudaGetLastError();
 }
 
-cudaError_t launch_gather_points(int64_t N, const float* src, const int32_t* perm, float* dst, cudaStream_t st) {
+cudaError_t launch_gather_points(int64_t N, const float* src, int32_t* perm, float* dst, cudaStream_t st) {
     if (N <= 0) return cudaSuccess;
     k_gather_points<<<nblk(N, 256), 256, 0, st>>>(N, src, perm, dst); gvc::note_launch();
     return cudaGetLastError();

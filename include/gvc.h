@@ -272,6 +272,13 @@ int gvc_debug_tc_gemm(gvc_ctx* ctx, const void* A, const void* B, int N, float* 
    GVC_ERR_TIMEOUT.  No counterpart in the reference. */
 int gvc_debug_wait_timeout(gvc_ctx* ctx, void* stream);
 
+/* Test hook: sorts n points [n,3] (4096 < n <= 2^20) by their Morton keys with the first 4096
+   withheld in every pass, so that each bounded wait for another block's published count runs
+   out (about 0.1 s a pass), over an order whose entries were no indices; then gathers the
+   sorted points.  perm [n] and slots [n,4] (x, y, z, bits of perm; 16-byte aligned, device): an
+   order that is wrong but within [0, n).  The next gvc_sync_status reports GVC_ERR_TIMEOUT. */
+int gvc_debug_sort_timeout(gvc_ctx* ctx, int64_t n, const float* pts, int32_t* perm, float* slots, void* stream);
+
 /* Test hook: the sample ordering of the last gvc_build_bvh: perm [S] int32 (sorted
    position -> caller index) and keys [S] uint32. */
 int gvc_debug_sample_order(gvc_ctx* ctx, int32_t* perm, uint32_t* keys, void* stream);
