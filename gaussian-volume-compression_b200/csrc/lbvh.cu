@@ -424,8 +424,10 @@ __device__ __forceinline__ uint32_t digit_rank(bool valid, uint32_t d, uint32_t*
         const uint32_t m = __ballot_sync(0xffffffffu, one);
         peers &= one ? m : ~m;
     }
-    // the first of them adds to the warp's count; the sum before is the rank of that lane.  The
-    // warp's additions are in program order, and one round need not wait for the one before.
+    // the first of them adds to the warp's count; the sum before is the rank of that lane.  Rounds
+    // may add to one count from different lanes: the barrier orders their additions (a shuffle
+    // orders no memory), and so the ranks, on which the sort's stability rests.
+    __syncwarp();
     const int leader = __ffs(peers) - 1;
     uint32_t pre = 0;
     if (valid && lane == leader) pre = atomicAdd(cnt + (d & 255u), (uint32_t)__popc(peers));
@@ -436,7 +438,7 @@ __device__ __forceinline__ uint32_t digit_rank(bool valid, uint32_t d, uint32_t*
 // What bounds a pass: the instructions of the ranking and the look-back, at few warps per
 // scheduler (43 KB of shared memory and 80 registers: three blocks per SM; four at 64 registers are as fast), and with
 // a handful of tiles their latency.  Loads all issued before the first key is ranked, votes and
-// pipelined shared-memory additions in place of match.any between warp barriers, 32-bit bounds,
+// one shared-memory addition a round in place of match.any, a read and a write, 32-bit bounds,
 // and a window of aggregates added whole: per pass 12.7 -> 7.3 us for 4096 keys, 17.2 -> 9.1
 // for 200k, 33 -> 25 for 2M, 60 -> 39 for 4M, 190 -> 122 for 16M.
 __global__ void __launch_bounds__(256, 3) k_os_scatter(const uint32_t* __restrict__ keys_in,
