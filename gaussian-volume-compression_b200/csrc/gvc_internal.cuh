@@ -54,14 +54,20 @@ struct __align__(16) BvhNode {
 
 constexpr uint32_t kLeafBit = 0x80000000u;
 
-// Growable device buffer owned by the context, or a view of memory that the caller lends.
+// Growable device buffer owned by the context; for a while a view of memory that the caller lends,
+// with what the context owns kept aside.
 struct DevBuf {
     void* ptr = nullptr;
     size_t bytes = 0;
     bool lent = false;
+    void* own_ptr = nullptr;  // while lent
+    size_t own_bytes = 0;
     cudaError_t ensure(size_t need) {
         if (need <= bytes && ptr) return cudaSuccess;
-        if (lent) give_back();
+        if (lent) {
+            give_back();
+            if (need <= bytes && ptr) return cudaSuccess;
+        }
         if (ptr) {
             cudaError_t e = cudaFree(ptr);
             if (e != cudaSuccess) return e;
@@ -77,20 +83,27 @@ struct DevBuf {
     template <class T>
     T* as() const { return reinterpret_cast<T*>(ptr); }
     void release() {
-        if (ptr && !lent) cudaFree(ptr);
+        give_back();
+        if (ptr) cudaFree(ptr);
         ptr = nullptr;
         bytes = 0;
-        lent = false;
     }
     // takes a view in place of memory of its own
     void lend(void* p, size_t n) {
-        release();
+        give_back();
+        own_ptr = ptr;
+        own_bytes = bytes;
         ptr = p;
         bytes = n;
         lent = true;
     }
     void give_back() {
-        if (lent) release();
+        if (!lent) return;
+        ptr = own_ptr;
+        bytes = own_bytes;
+        lent = false;
+        own_ptr = nullptr;
+        own_bytes = 0;
     }
 };
 

@@ -198,7 +198,8 @@ int gvc_training_samples(gvc_ctx* ctx, int64_t npts, const float* pts, int64_t C
 
 /* gvc_training_samples with its workspace lent by the caller (256-byte aligned device memory
    of gvc_training_workspace bytes; what does not fit is allocated as above).  The workspace
-   is used until `stream` has finished the call's work; the context keeps no address of it. */
+   is used until `stream` has finished the call's work; the context keeps no address of it, and
+   its own buffers as they were. */
 int64_t gvc_training_workspace(int64_t C, int64_t num_batches, int64_t batch_size, int with_gt);
 int gvc_training_samples_in(gvc_ctx* ctx, int64_t npts, const float* pts, int64_t C, const int32_t* conn4,
                             const double* values, int64_t num_batches, int64_t batch_size, uint64_t seed,
