@@ -65,6 +65,14 @@ def _download(dev, c, t, n, dtype):
     return out
 
 
+def _locate(dev, c, name, *args):
+    """A point location by context c, up to its end: the tree and the orders are the context's, and
+    another thread's call (on whatever stream) waits its turn for them."""
+    with c.lock:
+        c.call(name, *args, _stream(dev))
+        c.sync_status(torch.cuda.current_stream(dev).cuda_stream)
+
+
 def sample_mesh(dims_arr, origin_arr, spacing_arr, val_arr, samp_arr):
     """Uniform point field (x fastest) sampled by trilinear interpolation; outside -> -1
     in the values' dtype.  Output dtype follows the values (sample_mesh.cu:76-115)."""
@@ -177,9 +185,8 @@ def sample_meshu_cells(pts_arr, conn4, val_arr, samp_arr):
     d_samp = _dev(samples, np.float32)
     d_out = torch.empty(n, dtype=torch.float64, device="cuda:%d" % dev)
     d_cell = torch.empty(n, dtype=torch.int64, device="cuda:%d" % dev)
-    c.call("gvc_sample_tets", pts.shape[0], _n.ptr(d_pts), C, _n.ptr(d_conn), _n.ptr(d_vals), n,
-           _n.ptr(d_samp), _n.ptr(d_out), _n.ptr(d_cell), _stream(dev))
-    c.sync_status(torch.cuda.current_stream(dev).cuda_stream)
+    _locate(dev, c, "gvc_sample_tets", pts.shape[0], _n.ptr(d_pts), C, _n.ptr(d_conn), _n.ptr(d_vals), n,
+            _n.ptr(d_samp), _n.ptr(d_out), _n.ptr(d_cell))
     return d_out.cpu().numpy(), d_cell.cpu().numpy()
 
 
@@ -208,9 +215,8 @@ def sample_meshu_mixed(pts_arr, conn_arr, cell_types_arr, cell_offsets_arr, val_
     d_samp = _dev(samples, np.float32)
     d_out = torch.empty(n, dtype=torch.float64, device="cuda:%d" % dev)
     d_cell = torch.empty(n, dtype=torch.int64, device="cuda:%d" % dev)
-    c.call("gvc_sample_cells", pts.shape[0], _n.ptr(d_pts), C, _n.ptr(d_types), _n.ptr(d_offs), _n.ptr(d_conn),
-           _n.ptr(d_vals), n, _n.ptr(d_samp), _n.ptr(d_out), _n.ptr(d_cell), _stream(dev))
-    c.sync_status(torch.cuda.current_stream(dev).cuda_stream)
+    _locate(dev, c, "gvc_sample_cells", pts.shape[0], _n.ptr(d_pts), C, _n.ptr(d_types), _n.ptr(d_offs),
+            _n.ptr(d_conn), _n.ptr(d_vals), n, _n.ptr(d_samp), _n.ptr(d_out), _n.ptr(d_cell))
     return d_out.cpu().numpy(), d_cell.cpu().numpy()
 
 
@@ -236,12 +242,11 @@ def sample_meshu(pts_arr, conn_arr, cell_types_arr, cell_offsets_arr, val_arr, s
     if tets:
         # checked: four ids per cell, one cell after the other
         conn4 = cells.d_conn[int(cells.offs[0]):]
-        c.call("gvc_sample_tets", pts.shape[0], _n.ptr(d_pts), C, _n.ptr(conn4), _n.ptr(d_vals), n, _n.ptr(d_samp),
-               _n.ptr(d_out), None, _stream(dev))
+        _locate(dev, c, "gvc_sample_tets", pts.shape[0], _n.ptr(d_pts), C, _n.ptr(conn4), _n.ptr(d_vals), n,
+                _n.ptr(d_samp), _n.ptr(d_out), None)
     else:
-        c.call("gvc_sample_cells", pts.shape[0], _n.ptr(d_pts), C, _n.ptr(cells.d_types), _n.ptr(cells.d_offs),
-               _n.ptr(cells.d_conn), _n.ptr(d_vals), n, _n.ptr(d_samp), _n.ptr(d_out), None, _stream(dev))
-    c.sync_status(torch.cuda.current_stream(dev).cuda_stream)
+        _locate(dev, c, "gvc_sample_cells", pts.shape[0], _n.ptr(d_pts), C, _n.ptr(cells.d_types),
+                _n.ptr(cells.d_offs), _n.ptr(cells.d_conn), _n.ptr(d_vals), n, _n.ptr(d_samp), _n.ptr(d_out), None)
     return _download(dev, c, d_out, n, np.float64)
 
 

@@ -113,9 +113,13 @@ class GvcError(RuntimeError):
 
 
 class Context:
-    """Owns one gvc_ctx (created on the current CUDA device)."""
+    """Owns one gvc_ctx (created on the current CUDA device).
+
+    A native call works in the context's buffers, and the interpreter lets other threads run
+    meanwhile: threads that share a context hold `lock` while its buffers are in use."""
 
     def __init__(self):
+        self.lock = threading.RLock()
         L = lib()
         p = _vp()
         rc = L.gvc_ctx_create(ctypes.byref(p))

@@ -60,5 +60,6 @@ def distCUDA2(points):
     with torch.cuda.device(dev):
         c = _ctx(dev)
         st = torch.cuda.current_stream(dev).cuda_stream
-        c.call("gvc_knn3_mean_dist2", int(pts.shape[0]), _n.ptr(pts), _n.ptr(out), ctypes.c_void_p(st))
+        with c.lock:  # a call's launches are not mixed with another thread's
+            c.call("gvc_knn3_mean_dist2", int(pts.shape[0]), _n.ptr(pts), _n.ptr(out), ctypes.c_void_p(st))
     return out
