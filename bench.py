@@ -4,7 +4,7 @@
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
                     [--config large|medium|small|slice|tiny] [--eval-path plain|tensor_core|plain_tile] [--mesh] [--knn]
 
-Default configuration: FP32 forward (CTA pipeline) and the tensor-core backward reduction
+Default configuration: FP32 forward and the tensor-core backward reduction
 (--bwd-mode tensor_core); tc_vs_plain times FP32 throughout (the library default) and
 tensor cores throughout on the same step.
 
@@ -66,8 +66,8 @@ FP32_NOMINAL_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12
 #  -k regex:"k_backward_cta|k_forward_blocks" -s 2 -c 2 python bench.py --profile --steps 1 --warmup 1`
 # (and of k_backward_gauss with --bwd-mode deterministic); other workloads report null.
 # Tensor-pipe activity (sm__pipe_tc_cycles_active, share of peak) of the tensor-core kernels
-# in their committed --set full captures of the 2M x 4M profiling case (profiles/).
-TENSOR_PIPE_ACTIVE = {"k_backward_cta": 0.358, "k_forward_tc": 0.189}
+# in their committed captures of the 2M x 4M profiling case (profiles/).
+TENSOR_PIPE_ACTIVE = {"k_backward_cta": 0.355, "k_forward_tc": 0.185}
 MEASURED_TRAFFIC = {("large", "k_backward_cta"): 1.425e9 + 0.143e9,
                     ("large", "k_backward_gauss"): 1.327e9 + 0.124e9,
                     ("large", "k_forward_blocks"): 1.938e9 + 1.873e9}
@@ -83,8 +83,10 @@ def parse():
     # default: the fastest configuration within tolerance of the FP64 oracle (FP32 forward,
     # tensor-core backward reduction); the library's own default backward is the
     # deterministic one ("auto"), timed beside it in tc_vs_plain
-    p.add_argument("--bwd-mode", default="tensor_core", choices=["auto", "deterministic", "atomic", "tensor_core"])
-    p.add_argument("--eval-path", default="plain", choices=["plain", "tensor_core", "plain_tile"])
+    p.add_argument("--bwd-mode", default="tensor_core", choices=["auto", "deterministic", "atomic", "tensor_core"],
+                   help="'atomic' is 'deterministic' (GVC_OPT_BWD_MODE)")
+    p.add_argument("--eval-path", default="plain", choices=["plain", "tensor_core", "plain_tile"],
+                   help="'plain_tile' is 'plain' (GVC_OPT_EVAL_PATH)")
     p.add_argument("--traversal", default="stack", choices=["stack", "stackless"],
                    help="accepted, without effect (GVC_OPT_TRAVERSAL)")
     p.add_argument("--use-gaussian-bvh", action="store_true")
@@ -762,6 +764,15 @@ def knn_bench(dev, means, steps, warmup, with_cpu):
 # ----------------------------------------------------------------------------------------
 # Our arm
 # ----------------------------------------------------------------------------------------
+def forward_kernel(args, P, S, tc_bwd):
+    """The forward kernel that the library takes (capi.cu, forward_linked_rows of render.cuh)."""
+    if args.eval_path == "tensor_core":
+        return "k_forward_tc"
+    if tc_bwd:
+        return "k_forward_blocks" if S < 100_000 or (S >= 500_000 and S >= 2 * P) else "k_forward_cta"
+    return "k_forward_points" if float(S) * S < 360_000.0 * P else "k_forward_blocks"
+
+
 def run_ours(args):
     import torch
     import torch.distributed as dist
@@ -841,9 +852,9 @@ def run_ours(args):
     t_fwd = kt["fwd_kernel_ms"] / max(kt["fwd_kernel_calls"], 1)
     t_bwd = kt["bwd_kernel_ms"] / max(kt["bwd_kernel_calls"], 1)
     hbm, bf16, bf16s, src = measured_peaks()
-    bwd_kernel = "k_backward_cta" if args.bwd_mode == "tensor_core" or (
-        args.eval_path == "tensor_core" and args.bwd_mode == "auto") else "k_backward_gauss"
-    fwd_kernel = "k_forward_tc" if args.eval_path == "tensor_core" else "k_forward_blocks"
+    tc_bwd = args.bwd_mode == "tensor_core" or (args.eval_path == "tensor_core" and args.bwd_mode == "auto")
+    bwd_kernel = "k_backward_cta" if tc_bwd else "k_backward_gauss"
+    fwd_kernel = forward_kernel(args, P, S, tc_bwd)
     if t_bwd >= t_fwd:
         name, flops, t_k = bwd_kernel, f_bwd, t_bwd
     else:

@@ -293,7 +293,6 @@ int gvc_set_option(gvc_ctx* ctx, int option, int value) {
             return GVC_OK;
         case GVC_OPT_TRAVERSAL:
             if (value < 0 || value > 1) return fail(ctx, GVC_ERR_ARG, "traversal must be 0 or 1");
-            ctx->traversal = value;
             return GVC_OK;
         case GVC_OPT_TIME_KERNELS:
             drain_events(ctx);

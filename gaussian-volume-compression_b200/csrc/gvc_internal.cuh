@@ -128,7 +128,6 @@ struct gvc_ctx {
     int cov_grad_mode = 0;
     int bwd_mode = 0;
     int eval_path = 0;
-    int traversal = 0;      // GVC_OPT_TRAVERSAL
     int cand_log = 1;       // GVC_OPT_CAND_LOG
     int count_pairs = 0;
     int time_kernels = 0;   // record CUDA events around the evaluation kernels
