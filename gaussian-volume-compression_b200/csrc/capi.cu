@@ -497,7 +497,8 @@ int gvc_rasterize_gaussians(gvc_ctx* ctx, int64_t P, const float* means3D, const
         const int64_t n_blocks = (S + 127) / 128;
         if (ctx->clog.ensure(sizeof(int32_t) * kCandLogPerBlock * n_blocks) == cudaSuccess &&
             ctx->cmask.ensure(kCandLogPerBlock * n_blocks) == cudaSuccess &&
-            ctx->cend.ensure(sizeof(int32_t) * 8 * n_blocks) == cudaSuccess) {
+            ctx->cend.ensure(sizeof(int32_t) * 8 * n_blocks) == cudaSuccess &&
+            ctx->moved.ensure(sizeof(int)) == cudaSuccess) {
             fa.clog = ctx->clog.as<int32_t>();
             fa.cmask = ctx->cmask.as<uint8_t>();
             fa.cend = ctx->cend.as<int32_t>();
@@ -637,7 +638,6 @@ int gvc_rasterize_gaussians_backward(gvc_ctx* ctx, int64_t P, const float* means
             if (!same_gauss) {
                 if (!have_order) ctx->gauss_ready = false;  // the order below is not the forward's
                 if (use_log) {
-                    GVC_CUDA(ctx->moved.ensure(sizeof(int)), "alloc flag");
                     moved = ctx->moved.as<int>();
                     GVC_CUDA(cudaMemsetAsync(moved, 0, sizeof(int), st), "clear flag");
                 }

@@ -64,3 +64,30 @@ def test_copies_of_the_same_gaussians_read_the_log(cuda, orc):
     assert st["bwd_node_visits"] == 0
     assert_grads_close(g, oracle_backward(orc, tuple(a) + (samples,), fa[0].cpu().numpy(), fa[1].cpu().numpy(),
                                           fa[2].cpu().numpy().reshape(-1, 6), *up_np))
+
+
+def test_copies_under_capture(cuda, orc):
+    """A backward of copies is captured after one of the forward's own arrays has grown its buffers."""
+    import torch
+    a = orc.mixture_small(seed=3, P=4096)
+    samples = orc.grid_centres(48)
+    rng = np.random.default_rng(63)
+    up = [T(rng.normal(size=samples.shape[0]).astype(np.float32), cuda) for _ in range(2)]
+    with modes() as _C:
+        ta = [T(x, cuda) for x in a]
+        _C.build_bvh(T(samples, cuda), False, False)
+        out, outw, conics = forward(_C, ta)
+
+        def run(t):
+            return _C.rasterize_gaussians_backward(t[0], t[1], t[2], conics, t[3], t[4], out, outw, 1.0, 0, 0, 0, 1, 1, 1,
+                                                   -1.0, *up, False, False)
+        want = run(ta)
+        copies = [x.clone() for x in ta]
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = run(copies)
+        graph.replay()
+        _C.check_status()
+        # the atomics' order alone differs
+        for g, w in zip(got, want):
+            assert (g - w).abs().max() <= 1e-4 * w.abs().max()
